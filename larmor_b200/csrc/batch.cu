@@ -74,7 +74,7 @@ struct lar_batch_s {
     DeviceArray<DkiBatchJob> d_dki;
     DeviceArray<int64_t> dki_fit_first, dki_maps_first;
     int64_t dki_fit_tickets = 0, dki_maps_tickets = 0;
-    int dki_nmax = 0, dki_mmax = 0, dki_warps = 0;
+    int dki_nmax = 0, dki_mmax = 0, dki_warps = 0, dki_fast = 0;
     BatchViolators violators;
     double* refit_slots = nullptr;
     int refit_nslots = 0;
@@ -83,7 +83,7 @@ struct lar_batch_s {
     std::unique_ptr<MfodBatch, void (*)(MfodBatch*)> mfod{nullptr, mfod_batch_destroy};
     // Device scratch: counters, then the violator list and the re-fit slots.
     std::unique_ptr<void, CudaFree> scratch;
-    int* counters = nullptr;  // [0, 1] DTI queue, [2, 3] DKI fit queue, [4] violators, [5] re-fit queue
+    int* counters = nullptr;  // [0, 1] DTI queue, [2, 3] DKI fit queue, [4] violators, [5, 6] re-fit queues
 };
 
 extern "C" {
@@ -168,6 +168,7 @@ int lar_batch_finalize(lar_batch batch) {
             dki_voxels += j.v;
             b.dki_nmax = std::max(b.dki_nmax, j.d.n);
             b.dki_mmax = std::max(b.dki_mmax, j.d.m);
+            b.dki_fast += batch_fast_refit(j.d);
         }
         size_t viol_bytes = 0, slot_bytes = 0;
         if (!b.dki.empty()) {
@@ -229,8 +230,9 @@ int lar_batch_run(lar_batch batch, int families, void* stream) {
                                   b.dki_fit_tickets, b.dki_fit.weighted, b.dki_fit.max_rw, b.dki_fit.tol,
                                   b.counters + 2, b.violators, st);
             if (b.dki_mmax > 0)
-                launch_batch_refit(b.d_dki.ptr, b.violators, b.dki_fit.weighted, b.counters + 5, b.refit_slots,
-                                   b.refit_nslots, b.refit_slot_doubles, st);
+                launch_batch_refit(b.d_dki.ptr, int(b.dki.size()), b.dki_fast, b.dki_nmax, b.violators,
+                                   b.dki_fit.weighted, b.counters + 5, b.refit_slots, b.refit_nslots,
+                                   b.refit_slot_doubles, st);
             launch_batch_dki_maps(b.d_dki.ptr, b.dki_maps_first.ptr, int(b.dki.size()), b.dki_maps_tickets, st);
         }
         if ((families & LAR_BATCH_MFOD) && b.mfod) mfod_batch_run(b.mfod.get(), st);

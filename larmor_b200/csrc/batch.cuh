@@ -86,8 +86,11 @@ void launch_batch_log_warp(const DkiBatchJob* jobs, const int64_t* first, int n_
                            const BatchViolators& violators, cudaStream_t stream);
 size_t batch_refit_slot_doubles(int n_max, int p, int m_max);
 int batch_refit_slots();
-void launch_batch_refit(const DkiBatchJob* jobs, const BatchViolators& violators, int weighted, int* queue,
-                        double* workspace, int slots, size_t slot_doubles, cudaStream_t stream);
+// Whether a volume's violators take the fast re-fit.
+bool batch_fast_refit(const LogDesignDevice<double>& d);
+void launch_batch_refit(const DkiBatchJob* jobs, int n_jobs, int fast_jobs, int n_max, const BatchViolators& violators,
+                        int weighted, int* queue, double* workspace, int slots, size_t slot_doubles,
+                        cudaStream_t stream);
 void launch_batch_dki_maps(const DkiBatchJob* jobs, const int64_t* first, int n_jobs, int64_t tickets,
                            cudaStream_t stream);
 

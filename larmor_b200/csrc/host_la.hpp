@@ -182,6 +182,7 @@ struct LogDesignHost {
     std::vector<double> x;        // (n, p) row-major, scaled
     std::vector<double> pinv;     // (p, n) row-major
     std::vector<double> g;        // (m, p) row-major, scaled
+    bool dki = false;             // g has the form of DKI's constraints (dki_constraint_bound)
 };
 
 inline LogDesignHost prepare_log_design(const double* x, i64 n, i64 p, const double* g, i64 m) {

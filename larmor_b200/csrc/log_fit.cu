@@ -350,7 +350,7 @@ void set_smem(Kernel kernel, size_t bytes) {
                "cudaFuncSetAttribute");
 }
 
-// Scratch layout for a constrained fit of v voxels: [count, queue] ints, voxel ids, scaled
+// Scratch layout for a constrained fit of v voxels: [count, two queues] ints, voxel ids, scaled
 // parameters, then the warp slots of the re-fit.
 struct ScratchPlan {
     size_t ids_off, params_off, slots_off, total;
@@ -365,7 +365,7 @@ inline ScratchPlan plan_scratch(const lar::host::LogDesignHost& h, int64_t v) {
     s.params_off = up(s.ids_off + size_t(v) * sizeof(int64_t));
     s.slots_off = up(s.params_off + size_t(v) * h.p * sizeof(double));
     // As many warp slots as warps of the re-fit fit on the GPU at once.
-    const int64_t cap = constrained_resident_warps(int(h.n), int(h.p));
+    const int64_t cap = constrained_resident_warps(int(h.n), int(h.p), h.dki);
     s.slots = int(std::max<int64_t>(4, std::min<int64_t>((v + 3) / 4 * 4, cap)));
     s.total = s.slots_off + size_t(s.slots) * constrained_slot_doubles(int(h.n), int(h.p), int(h.m)) * sizeof(double);
     return s;
@@ -385,7 +385,7 @@ void launch_general(lar_log_design_s* h, const Src& src, int64_t v, int weighted
         require(v < (int64_t(1) << 31), "at most 2^31 - 1 voxels per constrained call");
         plan = plan_scratch(h->host, v);
         base = static_cast<char*>(h->scratch.reserve(plan.total));
-        cuda_check(cudaMemsetAsync(base, 0, 2 * sizeof(int), stream), "cudaMemsetAsync");
+        cuda_check(cudaMemsetAsync(base, 0, 3 * sizeof(int), stream), "cudaMemsetAsync");
         vl.count = reinterpret_cast<int*>(base);
         vl.capacity = int(v);
         vl.voxel = reinterpret_cast<int64_t*>(base + plan.ids_off);
@@ -533,8 +533,12 @@ int lar_log_design_create(const double* x, int64_t n, int64_t p, const double* g
         require(n >= p, "x must be (n, p) with n >= p: got (" + std::to_string(n) + ", " + std::to_string(p) + ")");
         auto h = std::make_unique<lar_log_design_s>();
         h->host = host::prepare_log_design(x, n, p, g, m);
+        double bound = 0.0;
+        h->host.dki = dki_constraint_bound(h->host.g.data(), m, p, &bound);
         upload_design<double>(h.get(), h->x64, h->pinvt64, h->z64, h->g64, h->scales64, h->d64);
         upload_design<float>(h.get(), h->x32, h->pinvt32, h->z32, h->g32, h->scales32, h->d32);
+        h->d64.dki = h->host.dki;
+        h->d64.bound = bound;
         h->d64.scales64 = h->scales64.ptr;
         h->d32.scales64 = h->scales64.ptr;
         *out = h.release();

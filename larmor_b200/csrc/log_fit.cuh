@@ -17,7 +17,34 @@ struct LogDesignDevice {
     const T* gt = nullptr;         // (p, m) the same, transposed (lanes over constraints read it coalesced)
     const T* scales = nullptr;     // (p,) column norms
     const double* scales64 = nullptr;  // (p,) column norms in double, for the outputs
+    // The constraints have DKI's form (dki_constraint_bound): rows D, V and bound D - V.
+    bool dki = false;
+    T bound = T(0);
 };
+
+// Whether the constraints g (m, p; host, row-major) have the form DKI's have: 256 rows D on columns
+// 1..6, 256 rows V on columns 7..21 and 256 rows b D - V (to rounding), b in *bound.
+constexpr int kDkiDirs = 256, kDkiP = 22, kDkiD = 6, kDkiV = 15;
+inline bool dki_constraint_bound(const double* g, int64_t m, int64_t p, double* bound) {
+    if (p != kDkiP || m != 3 * kDkiDirs) return false;
+    double b = 0.0;
+    for (int64_t i = 0; i < kDkiDirs && b == 0.0; ++i)
+        for (int64_t a = 1; a <= kDkiD && b == 0.0; ++a)
+            if (g[i * p + a] != 0.0) b = g[(2 * kDkiDirs + i) * p + a] / g[i * p + a];
+    const double eps = 4.0 * 2.220446049250313e-16;
+    for (int64_t i = 0; i < kDkiDirs; ++i) {
+        const double *d = g + i * p, *v = g + (kDkiDirs + i) * p, *c = g + (2 * kDkiDirs + i) * p;
+        for (int64_t a = 0; a < p; ++a) {
+            const bool in_d = a >= 1 && a <= kDkiD, in_v = a > kDkiD;
+            const double want = in_d ? b * d[a] : in_v ? -v[a] : 0.0;
+            const double err = c[a] - want, size = want < 0.0 ? -want : want;
+            if ((!in_d && d[a] != 0.0) || (!in_v && v[a] != 0.0)) return false;
+            if (!((err < 0.0 ? -err : err) <= eps * size)) return false;
+        }
+    }
+    *bound = b;
+    return true;
+}
 
 // ---- signal sources ---------------------------------------------------------------------
 //

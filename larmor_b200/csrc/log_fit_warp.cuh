@@ -40,10 +40,11 @@ inline size_t constrained_slot_doubles(int n, int p, int m) {
 // Re-fits the violators of `list` subject to g p >= 0 (cpp/src/dwi/log_fit.cpp:170-216), in
 // FP64, writing the constrained parameters (divided by the column scales) over `params` where
 // the re-fit succeeds. `workspace` holds `slots` warp slots of constrained_slot_doubles()
-// doubles; `queue` is a device int the kernel uses as its work counter (zeroed by the caller).
-// The warps of the constrained re-fit of designs of n measurements and p parameters that fit
-// on the GPU at once (its grid's size), a multiple of 4.
-int constrained_resident_warps(int n, int p);
+// doubles; `queue` is two device ints the kernels use as work counters (zeroed by the caller).
+// DKI's constraints take the fast kernel (list.voxel of what it fitted becomes ~voxel); the slots
+// are then for the few it hands on.
+// The warp slots a re-fit of this design uses at most (its grid's size), a multiple of 4.
+int constrained_resident_warps(int n, int p, bool dki);
 
 template <class Src>
 void launch_constrained(const LogDesignDevice<double>& d, const Src& src, int weighted,

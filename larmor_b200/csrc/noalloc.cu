@@ -75,7 +75,7 @@ extern "C" int lar_fit_log_signal_noalloc(const double* x, int64_t n, int64_t p,
         require(max_iter >= 0, "max_iter must be at least 0");
         if (v == 0) return;
 
-        // Scratch layout: [count, queue] ints | design (x, pinv^T, g, scales) | violator ids |
+        // Scratch layout: [count, two queues] ints | design (x, pinv^T, g, scales) | violator ids |
         // violator parameters | warp slots of the constrained re-fit.
         const size_t design_doubles = size_t(2 * n * p + 2 * m * p + p);
         const size_t design_off = 256;
@@ -111,13 +111,15 @@ extern "C" int lar_fit_log_signal_noalloc(const double* x, int64_t n, int64_t p,
         }
 
         require(log_s && params && broke, "log_s, params and broke must not be NULL");
-        // As many warp slots as the re-fit keeps resident, as far as the array has room.
-        if (m > 0) slots = std::max(4, std::min(slots, constrained_resident_warps(int(n), int(p))) / 4 * 4);
         unsigned char* base = noalloc_scratch_address();
         auto st = static_cast<cudaStream_t>(stream);
 
         // The prepared design, in FP64, copied into the static array.
-        const host::LogDesignHost h = host::prepare_log_design(x, n, p, g, m);
+        host::LogDesignHost h = host::prepare_log_design(x, n, p, g, m);
+        double bound = 0.0;
+        h.dki = dki_constraint_bound(h.g.data(), m, p, &bound);
+        // As many warp slots as the re-fit keeps resident, as far as the array has room.
+        if (m > 0) slots = std::max(4, std::min(slots, constrained_resident_warps(int(n), int(p), h.dki)) / 4 * 4);
         std::vector<double> packed(design_doubles);
         double* px_ = packed.data();
         double* ppinvt = px_ + n * p;
@@ -149,10 +151,12 @@ extern "C" int lar_fit_log_signal_noalloc(const double* x, int64_t n, int64_t p,
         d.gt = m > 0 ? dx + 2 * n * p + m * p : nullptr;
         d.scales = dx + 2 * n * p + 2 * m * p;
         d.scales64 = d.scales;
+        d.dki = h.dki;
+        d.bound = bound;
 
         ViolatorList<double> list;
         if (m > 0) {
-            cuda_check(cudaMemsetAsync(base, 0, 2 * sizeof(int), st), "cudaMemsetAsync (no-alloc counters)");
+            cuda_check(cudaMemsetAsync(base, 0, 3 * sizeof(int), st), "cudaMemsetAsync (no-alloc counters)");
             list.count = reinterpret_cast<int*>(base);
             list.capacity = int(v);
             list.voxel = reinterpret_cast<int64_t*>(base + ids_off);
