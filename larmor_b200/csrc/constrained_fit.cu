@@ -493,7 +493,7 @@ __device__ __forceinline__ void refit_violator(const LogDesignDevice<double>& d,
 // The old kernels below built a Householder QR with a warp reduction per column, read the 768 x 22
 // constraints from L2 in every gradient and refactored the active columns from scratch in every
 // fit: 1.7 M cycles per violator, 180 ms for the 179,846 violators of a 199,768-voxel volume of 134
-// measurements (3.9 ms for 2,832 of 95); this kernel takes 17.0 ms (0.26 ms). It is bound by the
+// measurements (3.9 ms for 2,832 of 95); this kernel takes 15.6 ms (0.24 ms). It is bound by the
 // latency of a warp's chain of steps at twelve warps per SM. What a step here cannot take (a Cholesky pivot or an active
 // column that rounding makes dependent, a table past kFastMaxRows) they fit from the start.
 
@@ -551,8 +551,9 @@ __device__ __forceinline__ void store_gram(const double (&acc)[6][2], double* a,
 }
 
 // a (kP rows, stride kR, its lower triangle G = L L^T) <- L^-T. A lane holds a row of G, then a column
-// of L^-1, in registers. False when a pivot is not positive.
-__device__ __noinline__ bool cholesky_inverse(double* a, int lane) {
+// of L^-1, in registers; each finished column of L goes round through buf (two 24-entry halves in
+// turn: a shuffle would move one value at a time). False when a pivot is not positive.
+__device__ __noinline__ bool cholesky_inverse(double* a, double* buf, int lane) {
     const int row = lane < kP ? lane : kP - 1;
     double g[kP];
 #pragma unroll
@@ -566,8 +567,11 @@ __device__ __noinline__ bool cholesky_inverse(double* a, int lane) {
         // Column k of L; its diagonal entry keeps the reciprocal.
         const double l = g[k] * inv;
         g[k] = lane == k ? inv : l;
+        double* column = buf + (k & 1) * 24;
+        if (lane < kP) column[lane] = l;
+        __syncwarp();
 #pragma unroll
-        for (int j = k + 1; j < kP; ++j) g[j] = fma(-l, __shfl_sync(0xffffffffu, l, j), g[j]);
+        for (int j = k + 1; j < kP; ++j) g[j] = fma(-l, column[j], g[j]);
     }
     if (!ok) return false;
     __syncwarp();
@@ -649,7 +653,7 @@ __device__ __forceinline__ bool fast_refit(const FastDesign d, const Src& src, i
         store_gram(acc, S, kP, lane);
     }
     __syncwarp();
-    if (!cholesky_inverse(S, lane)) return false;
+    if (!cholesky_inverse(S, cs, lane)) return false;
     // Second round: the Gram matrix of Q = W^(1/2) X S with the weighted signals as column 22.
     {
         double acc[6][2], bs[12];
@@ -696,7 +700,7 @@ __device__ __forceinline__ bool fast_refit(const FastDesign d, const Src& src, i
     }
     __syncwarp();
     const double qty = lane < kP ? Q[kP * kR + lane] : 0.0;
-    if (!cholesky_inverse(Q, lane)) return false;
+    if (!cholesky_inverse(Q, cs, lane)) return false;
     // S <- S S2 (both upper triangular), p_free = S (S2^T Q^T y).
     if (lane < kP) gv[lane] = qty;
     __syncwarp();

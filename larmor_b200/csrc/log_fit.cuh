@@ -129,15 +129,18 @@ struct CappedSource {
         }
         const double s0v = s0[voxel];
         // The mean of the voxel's own b0s, summed in measurement order as numpy does for short
-        // rows: lane 0 adds them up.
+        // rows.
         double own = 0.0;
         int count = 0;
-        if (lane == 0) {
-            for (int j = 0; j < n; ++j)
-                if (is_b0[j]) { own += double(s[voxel * n + j]); ++count; }
-            own = count ? own / count : 0.0;
+        for (int j0 = 0; j0 < n; j0 += 32) {
+            const int j = j0 + lane;
+            const bool b0 = j < n && is_b0[j];
+            const double x = b0 ? double(s[voxel * n + j]) : 0.0;
+            unsigned set = __ballot_sync(0xffffffffu, b0);
+            count += __popc(set);
+            for (; set; set &= set - 1u) own += __shfl_sync(0xffffffffu, x, __ffs(set) - 1);
         }
-        own = __shfl_sync(0xffffffffu, own, 0);
+        own = count ? own / count : 0.0;
         const bool repaired = !(fabs(s0v - own) <= 1e-9 * fabs(own));
         for (int j = lane; j < n; j += 32) {
             double x = double(s[voxel * n + j]);
