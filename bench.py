@@ -508,8 +508,8 @@ class MfodWorkload(_SdWorkloadBase):
     (float64 signals in, new FOD and fraction arrays out)."""
 
     name = "mfod_3tissue_110x110x70"
-    kernels = ("correlate_kernel", "ridge_nnls_half_kernel<3>", "ridge_nnls_kernel<1,2>", "lr_fractions_kernel",
-               "ridge_nnls_first_kernel<1,10>", "ridge_nnls_kernel<8,10>", "hr_fractions_kernel")
+    kernels = ("correlate_kernel", "ridge_nnls_low_kernel", "ridge_nnls_kernel<1,2>", "lr_fractions_kernel",
+               "ridge_nnls_high_kernel", "ridge_nnls_kernel<8,10>", "hr_fractions_kernel")
     has_fp32 = True
     fraction_tol = 1e-7
     # The plain FP32 fit takes seconds per step: a few timed steps bound the run.
@@ -592,10 +592,10 @@ class MfodWorkload(_SdWorkloadBase):
         # pass with a 32-column factor; the full-factor kernels refit only the few voxels handed
         # back (counted with the first kernels').
         return {"correlate_kernel": vr * 8 * (m + c_lr) + self.v * 8 * (m + c_hr),
-                "ridge_nnls_half_kernel<3>": vr * 8 * 2 * c_lr,
+                "ridge_nnls_low_kernel": vr * 8 * 2 * c_lr,
                 "ridge_nnls_kernel<1,2>": 0,
                 "lr_fractions_kernel": vr * 8 * (c_lr + m + 3),
-                "ridge_nnls_first_kernel<1,10>": self.v * 8 * 2 * c_hr,
+                "ridge_nnls_high_kernel": self.v * 8 * 2 * c_hr,
                 "ridge_nnls_kernel<8,10>": 0,
                 "hr_fractions_kernel": self.v * 8 * (c_hr + m + 3)}
 
@@ -778,10 +778,10 @@ def _job_kernel_bytes(job) -> dict:
     vr = int(job.out["rounds"].sum().item())
     c_lr, c_hr = job.handles["k_lr"].ca, job.handles["k_hr"].ca
     return {"correlate_kernel": vr * 8 * (n + c_lr) + v * 8 * (n + c_hr),
-            "ridge_nnls_half_kernel<3>": vr * 8 * 2 * c_lr,
+            "ridge_nnls_low_kernel": vr * 8 * 2 * c_lr,
             "ridge_nnls_kernel<1,2>": 0,
             "lr_fractions_kernel": vr * 8 * (c_lr + n + 3),
-            "ridge_nnls_first_kernel<1,10>": v * 8 * 2 * c_hr,
+            "ridge_nnls_high_kernel": v * 8 * 2 * c_hr,
             "ridge_nnls_kernel<8,10>": 0,
             "hr_fractions_kernel": v * 8 * (c_hr + n + 3)}
 
@@ -791,9 +791,9 @@ def _job_kernel_bytes(job) -> dict:
 QUEUE_KERNELS = {"batch_dti_kernel": "fit_dti_maps_kernel", "batch_log_warp_kernel": "fit_log_warp_kernel",
                  "batch_refit_kernel": "constrained_fit_kernel", "batch_dki_maps_kernel": "dki_maps_kernel",
                  "batch_plan_kernel": None, "batch_correlate_kernel": "correlate_kernel",
-                 "batch_half_kernel<3>": "ridge_nnls_half_kernel<3>", "batch_redo_kernel<1,2>": "ridge_nnls_kernel<1,2>",
+                 "batch_low_kernel": "ridge_nnls_low_kernel", "batch_redo_kernel<1,2>": "ridge_nnls_kernel<1,2>",
                  "batch_lr_fractions_kernel": "lr_fractions_kernel",
-                 "batch_first_kernel<1,10>": "ridge_nnls_first_kernel<1,10>",
+                 "batch_high_kernel": "ridge_nnls_high_kernel",
                  "batch_redo_kernel<8,10>": "ridge_nnls_kernel<8,10>",
                  "batch_hr_fractions_kernel": "hr_fractions_kernel"}
 

@@ -17,8 +17,10 @@
 //   correlate_kernel  K^T max(s_w - W_iso f_iso, 0) for 32 voxels x 16 RC columns per CTA, the
 //                     signals built while the tile is staged in shared memory (a tiled FP64
 //                     product, each entry summed over the measurements in increasing order);
-//   ridge_nnls_kernel the active-set NNLS on the Gram matrix and those correlations, one warp per
-//                     voxel (no work of the measurements' length unless the QR fallback runs);
+//   ridge_nnls_low_kernel the active-set NNLS on the Gram matrix and those correlations, one warp per
+//                     voxel (lean_nnls.cuh; ridge_nnls_high_kernel at high resolution); the few
+//                     voxels it hands back, and other sizes, take ridge_nnls_kernel (no work of the
+//                     measurements' length unless its QR fallback runs);
 //   lr_fractions_kernel  the fractions, the convergence test and the next round's voxel list.
 // The high-resolution FOD then runs the first two for all voxels, and hr_fractions_kernel the
 // final fractions. Each kernel's code is small (the warps of an SM share their instruction
@@ -35,7 +37,7 @@
 #include "common.cuh"
 #include "host_la.hpp"
 #include "drl.cuh"
-#include "group_nnls.cuh"
+#include "lean_nnls.cuh"
 #include "plain_fp32.cuh"
 #include "warp_chol.cuh"
 #include "warp_nnls.cuh"
@@ -262,14 +264,10 @@ __device__ __noinline__ bool ridge_qr_fit(const RidgeDev R, const double* sig, c
 // the flags, the workspace pointers) stays in registers; the outer (entering column) and inner
 // (blocking step) iterations of Lawson-Hanson share one loop with one fit, so the factor code
 // is emitted once.
-//
-// With REDO, a fit the factor cannot take (more than VPL * 32 active columns, or a pivot below the
-// relative tolerance) stops at once with *redo set, instead of continuing by QR: the caller refits
-// that voxel from the start with a larger factor, which takes the same steps up to that point.
-template <int VPL, int CPL, bool REDO = false, class State>
+template <int VPL, int CPL, class State>
 __device__ __forceinline__ bool ridge_nnls(const RidgeDev R, const SignalDev S, int64_t voxel,
                                            const double* __restrict__ corr, const NnlsSlot sl, State& st,
-                                           int lane, bool* redo = nullptr) {
+                                           int lane) {
     const int c = R.c;
     const InvFactor fac{sl.L, sl.M, sl.h, sl.w, sl.y, st.cols, VPL * 32};
     for (int j = lane; j < c; j += 32) {
@@ -382,10 +380,6 @@ __device__ __forceinline__ bool ridge_nnls(const RidgeDev R, const SignalDev S, 
                         ? inv_append<1>(fac, na, gee, corr[entering], entering, kMinPivot, lane)
                         : inv_append<VPL>(fac, na, gee, corr[entering], entering, kMinPivot, lane);
                 if (!appended) {
-                    if constexpr (REDO) {
-                        *redo = true;
-                        return true;
-                    }
                     failed = true;
                 } else {
                     if (lane == 0) sl.inf[entering] = 1;
@@ -444,219 +438,65 @@ __global__ void __launch_bounds__(kMtWarps * 32, (CPL <= 2 ? 6 : 4)) ridge_nnls_
     }
 }
 
-// The first pass of the high-resolution NNLS: one warp per voxel with a factor of VPL * 32 columns
-// (the active sets of the 300-direction FODs stay below 32; a larger factor takes more shared
-// memory and registers and fewer warps per SM); a voxel whose fit outgrows it, or needs the QR
-// fallback, goes on `redo` for ridge_nnls_kernel with the full factor, which fits it from the
-// start. Below the capacity the two take the same steps with the same factor code, so every
-// voxel gets the result the full-factor kernel gives.
-template <int VPL, int CPL>
-__global__ void __launch_bounds__(kMtWarps * 32, 4) ridge_nnls_first_kernel(
-    RidgeDev R, SignalDev S, int64_t count, const double* __restrict__ corr, int ldc, double* __restrict__ x_out,
-    int ldx, int* __restrict__ redo, int* redo_count, int* queue, double* __restrict__ workspace, size_t slot_size) {
-    using State = NnlsState<VPL * 32, CPL * 32>;
-    __shared__ State states[kMtWarps];
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+// ---- ridge NNLS of small active sets (lean_nnls.cuh) ---------------------------------------------
+
+// Low-resolution kernels (at most kLowCols columns): the Gram matrix in the CTA's shared memory.
+constexpr int kLowCols = 48, kLowWarps = 16;
+inline size_t low_smem_bytes(int c) {
+    return (size_t(kLowWarps) * kLeanWarpDoubles + size_t(c) * c) * sizeof(double);
+}
+// High-resolution kernels: its rows come from L2.
+constexpr int kHighWarps = 4, kHighCtas = 5;
+inline size_t high_smem_bytes() { return size_t(kHighWarps) * kLeanWarpDoubles * sizeof(double); }
+
+__device__ __forceinline__ void stage_gram(double* gs, const RidgeDev& R) {
+    for (int i = threadIdx.x; i < R.c * R.c; i += blockDim.x) gs[i] = R.gram[i];
+}
+
+// One warp per listed voxel, pulled from a device counter: x(v) <- the ridge NNLS of corr(v), or v
+// appended to `redo` when it needs the full-factor kernel.
+__global__ void __launch_bounds__(kLowWarps * 32, 2) ridge_nnls_low_kernel(
+    RidgeDev R, const int* __restrict__ list, int64_t count, const int* __restrict__ count_dev,
+    const double* __restrict__ corr, int ldc, double* __restrict__ x_out, int ldx, int* __restrict__ redo,
+    int* redo_count, int* queue) {
+    if (count_dev) count = min(count, int64_t(*count_dev));
+    if (count == 0) return;
+    extern __shared__ __align__(16) double lsm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    State& st = states[warp];
-    NnlsSlot sl = carve_nnls(workspace + (size_t(blockIdx.x) * kMtWarps + warp) * slot_size,
-                             smem_raw + warp * nnls_smem_bytes(R.c, VPL * 32), R.m, R.c, VPL * 32);
+    const LeanWarp q(lsm + warp * kLeanWarpDoubles);
+    double* const gs = lsm + kLowWarps * kLeanWarpDoubles;
+    stage_gram(gs, R);
+    __syncthreads();
     for (;;) {
-        int64_t voxel = 0;
-        if (lane == 0) voxel = atomicAdd(queue, 1);
-        voxel = __shfl_sync(0xffffffffu, voxel, 0);
-        if (voxel >= count) break;
-        bool again = false;
-        ridge_nnls<VPL, CPL, true>(R, S, voxel, corr + voxel * ldc, sl, st, lane, &again);
-        if (again) {
-            if (lane == 0) redo[atomicAdd(redo_count, 1)] = int(voxel);
-        } else {
-            for (int j = lane; j < R.c; j += 32) x_out[voxel * ldx + j] = sl.x[j];
-        }
+        int p = 0;
+        if (lane == 0) p = atomicAdd(queue, 1);
+        p = __shfl_sync(0xffffffffu, p, 0);
+        if (p >= count) break;
+        const int64_t voxel = listed(list, p);
+        if (!lean_nnls<2>(gs, R.c, R.c, R.tol, kMinPivot, corr + voxel * ldc, q, x_out + voxel * ldx, lane) && lane == 0)
+            redo[atomicAdd(redo_count, 1)] = int(voxel);
         __syncwarp();
     }
 }
 
-// ---- ridge NNLS, two voxels per warp (at most 48 directions) ---------------------------------
-
-// A half-warp's workspace: x, z (c each), the factor's vectors h, w, y (32 each) and the two
-// flag arrays in shared memory; the factor and its inverse (32 columns) in its global slot.
-struct HalfSlot {
-    double *x, *z, *h, *w, *y, *L, *M;
-    uint8_t *flag, *inf;
-};
-
-inline size_t half_slot_doubles() { return 2 * size_t(packed_size(2 * kHalf)) + 8; }
-
-__host__ __device__ inline size_t half_smem_bytes(int c) {
-    return ((2 * size_t(c) + 3 * 2 * kHalf) * sizeof(double) + 2 * size_t(c) + 15) / 16 * 16;
-}
-
-__device__ HalfSlot carve_half(double* base, unsigned char* smem, int c) {
-    HalfSlot s;
-    s.L = base;
-    s.M = base + packed_size(2 * kHalf);
-    double* q = reinterpret_cast<double*>(smem);
-    s.x = q; q += c;
-    s.z = q; q += c;
-    s.h = q; q += 2 * kHalf;
-    s.w = q; q += 2 * kHalf;
-    s.y = q; q += 2 * kHalf;
-    s.flag = reinterpret_cast<uint8_t*>(q);
-    s.inf = s.flag + c;
-    return s;
-}
-
-template <int CPL>
-struct HalfState {
-    int cols[2 * kHalf];      // factor columns, joining order
-    int sorted[kHalf * CPL];  // columns with x != 0, increasing
-};
-
-// ridge_nnls for one voxel on a half-warp (see group_nnls.cuh): the same steps, rules and
-// tolerances. False when the voxel needs the QR fallback (a pivot below the tolerance or more
-// than 32 active columns); the caller then hands it to the one-warp kernel.
-template <int CPL>
-__device__ __forceinline__ bool ridge_nnls_half(const RidgeDev R, const double* __restrict__ corr, const HalfSlot sl,
-                                                HalfState<CPL>& st, const HalfWarp hw) {
-    const int c = R.c;
-    const InvFactor fac{sl.L, sl.M, sl.h, sl.w, sl.y, st.cols, 2 * kHalf};
-    for (int j = hw.lane; j < c; j += kHalf) {
-        sl.x[j] = 0.0;
-        sl.z[j] = 0.0;
-        sl.flag[j] = 0;
-        sl.inf[j] = 0;
-    }
-    hw.sync();
-    int na = 0, inner = 0;
-    const int max_inner = 3 * c;
-    bool blocked = false;
+// The first pass of the high-resolution NNLS (65 to 320 columns): the active sets of the 300-direction
+// FODs rarely pass 32 columns, and the voxels that do go on `redo`.
+__global__ void __launch_bounds__(kHighWarps * 32, kHighCtas) ridge_nnls_high_kernel(
+    RidgeDev R, int64_t count, const double* __restrict__ corr, int ldc, double* __restrict__ x_out, int ldx,
+    int* __restrict__ redo, int* redo_count, int* queue) {
+    extern __shared__ __align__(16) double lsm[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const LeanWarp q(lsm + warp * kLeanWarpDoubles);
     for (;;) {
-        int entering = -1;
-        if (!blocked) {
-            int n_sorted = 0;
-            for (int base = 0; base < c; base += kHalf) {
-                const int j = base + hw.lane;
-                const bool nz = j < c && sl.x[j] != 0.0;
-                const unsigned ballot = hw.ballot(nz);
-                if (nz) st.sorted[n_sorted + __popc(ballot & ((1u << hw.lane) - 1u))] = j;
-                n_sorted += __popc(ballot);
-            }
-            hw.sync();
-            double g[CPL];
-#pragma unroll
-            for (int t = 0; t < CPL; ++t) {
-                const int j = hw.lane + kHalf * t;
-                g[t] = j < c ? corr[j] : 0.0;
-            }
-            for (int q = 0; q < n_sorted; ++q) {
-                const int col = st.sorted[q];
-                const double xc = sl.x[col];
-                const double* row = R.gram + size_t(col) * c;
-#pragma unroll
-                for (int t = 0; t < CPL; ++t) {
-                    const int j = hw.lane + kHalf * t;
-                    if (j < c) g[t] -= xc * row[j];
-                }
-            }
-            double bv = 0.0;
-            int bi = -1;
-#pragma unroll
-            for (int t = 0; t < CPL; ++t) {
-                const int j = hw.lane + kHalf * t;
-                if (j < c && !sl.flag[j] && (bi < 0 || g[t] > bv)) { bv = g[t]; bi = j; }
-            }
-            const int e = hw.argmax_first(bv, bi);
-            const double ge = e >= 0 ? hw.from(bv, e & (kHalf - 1)) : 0.0;
-            if (e < 0 || ge <= R.tol) break;
-            if (hw.lane == 0) sl.flag[e] = 1;
-            hw.sync();
-            entering = e;
-        } else {
-            if (++inner > max_inner) {
-                for (int j = hw.lane; j < c; j += kHalf) sl.x[j] = sl.z[j];
-                hw.sync();
-                return true;
-            }
-            double sv = 0.0;
-            int si = -1;
-            for (int j = hw.lane; j < c; j += kHalf) {
-                if (!sl.flag[j] || sl.z[j] > 0.0) continue;
-                const double dist = sl.x[j] - sl.z[j];
-                const double stp = dist > 0.0 ? sl.x[j] / dist : 0.0;
-                if (si < 0 || stp < sv) { sv = stp; si = j; }
-            }
-            double step;
-            const int b = hw.argmin_first(sv, si, &step);
-            for (int j = hw.lane; j < c; j += kHalf) sl.x[j] += step * (sl.z[j] - sl.x[j]);
-            hw.sync();
-            if (hw.lane == 0) {
-                sl.x[b] = 0.0;
-                sl.flag[b] = 0;
-            }
-            hw.sync();
-            for (int j = hw.lane; j < c; j += kHalf)
-                if (sl.flag[j] && !(fabs(sl.x[j]) >= R.tol)) sl.flag[j] = 0;
-            hw.sync();
-        }
-        for (int pos = na - 1; pos >= 0; --pos) {
-            const int col = st.cols[pos];
-            if (sl.flag[col]) continue;
-            half_remove(fac, na, pos, hw);
-            if (hw.lane == 0) sl.inf[col] = 0;
-            --na;
-            hw.sync();
-        }
-        if (entering >= 0) {
-            if (na >= 2 * kHalf) return false;
-            for (int r = hw.lane; r < na; r += kHalf) sl.h[r] = R.gram[size_t(st.cols[r]) * c + entering];
-            hw.sync();
-            if (!half_append(fac, na, R.gram[size_t(entering) * c + entering], corr[entering], entering, kMinPivot,
-                             hw))
-                return false;
-            if (hw.lane == 0) sl.inf[entering] = 1;
-            hw.sync();
-        }
-        half_solve(fac, na, sl.z, c, hw);
-        bool any = false;
-        for (int j = hw.lane; j < c; j += kHalf) any |= sl.flag[j] && sl.z[j] <= 0.0;
-        blocked = hw.any(any);
-        if (!blocked) {
-            for (int j = hw.lane; j < c; j += kHalf) sl.x[j] = sl.z[j];
-            hw.sync();
-        }
-    }
-    return true;
-}
-
-// Two listed voxels per warp, one per half, pulled from a device counter: x(v) <- the ridge
-// NNLS of corr(v), or v appended to `redo` when it needs the QR fallback.
-template <int CPL>
-__global__ void __launch_bounds__(kMtWarps * 32, 8) ridge_nnls_half_kernel(
-    RidgeDev R, const int* __restrict__ list, int64_t count, const int* __restrict__ count_dev,
-    const double* __restrict__ corr, int ldc, double* __restrict__ x_out, int ldx, int* __restrict__ redo,
-    int* redo_count, int* queue, double* __restrict__ workspace, size_t slot_size) {
-    if (count_dev) count = min(count, int64_t(*count_dev));
-    __shared__ HalfState<CPL> states[2 * kMtWarps];
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const HalfWarp hw(threadIdx.x & 31);
-    const int gid = int(threadIdx.x >> 4);  // half-warp within the CTA
-    HalfState<CPL>& st = states[gid];
-    const HalfSlot sl = carve_half(workspace + (size_t(blockIdx.x) * 2 * kMtWarps + gid) * slot_size,
-                                   smem_raw + gid * half_smem_bytes(R.c), R.c);
-    for (;;) {
-        long long p = 0;
-        if (hw.lane == 0) p = atomicAdd(queue, 1);
-        p = hw.from(p, 0);
-        if (p >= count) break;
-        const int64_t voxel = listed(list, p);
-        const bool done = ridge_nnls_half<CPL>(R, corr + voxel * ldc, sl, st, hw);
-        if (done) {
-            for (int j = hw.lane; j < R.c; j += kHalf) x_out[voxel * ldx + j] = sl.x[j];
-        } else if (hw.lane == 0) {
-            redo[atomicAdd(redo_count, 1)] = int(voxel);
-        }
-        hw.sync();
+        int voxel = 0;
+        if (lane == 0) voxel = atomicAdd(queue, 1);
+        voxel = __shfl_sync(0xffffffffu, voxel, 0);
+        if (voxel >= count) break;
+        if (!lean_nnls<10>(R.gram, R.c, R.c, R.tol, kMinPivot, corr + int64_t(voxel) * ldc, q,
+                           x_out + int64_t(voxel) * ldx, lane) &&
+            lane == 0)
+            redo[atomicAdd(redo_count, 1)] = voxel;
+        __syncwarp();
     }
 }
 
@@ -1050,6 +890,8 @@ __global__ void __launch_bounds__(kMtWarps * 32, 5) hr_fractions_kernel(
 
 // ---- batches (batch.cuh): every mFOD volume of a batch through one queue per stage ------------
 
+constexpr int kLowTicket = 256;  // voxels of a ticket of the low-resolution NNLS
+
 // A volume of a batch: its solvers and kernels, signals, shell weights and outputs.
 struct MfodBatchJob {
     int64_t v, off;  // voxels; the row of its first voxel in the batch's per-voxel state
@@ -1072,6 +914,7 @@ struct MfodBatchState {
     uint8_t* bad;
     int64_t* vfirst;   // (n_jobs + 1) this stage's first voxel ticket per volume
     int64_t* tfirst;   // (n_jobs + 1) its first correlation tile per volume
+    int64_t* qfirst;   // (n_jobs + 1) its first ticket of kLowTicket voxels per volume
     int64_t* redo;     // volume << 32 | voxel, for the one-warp NNLS
     int* redo_count;
 };
@@ -1096,16 +939,19 @@ __device__ __forceinline__ SignalDev batch_signal(const MfodBatchState& B, const
 // The tickets of a stage from each volume's count (null: every voxel).
 __global__ void batch_plan_kernel(MfodBatchState B, const int* __restrict__ counts) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    int64_t a = 0, b = 0;
+    int64_t a = 0, b = 0, q = 0;
     for (int j = 0; j < B.n_jobs; ++j) {
         B.vfirst[j] = a;
         B.tfirst[j] = b;
+        B.qfirst[j] = q;
         const int64_t c = counts ? int64_t(counts[j]) : B.jobs[j].v;
         a += c;
         b += (c + kCorrVoxels - 1) / kCorrVoxels;
+        q += (c + kLowTicket - 1) / kLowTicket;
     }
     B.vfirst[B.n_jobs] = a;
     B.tfirst[B.n_jobs] = b;
+    B.qfirst[B.n_jobs] = q;
 }
 
 // correlate_kernel over every volume: a CTA per (volume, tile of kCorrVoxels listed voxels).
@@ -1132,35 +978,47 @@ __global__ void __launch_bounds__(128) batch_correlate_kernel(MfodBatchState B, 
     }
 }
 
-// ridge_nnls_half_kernel over every volume's list.
-template <int CPL>
-__global__ void __launch_bounds__(kMtWarps * 32, 8) batch_half_kernel(MfodBatchState B, const int* __restrict__ list,
-                                                                     int c_max, int* queue,
-                                                                     double* __restrict__ workspace,
-                                                                     size_t slot_size) {
-    __shared__ HalfState<CPL> states[2 * kMtWarps];
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const HalfWarp hw(threadIdx.x & 31);
-    const int gid = int(threadIdx.x >> 4);
-    HalfState<CPL>& st = states[gid];
-    const HalfSlot sl = carve_half(workspace + (size_t(blockIdx.x) * 2 * kMtWarps + gid) * slot_size,
-                                   smem_raw + gid * half_smem_bytes(c_max), c_max);
-    const int64_t total = B.vfirst[B.n_jobs];
+// ridge_nnls_low_kernel over every volume's list: a CTA takes a ticket of kLowTicket listed voxels of
+// one volume, whose Gram matrix it keeps until its ticket moves to another.
+__global__ void __launch_bounds__(kLowWarps * 32, 2) batch_low_kernel(MfodBatchState B, const int* __restrict__ list,
+                                                                     int* queue) {
+    extern __shared__ __align__(16) double lsm[];
+    __shared__ int ticket, taken;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const LeanWarp q(lsm + warp * kLeanWarpDoubles);
+    double* const gs = lsm + kLowWarps * kLeanWarpDoubles;
+    const int64_t total = B.qfirst[B.n_jobs];
+    int cur = -1;
     for (;;) {
-        long long p = 0;
-        if (hw.lane == 0) p = atomicAdd(queue, 1);
-        p = hw.from(p, 0);
-        if (p >= total) break;
-        const BatchItem it = batch_item(B, list, p);
-        const MfodBatchJob& J = B.jobs[it.job];
-        const RidgeDev R = J.lr;
-        const int64_t row = J.off + it.voxel;
-        if (ridge_nnls_half<CPL>(R, B.corr + row * B.ldc, sl, st, hw)) {
-            for (int j = hw.lane; j < R.c; j += kHalf) B.xlr[row * B.ldx + j] = sl.x[j];
-        } else if (hw.lane == 0) {
-            B.redo[atomicAdd(B.redo_count, 1)] = (int64_t(it.job) << 32) | it.voxel;
+        __syncthreads();  // every warp is done with the last ticket
+        if (threadIdx.x == 0) {
+            ticket = atomicAdd(queue, 1);
+            taken = 0;
         }
-        hw.sync();
+        __syncthreads();
+        const int64_t t = ticket;
+        if (t >= total) break;
+        const int j = ticket_job(B.qfirst, B.n_jobs, t);
+        const MfodBatchJob& J = B.jobs[j];
+        const RidgeDev R = J.lr;
+        if (j != cur) {
+            stage_gram(gs, R);
+            cur = j;
+            __syncthreads();
+        }
+        const int64_t p0 = (t - B.qfirst[j]) * kLowTicket;
+        const int64_t count = min(int64_t(kLowTicket), B.vfirst[j + 1] - B.vfirst[j] - p0);
+        for (;;) {
+            int p = 0;
+            if (lane == 0) p = atomicAdd(&taken, 1);
+            p = __shfl_sync(0xffffffffu, p, 0);
+            if (p >= count) break;
+            const int64_t voxel = list ? int64_t(list[J.off + p0 + p]) : p0 + p, row = J.off + voxel;
+            if (!lean_nnls<2>(gs, R.c, R.c, R.tol, kMinPivot, B.corr + row * B.ldc, q, B.xlr + row * B.ldx, lane) &&
+                lane == 0)
+                B.redo[atomicAdd(B.redo_count, 1)] = (int64_t(j) << 32) | voxel;
+            __syncwarp();
+        }
     }
 }
 
@@ -1196,17 +1054,11 @@ __global__ void __launch_bounds__(kMtWarps * 32, (CPL <= 2 ? 6 : 4)) batch_redo_
     }
 }
 
-// ridge_nnls_first_kernel<1, 10> over every voxel of every volume.
-__global__ void __launch_bounds__(kMtWarps * 32, 5) batch_first_kernel(MfodBatchState B, int c_max, int* queue,
-                                                                      double* __restrict__ workspace,
-                                                                      size_t slot_size) {
-    using State = NnlsState<32, 10 * 32>;
-    __shared__ State states[kMtWarps];
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+// ridge_nnls_high_kernel over every voxel of every volume.
+__global__ void __launch_bounds__(kHighWarps * 32, kHighCtas) batch_high_kernel(MfodBatchState B, int* queue) {
+    extern __shared__ __align__(16) double lsm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    State& st = states[warp];
-    double* slot = workspace + (size_t(blockIdx.x) * kMtWarps + warp) * slot_size;
-    unsigned char* wsm = smem_raw + warp * nnls_smem_bytes(c_max, 32);
+    const LeanWarp q(lsm + warp * kLeanWarpDoubles);
     const int64_t total = B.vfirst[B.n_jobs];
     for (;;) {
         long long p = 0;
@@ -1216,15 +1068,10 @@ __global__ void __launch_bounds__(kMtWarps * 32, 5) batch_first_kernel(MfodBatch
         const BatchItem it = batch_item(B, nullptr, p);
         const MfodBatchJob& J = B.jobs[it.job];
         const RidgeDev R = J.hr;
-        NnlsSlot sl = carve_nnls(slot, wsm, R.m, R.c, 32);
-        const int64_t row = J.off + it.voxel;
-        bool again = false;
-        ridge_nnls<1, 10, true>(R, batch_signal(B, J, J.hrt), it.voxel, B.corr + row * B.ldc, sl, st, lane, &again);
-        if (again) {
-            if (lane == 0) B.redo[atomicAdd(B.redo_count, 1)] = (int64_t(it.job) << 32) | it.voxel;
-        } else {
-            for (int j = lane; j < R.c; j += 32) J.fods[it.voxel * R.c + j] = sl.x[j];
-        }
+        if (!lean_nnls<10>(R.gram, R.c, R.c, R.tol, kMinPivot, B.corr + (J.off + it.voxel) * B.ldc, q,
+                           J.fods + it.voxel * R.c, lane) &&
+            lane == 0)
+            B.redo[atomicAdd(B.redo_count, 1)] = (int64_t(it.job) << 32) | it.voxel;
         __syncwarp();
     }
 }
@@ -1301,18 +1148,18 @@ __global__ void __launch_bounds__(kMtWarps * 32, 4) batch_hr_fractions_kernel(Mf
 // ---- host side -------------------------------------------------------------------------
 
 // The warps of a persistent grid: as many as the SMs hold at once (or one per item), in whole
-// CTAs of kMtWarps.
+// CTAs of `warps`.
 template <class Kernel>
-int64_t resident_slots(Kernel kernel, size_t smem, int64_t items, const char* setting) {
+int64_t resident_slots(Kernel kernel, size_t smem, int64_t items, const char* setting, int warps = kMtWarps) {
     require(smem <= 200 * 1024, "the kernel has too many columns for the shared-memory solver");
     cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
                "cudaFuncSetAttribute");
     int per_sm = 0;
-    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kMtWarps * 32, smem),
+    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, smem),
                "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
-    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((items + kMtWarps - 1) / kMtWarps,
+    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((items + warps - 1) / warps,
                                                                   int64_t(sm_count()) * ctas_per_sm(per_sm, setting)));
-    return blocks * kMtWarps;
+    return blocks * warps;
 }
 
 // A bump allocator over one device buffer, 256-byte aligned pieces.
@@ -1505,30 +1352,26 @@ static int fit_multi_tissue(const double* signals, int64_t v, const double* weig
                                  3 * sizeof(int) + 1;
         const int64_t n_max = std::min<int64_t>(v, std::max<int64_t>(4096, int64_t((size_t(4) << 30) / per_voxel)));
         const int64_t lr_slots = lr_drl ? 0 : resident_slots(lr_nnls.kernel, lr_smem, n_max, "sd.nnls.ctas_per_sm");
-        // Low-resolution kernels of at most 48 directions with normal equations: two voxels per
-        // warp (ridge_nnls_half_kernel), the voxels that need the QR fallback then refitted by
-        // the one-warp kernel.
-        const bool half = !lr_drl && lrs.normal_equations && c_lr <= 48;
-        auto half_kernel = ridge_nnls_half_kernel<3>;
-        const size_t half_smem = half_smem_bytes(c_lr) * 2 * kMtWarps;
-        const int64_t half_warps = half ? resident_slots(half_kernel, half_smem, n_max, "sd.nnls.ctas_per_sm") : 0;
+        // Low-resolution kernels of at most 48 directions with normal equations: the lean NNLS with the
+        // Gram matrix in shared memory, the voxels that need the QR fallback or a larger factor then
+        // refitted by the full-factor kernel.
+        const bool low = !lr_drl && lrs.normal_equations && c_lr <= kLowCols;
+        const size_t low_smem = low_smem_bytes(c_lr);
+        const int64_t low_slots =
+            low ? resident_slots(ridge_nnls_low_kernel, low_smem, n_max, "sd.nnls.ctas_per_sm", kLowWarps) : 0;
         const int64_t hr_slots = hr_drl ? 0 : resident_slots(hr_nnls.kernel, hr_smem, n_max, "sd.nnls.ctas_per_sm");
-        // High-resolution kernels of 65 to 320 directions with normal equations: a first pass with
-        // a 32-column factor, the voxels that outgrow it refitted by the full-factor kernel.
-        const bool hr_first = !hr_drl && hrs.normal_equations && c_hr > 64 && c_hr <= 320;
-        auto first_kernel = ridge_nnls_first_kernel<1, 10>;
-        const size_t first_smem = nnls_smem_bytes(c_hr, 32) * kMtWarps;
-        const int64_t first_slots = hr_first ? resident_slots(first_kernel, first_smem, n_max, "sd.nnls.ctas_per_sm") : 0;
-        const size_t first_slot = nnls_slot_doubles(mi, 32);
+        // High-resolution kernels of 65 to 320 directions with normal equations: the same, with the
+        // Gram matrix in L2.
+        const bool high = !hr_drl && hrs.normal_equations && c_hr > 64 && c_hr <= 320;
+        const int64_t high_slots =
+            high ? resident_slots(ridge_nnls_high_kernel, high_smem_bytes(), n_max, "sd.nnls.ctas_per_sm", kHighWarps) : 0;
         const int64_t lf_slots = resident_slots(lr_fractions_kernel, 0, n_max, "sd.fractions.ctas_per_sm");
         const int64_t hf_slots = resident_slots(hr_fractions_kernel, 0, n_max, "sd.fractions.ctas_per_sm");
         const size_t lr_slot = nnls_slot_doubles(mi, lr_nnls.cap), hr_slot = nnls_slot_doubles(mi, hr_nnls.cap);
         const size_t lf_slot = frac_slot_doubles(mi, c_lr, 1 + ci), hf_slot = frac_slot_doubles(mi, c_hr, nf);
         const size_t slot_doubles =
-            std::max(std::max(std::max(std::max(size_t(lr_slots) * lr_slot, size_t(hr_slots) * hr_slot),
-                                       std::max(size_t(lf_slots) * lf_slot, size_t(hf_slots) * hf_slot)),
-                              size_t(2 * half_warps) * half_slot_doubles()),
-                     size_t(first_slots) * first_slot);
+            std::max(std::max(size_t(lr_slots) * lr_slot, size_t(hr_slots) * hr_slot),
+                     std::max(size_t(lf_slots) * lf_slot, size_t(hf_slots) * hf_slot));
         struct Pieces {
             int* counters;  // [0] the persistent kernels' work counter, [2], [3] the two lists' counts,
                             // [4] the voxels to refit by the one-warp NNLS
@@ -1566,8 +1409,15 @@ static int fit_multi_tissue(const double* signals, int64_t v, const double* weig
         const bool graph = capturing || device_rounds;
         const double* dweights = hr_solver->device_weights(weights, m, capturing);
         int* host_count = graph ? nullptr : hr_solver->count_buffer();
-        auto blocks = [](int64_t slots, int64_t count) {
-            return unsigned(std::max<int64_t>(1, std::min<int64_t>(slots / kMtWarps, (count + kMtWarps - 1) / kMtWarps)));
+        auto blocks = [](int64_t slots, int64_t count, int warps = kMtWarps) {
+            return unsigned(std::max<int64_t>(1, std::min<int64_t>(slots / warps, (count + warps - 1) / warps)));
+        };
+        // The low-resolution kernel's wide CTAs: a short list still takes a CTA per SM, so that its voxels
+        // do not queue on a few SMs.
+        auto low_blocks = [&](int64_t slots, int64_t count) {
+            return unsigned(std::min<int64_t>(slots / kLowWarps,
+                                              std::max<int64_t>((count + kLowWarps - 1) / kLowWarps,
+                                                                std::min<int64_t>(count, sm_count()))));
         };
         auto reset_queue = [&] { cuda_check(cudaMemsetAsync(P.counters, 0, sizeof(int), st), "cudaMemsetAsync"); };
         for (int64_t v0 = 0; v0 < v; v0 += n_max) {
@@ -1592,18 +1442,16 @@ static int fit_multi_tissue(const double* signals, int64_t v, const double* weig
                 if (lr_drl) {
                     const DrlSignal lr_as{sig, dweights, lrt.wiso, P.fiso, mi, ci};
                     launch_drl_listed(lr_solver->drl, lr_as, cur, count, cur_count, P.xlr, c_lr, st);
-                } else if (half) {
+                } else if (low) {
                     cuda_check(cudaMemsetAsync(P.counters + 4, 0, sizeof(int), st), "cudaMemsetAsync");
                     {
-                        LaunchScope scope("ridge_nnls_half_kernel<3>", st);
-                        half_kernel<<<blocks(half_warps, (count + 1) / 2), kMtWarps * 32, half_smem, st>>>(
-                            lrs, cur, count, cur_count, P.corr, c_lr, P.xlr, c_lr, P.redo, P.counters + 4, P.counters,
-                            P.slots, half_slot_doubles());
-                        cuda_check(cudaGetLastError(), "ridge_nnls_half_kernel launch");
+                        LaunchScope scope("ridge_nnls_low_kernel", st);
+                        ridge_nnls_low_kernel<<<low_blocks(low_slots, count), kLowWarps * 32, low_smem, st>>>(
+                            lrs, cur, count, cur_count, P.corr, c_lr, P.xlr, c_lr, P.redo, P.counters + 4, P.counters);
+                        cuda_check(cudaGetLastError(), "ridge_nnls_low_kernel launch");
                     }
                     reset_queue();
-                    // The voxels the two-voxel kernel handed back are rare (its QR fallback): a
-                    // persistent grid of one CTA per SM takes them.
+                    // The voxels it handed back are rare: a persistent grid of one CTA per SM takes them.
                     LaunchScope scope(lr_nnls.name, st);
                     const unsigned redo_blocks = std::min<unsigned>(blocks(lr_slots, count), unsigned(sm_count()));
                     lr_nnls.kernel<<<redo_blocks, kMtWarps * 32, lr_smem, st>>>(
@@ -1643,14 +1491,14 @@ static int fit_multi_tissue(const double* signals, int64_t v, const double* weig
             } else {
                 launch_correlate(hr_sig, nullptr, n, nullptr, hrs, P.corr, c_hr, st);
                 reset_queue();
-                if (hr_first) {
+                if (high) {
                     cuda_check(cudaMemsetAsync(P.counters + 4, 0, sizeof(int), st), "cudaMemsetAsync");
                     {
-                        LaunchScope scope("ridge_nnls_first_kernel<1,10>", st);
-                        first_kernel<<<blocks(first_slots, n), kMtWarps * 32, first_smem, st>>>(
-                            hrs, hr_sig, n, P.corr, c_hr, fods + v0 * c_hr, c_hr, P.redo, P.counters + 4, P.counters,
-                            P.slots, first_slot);
-                        cuda_check(cudaGetLastError(), "ridge_nnls_first_kernel launch");
+                        LaunchScope scope("ridge_nnls_high_kernel", st);
+                        ridge_nnls_high_kernel<<<blocks(high_slots, n, kHighWarps), kHighWarps * 32, high_smem_bytes(),
+                                                 st>>>(hrs, n, P.corr, c_hr, fods + v0 * c_hr, c_hr, P.redo,
+                                                       P.counters + 4, P.counters);
+                        cuda_check(cudaGetLastError(), "ridge_nnls_high_kernel launch");
                     }
                     reset_queue();
                     // The voxels the first pass handed back (rare): a grid of one CTA per SM.
@@ -1696,9 +1544,9 @@ struct MfodBatch {
     MfodBatchState B{};
     int *list[2] = {nullptr, nullptr}, *counts[2] = {nullptr, nullptr}, *queue = nullptr;
     double* slots = nullptr;
-    int64_t half_warps = 0, lr_slots = 0, first_slots = 0, hr_slots = 0, lf_slots = 0, hf_slots = 0;
-    size_t half_smem = 0, lr_smem = 0, first_smem = 0, hr_smem = 0;
-    size_t lr_slot = 0, first_slot = 0, hr_slot = 0, lf_slot = 0, hf_slot = 0;
+    int64_t low_slots = 0, high_slots = 0, lr_slots = 0, hr_slots = 0, lf_slots = 0, hf_slots = 0;
+    size_t low_smem = 0, lr_smem = 0, hr_smem = 0;
+    size_t lr_slot = 0, hr_slot = 0, lf_slot = 0, hf_slot = 0;
     ~MfodBatch() {
         if (scratch) cudaFree(scratch);
     }
@@ -1771,25 +1619,22 @@ void mfod_batch_finalize(MfodBatch* b) {
     const int64_t V = b->voxels, nj = int64_t(b->jobs.size());
     const int ci = b->ci, mi = b->m_max, ldc = std::max(b->c_lr_max, b->c_hr_max), ldx = b->c_lr_max;
     // Launch shapes: the single-volume fit's persistent grids, sized for the whole batch.
-    b->half_smem = half_smem_bytes(b->c_lr_max) * 2 * kMtWarps;
-    b->half_warps = resident_slots(batch_half_kernel<3>, b->half_smem, V, "sd.nnls.ctas_per_sm");
+    b->low_smem = low_smem_bytes(b->c_lr_max);
+    b->low_slots = resident_slots(batch_low_kernel, b->low_smem, V, "sd.nnls.ctas_per_sm", kLowWarps);
+    b->high_slots = resident_slots(batch_high_kernel, high_smem_bytes(), V, "sd.nnls.ctas_per_sm", kHighWarps);
     b->lr_smem = nnls_smem_bytes(b->c_lr_max, 32) * kMtWarps;
     b->lr_slots = resident_slots(batch_redo_kernel<1, 2, false>, b->lr_smem, V, "sd.nnls.ctas_per_sm");
-    b->first_smem = nnls_smem_bytes(b->c_hr_max, 32) * kMtWarps;
-    b->first_slots = resident_slots(batch_first_kernel, b->first_smem, V, "sd.nnls.ctas_per_sm");
     b->hr_smem = nnls_smem_bytes(b->c_hr_max, kCholCap) * kMtWarps;
     b->hr_slots = resident_slots(batch_redo_kernel<kCholCap / 32, 10, true>, b->hr_smem, V, "sd.nnls.ctas_per_sm");
     b->lf_slots = resident_slots(batch_lr_fractions_kernel, 0, V, "sd.fractions.ctas_per_sm");
     b->hf_slots = resident_slots(batch_hr_fractions_kernel, 0, V, "sd.fractions.ctas_per_sm");
     b->lr_slot = nnls_slot_doubles(mi, 32);
-    b->first_slot = nnls_slot_doubles(mi, 32);
     b->hr_slot = nnls_slot_doubles(mi, kCholCap);
     b->lf_slot = frac_slot_doubles(mi, b->c_lr_max, 1 + ci);
     b->hf_slot = frac_slot_doubles(mi, b->c_hr_max, b->nf_max);
-    const size_t slot_doubles = std::max(
-        {size_t(2 * b->half_warps) * half_slot_doubles(), size_t(b->lr_slots) * b->lr_slot,
-         size_t(b->first_slots) * b->first_slot, size_t(b->hr_slots) * b->hr_slot, size_t(b->lf_slots) * b->lf_slot,
-         size_t(b->hf_slots) * b->hf_slot});
+    const size_t slot_doubles =
+        std::max({size_t(b->lr_slots) * b->lr_slot, size_t(b->hr_slots) * b->hr_slot,
+                  size_t(b->lf_slots) * b->lf_slot, size_t(b->hf_slots) * b->hf_slot});
     auto carve_all = [&](Carver& cv) {
         MfodBatchState s{};
         s.jobs = b->d_jobs.ptr;
@@ -1805,6 +1650,7 @@ void mfod_batch_finalize(MfodBatch* b) {
         s.bad = cv.take<uint8_t>(size_t(V));
         s.vfirst = cv.take<int64_t>(size_t(nj) + 1);
         s.tfirst = cv.take<int64_t>(size_t(nj) + 1);
+        s.qfirst = cv.take<int64_t>(size_t(nj) + 1);
         s.redo = cv.take<int64_t>(size_t(V));
         s.redo_count = cv.take<int>(1);
         b->list[0] = cv.take<int>(size_t(V));
@@ -1827,8 +1673,8 @@ void mfod_batch_run(MfodBatch* b, cudaStream_t st) {
     const MfodBatchState& B = b->B;
     const int64_t V = b->voxels, nj = int64_t(b->jobs.size());
     const int ci = b->ci;
-    auto blocks = [](int64_t slots, int64_t count) {
-        return unsigned(std::max<int64_t>(1, std::min<int64_t>(slots / kMtWarps, (count + kMtWarps - 1) / kMtWarps)));
+    auto blocks = [](int64_t slots, int64_t count, int warps = kMtWarps) {
+        return unsigned(std::max<int64_t>(1, std::min<int64_t>(slots / warps, (count + warps - 1) / warps)));
     };
     auto zero = [&](void* p, size_t bytes) { cuda_check(cudaMemsetAsync(p, 0, bytes, st), "cudaMemsetAsync"); };
     auto launched = [](const char* what) { cuda_check(cudaGetLastError(), what); };
@@ -1861,10 +1707,9 @@ void mfod_batch_run(MfodBatch* b, cudaStream_t st) {
         zero(nxt_counts, size_t(nj) * sizeof(int));
         zero(B.redo_count, sizeof(int));
         {
-            LaunchScope scope("batch_half_kernel<3>", st);
-            batch_half_kernel<3><<<blocks(b->half_warps, (V + 1) / 2), kMtWarps * 32, b->half_smem, st>>>(
-                B, cur, b->c_lr_max, b->queue, b->slots, half_slot_doubles());
-            launched("batch_half_kernel launch");
+            LaunchScope scope("batch_low_kernel", st);
+            batch_low_kernel<<<blocks(b->low_slots, V, kLowWarps), kLowWarps * 32, b->low_smem, st>>>(B, cur, b->queue);
+            launched("batch_low_kernel launch");
         }
         zero(b->queue, sizeof(int));
         {
@@ -1898,10 +1743,9 @@ void mfod_batch_run(MfodBatch* b, cudaStream_t st) {
     zero(b->queue, sizeof(int));
     zero(B.redo_count, sizeof(int));
     {
-        LaunchScope scope("batch_first_kernel<1,10>", st);
-        batch_first_kernel<<<blocks(b->first_slots, V), kMtWarps * 32, b->first_smem, st>>>(
-            B, b->c_hr_max, b->queue, b->slots, b->first_slot);
-        launched("batch_first_kernel launch");
+        LaunchScope scope("batch_high_kernel", st);
+        batch_high_kernel<<<blocks(b->high_slots, V, kHighWarps), kHighWarps * 32, high_smem_bytes(), st>>>(B, b->queue);
+        launched("batch_high_kernel launch");
     }
     zero(b->queue, sizeof(int));
     {
