@@ -93,6 +93,121 @@ struct SignalDev {
 __device__ __forceinline__ int64_t listed(const int* list, int64_t p) { return list ? int64_t(list[p]) : p; }
 
 // ---- correlations ----------------------------------------------------------------------
+//
+// The product of the signals and K on the FP64 tensor cores (mma.sync m8n8k4): a CTA keeps 48 columns
+// of K for every measurement in shared memory (127 KB at 280), and a warp takes eight voxels, whose
+// signals go straight from global memory into its A fragments (four consecutive samples of a voxel
+// per step, a sector each; 32 samples ahead in registers) with the weights and the isotropic part
+// applied on the way. What bounds it: the tensor cores (13.4 kFMA per voxel and 44 columns). The
+// CUDA-core tiles below re-staged 16 measurements at a time behind two barriers and their loads'
+// latency: CORR_FIGURES They take what does not fit here (corr_tc_fits).
+
+constexpr int kCorrTcCols = 48, kCorrTcWarps = 16, kCorrTcLd = 52;  // 4 mod 16 doubles
+constexpr int kCorrTcMaxIso = 3, kCorrTcUnit = 8;
+constexpr int kCorrTcTicket = kCorrTcUnit * kCorrTcWarps;  // voxels of a batch's ticket
+__host__ __device__ inline int corr_tc_rows(int m) { return (m + 31) / 32 * 32; }
+__host__ __device__ inline size_t corr_tc_smem(int m, int ci) {
+    return size_t(corr_tc_rows(m)) * (kCorrTcLd + 1 + ci) * sizeof(double);
+}
+__host__ __device__ inline bool corr_tc_fits(int m, int ci) {
+    return ci <= kCorrTcMaxIso && corr_tc_smem(m, ci) <= 227 * 1024;
+}
+
+__device__ __forceinline__ void corr_mma(double (&d)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(d[0]), "+d"(d[1])
+                 : "d"(a), "d"(b));
+}
+
+// Columns col0.. of K, the weights and W_iso into shared memory, zero past the last measurement and
+// column (the CTA; the caller synchronises).
+__device__ __forceinline__ void corr_tc_stage(double* sm, const SignalDev& S, const double* __restrict__ k, int c,
+                                              int col0) {
+    const int m = S.m, rows = corr_tc_rows(m);
+    for (int e = threadIdx.x; e < rows * kCorrTcCols; e += blockDim.x) {
+        const int i = e / kCorrTcCols, j = e % kCorrTcCols;
+        sm[i * kCorrTcLd + j] = i < m && col0 + j < c ? k[size_t(i) * c + col0 + j] : 0.0;
+    }
+    double* ws = sm + size_t(rows) * kCorrTcLd;
+    for (int i = threadIdx.x; i < rows; i += blockDim.x) ws[i] = i < m && S.w ? S.w[i] : 1.0;
+    for (int i = threadIdx.x; i < rows * S.ci; i += blockDim.x) ws[rows + i] = i < m * S.ci ? S.wiso[i] : 0.0;
+}
+
+// A warp's eight voxels (voxel: the lane's, lane / 4 of the eight; -1: none) against the staged columns.
+// CI isotropic tissues; CI < 0: the plain signal.
+template <int CI>
+__device__ __forceinline__ void corr_tc_unit(const double* sm, const SignalDev& S, int64_t voxel, int c, int col0,
+                                             double* __restrict__ corr, int ldc, int lane) {
+    const int m = S.m, rows = corr_tc_rows(m), l = lane & 3, v = lane >> 2;
+    const double* ws = sm + size_t(rows) * kCorrTcLd;
+    const double* wi = ws + rows;
+    const double* s = S.s + (voxel < 0 ? 0 : voxel) * m;
+    double f[CI > 0 ? CI : 1];
+#pragma unroll
+    for (int t = 0; t < CI; ++t) f[t] = voxel < 0 ? 0.0 : S.fiso[voxel * CI + t];
+    double acc[6][2];
+#pragma unroll
+    for (int t = 0; t < 6; ++t) acc[t][0] = acc[t][1] = 0.0;
+    double ahead[8];
+    auto load = [&](int i0) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int i = i0 + 4 * q + l;
+            ahead[q] = voxel >= 0 && i < m ? s[i] : 0.0;
+        }
+    };
+    load(0);
+    for (int i0 = 0; i0 < m; i0 += 32) {
+        double raw[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) raw[q] = ahead[q];
+        if (i0 + 32 < m) load(i0 + 32);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int i = i0 + 4 * q + l;
+            double a = raw[q];
+            if constexpr (CI >= 0) {
+                // max(s w - W_iso f_iso, 0) (SignalDev); rows past m have no columns.
+                const double weighted = __dmul_rn(a, ws[i]);
+                double r = 0.0;
+#pragma unroll
+                for (int t = 0; t < CI; ++t) r = fma(wi[i * CI + t], f[t], r);
+                a = fmax(weighted - r, 0.0);
+            }
+            const double* kr = sm + i * kCorrTcLd + v;
+#pragma unroll
+            for (int t = 0; t < 6; ++t) corr_mma(acc[t], a, kr[8 * t]);
+        }
+    }
+    if (voxel < 0) return;
+    double* out = corr + voxel * ldc + col0;
+#pragma unroll
+    for (int t = 0; t < 6; ++t)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int j = 8 * t + 2 * l + h;
+            if (col0 + j < c) out[j] = acc[t][h];
+        }
+}
+
+// corr(v, j) of the listed voxels, columns 48 blockIdx.y on: the units of eight voxels dealt to the CTAs
+// first, so that a short list spreads over the SMs.
+template <int CI>
+__global__ void __launch_bounds__(kCorrTcWarps * 32, 1) correlate_tc_kernel(
+    SignalDev S, const int* __restrict__ list, int64_t count, const int* __restrict__ count_dev,
+    const double* __restrict__ k, int c, double* __restrict__ corr, int ldc) {
+    if (count_dev) count = min(count, int64_t(*count_dev));
+    if (count <= int64_t(blockIdx.x) * kCorrTcUnit) return;
+    extern __shared__ __align__(16) double csm[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col0 = blockIdx.y * kCorrTcCols;
+    corr_tc_stage(csm, S, k, c, col0);
+    __syncthreads();
+    for (int64_t p0 = (blockIdx.x + int64_t(gridDim.x) * warp) * kCorrTcUnit; p0 < count;
+         p0 += int64_t(gridDim.x) * kCorrTcWarps * kCorrTcUnit) {
+        const int64_t p = p0 + (lane >> 2);
+        corr_tc_unit<CI>(csm, S, p < count ? listed(list, p) : -1, c, col0, corr, ldc, lane);
+    }
+}
 
 constexpr int kCorrVoxels = 32;  // voxels per CTA tile
 constexpr int kCorrResidentCtas = 8;  // CTAs per SM of a correlation grid whose count is on the device
@@ -915,6 +1030,7 @@ struct MfodBatchState {
     int64_t* vfirst;   // (n_jobs + 1) this stage's first voxel ticket per volume
     int64_t* tfirst;   // (n_jobs + 1) its first correlation tile per volume
     int64_t* qfirst;   // (n_jobs + 1) its first ticket of kLowTicket voxels per volume
+    int64_t* cfirst;   // (n_jobs + 1) its first ticket of kCorrTcTicket voxels per volume
     int64_t* redo;     // volume << 32 | voxel, for the one-warp NNLS
     int* redo_count;
 };
@@ -939,22 +1055,26 @@ __device__ __forceinline__ SignalDev batch_signal(const MfodBatchState& B, const
 // The tickets of a stage from each volume's count (null: every voxel).
 __global__ void batch_plan_kernel(MfodBatchState B, const int* __restrict__ counts) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    int64_t a = 0, b = 0, q = 0;
+    int64_t a = 0, b = 0, q = 0, e = 0;
     for (int j = 0; j < B.n_jobs; ++j) {
         B.vfirst[j] = a;
         B.tfirst[j] = b;
         B.qfirst[j] = q;
+        B.cfirst[j] = e;
         const int64_t c = counts ? int64_t(counts[j]) : B.jobs[j].v;
         a += c;
         b += (c + kCorrVoxels - 1) / kCorrVoxels;
         q += (c + kLowTicket - 1) / kLowTicket;
+        e += (c + kCorrTcTicket - 1) / kCorrTcTicket;
     }
     B.vfirst[B.n_jobs] = a;
     B.tfirst[B.n_jobs] = b;
     B.qfirst[B.n_jobs] = q;
+    B.cfirst[B.n_jobs] = e;
 }
 
-// correlate_kernel over every volume: a CTA per (volume, tile of kCorrVoxels listed voxels).
+// correlate_kernel over the volumes that do not fit correlate_tc_kernel: a CTA per (volume, tile of
+// kCorrVoxels listed voxels).
 template <int RC, bool HR>
 __global__ void __launch_bounds__(128) batch_correlate_kernel(MfodBatchState B, const int* __restrict__ list) {
     __shared__ int64_t vox[kCorrVoxels];
@@ -963,6 +1083,8 @@ __global__ void __launch_bounds__(128) batch_correlate_kernel(MfodBatchState B, 
     for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
         const int j = ticket_job(B.tfirst, B.n_jobs, t);
         const MfodBatchJob& J = B.jobs[j];
+        const RidgeDev R = HR ? J.hr : J.lr;
+        if (corr_tc_fits(R.m, B.ci)) continue;
         const int64_t count = B.vfirst[j + 1] - B.vfirst[j];
         const int64_t p0 = (t - B.tfirst[j]) * kCorrVoxels;
         __syncthreads();  // the previous tile's voxels are read
@@ -971,10 +1093,37 @@ __global__ void __launch_bounds__(128) batch_correlate_kernel(MfodBatchState B, 
             vox[tid] = q < count ? (list ? int64_t(list[J.off + q]) : q) : -1;
         }
         __syncthreads();
-        const RidgeDev R = HR ? J.hr : J.lr;
         const TissueDev T = HR ? J.hrt : J.lrt;
         correlate_tile<RC>(batch_signal(B, J, T), vox, R.k, R.c, blockIdx.y * 16 * RC, B.corr + J.off * B.ldc,
                            B.ldc);
+    }
+}
+
+// correlate_tc_kernel over every volume: a CTA takes a ticket of kCorrTcTicket listed voxels, eight to
+// a warp, and restages when its ticket moves to another volume.
+template <int CI, bool HR>
+__global__ void __launch_bounds__(kCorrTcWarps * 32, 1) batch_correlate_tc_kernel(MfodBatchState B,
+                                                                                 const int* __restrict__ list) {
+    extern __shared__ __align__(16) double csm[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col0 = blockIdx.y * kCorrTcCols;
+    const int64_t total = B.cfirst[B.n_jobs];
+    int cur = -1;
+    for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
+        const int j = ticket_job(B.cfirst, B.n_jobs, t);
+        const MfodBatchJob& J = B.jobs[j];
+        const RidgeDev R = HR ? J.hr : J.lr;
+        if (!corr_tc_fits(R.m, CI) || col0 >= R.c) continue;
+        const SignalDev S = batch_signal(B, J, HR ? J.hrt : J.lrt);
+        if (j != cur) {
+            __syncthreads();
+            corr_tc_stage(csm, S, R.k, R.c, col0);
+            cur = j;
+            __syncthreads();
+        }
+        const int64_t p = (t - B.cfirst[j]) * kCorrTcTicket + warp * kCorrTcUnit + (lane >> 2);
+        const int64_t count = B.vfirst[j + 1] - B.vfirst[j];
+        const int64_t voxel = p < count ? (list ? int64_t(list[J.off + p]) : p) : -1;
+        corr_tc_unit<CI>(csm, S, voxel, R.c, col0, B.corr + J.off * B.ldc, B.ldc, lane);
     }
 }
 
@@ -1193,6 +1342,25 @@ inline NnlsLaunch nnls_variant(int c) {
 inline void launch_correlate(const SignalDev& S, const int* list, int64_t count, const int* count_dev,
                              const RidgeDev& R, double* corr, int ldc, cudaStream_t st) {
     if (count == 0) return;
+    if (corr_tc_fits(R.m, S.w ? S.ci : 0)) {
+        const unsigned gy = unsigned((R.c + kCorrTcCols - 1) / kCorrTcCols);
+        const int64_t units = (count + kCorrTcUnit - 1) / kCorrTcUnit;
+        const unsigned gx = unsigned(std::max<int64_t>(1, std::min<int64_t>(units, sm_count() / gy)));
+        const size_t smem = corr_tc_smem(R.m, S.w ? S.ci : 0);
+        auto run = [&](auto kernel) {
+            cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
+                       "cudaFuncSetAttribute");
+            LaunchScope scope("correlate_kernel", st);
+            kernel<<<dim3(gx, gy), kCorrTcWarps * 32, smem, st>>>(S, list, count, count_dev, R.k, R.c, corr, ldc);
+            cuda_check(cudaGetLastError(), "correlate_tc_kernel launch");
+        };
+        if (S.w == nullptr) run(correlate_tc_kernel<-1>);
+        else if (S.ci == 0) run(correlate_tc_kernel<0>);
+        else if (S.ci == 1) run(correlate_tc_kernel<1>);
+        else if (S.ci == 2) run(correlate_tc_kernel<2>);
+        else run(correlate_tc_kernel<3>);
+        return;
+    }
     // count is exact unless the round's count lives on the device (count_dev): then it is an
     // upper bound and the grid stays resident-sized, the CTAs striding over the live tiles.
     int64_t tiles = (count + kCorrVoxels - 1) / kCorrVoxels;
@@ -1550,6 +1718,36 @@ struct MfodBatch {
     ~MfodBatch() {
         if (scratch) cudaFree(scratch);
     }
+    int tc_m = 0;         // the most measurements of the volumes the tensor-core correlations take
+    bool tc_all = true;   // they take every volume
+    // A stage's correlations: the tensor-core kernel's volumes, then the others.
+    template <bool HR>
+    void correlate(const int* list, unsigned grid, cudaStream_t st) {
+        const int c_max = HR ? c_hr_max : c_lr_max;
+        if (tc_m > 0) {
+            const size_t smem = corr_tc_smem(tc_m, ci);
+            const unsigned gy = unsigned((c_max + kCorrTcCols - 1) / kCorrTcCols);
+            const unsigned gx = std::max(1u, unsigned(sm_count()) / gy);
+            auto run = [&](auto kernel) {
+                cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
+                           "cudaFuncSetAttribute");
+                LaunchScope scope("batch_correlate_kernel", st);
+                kernel<<<dim3(gx, gy), kCorrTcWarps * 32, smem, st>>>(B, list);
+                cuda_check(cudaGetLastError(), "batch_correlate_tc_kernel launch");
+            };
+            if (ci == 0) run(batch_correlate_tc_kernel<0, HR>);
+            else if (ci == 1) run(batch_correlate_tc_kernel<1, HR>);
+            else if (ci == 2) run(batch_correlate_tc_kernel<2, HR>);
+            else run(batch_correlate_tc_kernel<3, HR>);
+        }
+        if (tc_all) return;
+        LaunchScope scope("batch_correlate_kernel", st);
+        if constexpr (HR)
+            batch_correlate_kernel<4, true><<<dim3(grid, unsigned((c_max + 63) / 64)), 128, 0, st>>>(B, list);
+        else
+            batch_correlate_kernel<3, false><<<grid, 128, 0, st>>>(B, list);
+        cuda_check(cudaGetLastError(), "batch_correlate_kernel launch");
+    }
 };
 
 MfodBatch* mfod_batch_create() { return new MfodBatch(); }
@@ -1602,6 +1800,8 @@ void mfod_batch_add(MfodBatch* b, const double* signals, int64_t v, const double
     b->voxels += v;
     b->tiles += (v + kCorrVoxels - 1) / kCorrVoxels;
     b->m_max = std::max(b->m_max, int(m));
+    if (corr_tc_fits(int(m), int(lr->ci))) b->tc_m = std::max(b->tc_m, int(m));
+    else b->tc_all = false;
     b->c_lr_max = std::max(b->c_lr_max, int(lr->ca));
     b->c_hr_max = std::max(b->c_hr_max, int(hr->ca));
     b->nf_max = std::max(b->nf_max, int(hr->nb + hr->ci));
@@ -1651,6 +1851,7 @@ void mfod_batch_finalize(MfodBatch* b) {
         s.vfirst = cv.take<int64_t>(size_t(nj) + 1);
         s.tfirst = cv.take<int64_t>(size_t(nj) + 1);
         s.qfirst = cv.take<int64_t>(size_t(nj) + 1);
+        s.cfirst = cv.take<int64_t>(size_t(nj) + 1);
         s.redo = cv.take<int64_t>(size_t(V));
         s.redo_count = cv.take<int>(1);
         b->list[0] = cv.take<int>(size_t(V));
@@ -1698,11 +1899,7 @@ void mfod_batch_run(MfodBatch* b, cudaStream_t st) {
             batch_plan_kernel<<<1, 32, 0, st>>>(B, cur_counts);
             launched("batch_plan_kernel launch");
         }
-        {
-            LaunchScope scope("batch_correlate_kernel", st);
-            batch_correlate_kernel<3, false><<<corr_grid, 128, 0, st>>>(B, cur);
-            launched("batch_correlate_kernel launch");
-        }
+        b->correlate<false>(cur, corr_grid, st);
         zero(b->queue, sizeof(int));
         zero(nxt_counts, size_t(nj) * sizeof(int));
         zero(B.redo_count, sizeof(int));
@@ -1734,12 +1931,7 @@ void mfod_batch_run(MfodBatch* b, cudaStream_t st) {
         batch_plan_kernel<<<1, 32, 0, st>>>(B, nullptr);
         launched("batch_plan_kernel launch");
     }
-    {
-        LaunchScope scope("batch_correlate_kernel", st);
-        batch_correlate_kernel<4, true><<<dim3(corr_grid, unsigned((b->c_hr_max + 63) / 64)), 128, 0, st>>>(
-            B, nullptr);
-        launched("batch_correlate_kernel launch");
-    }
+    b->correlate<true>(nullptr, corr_grid, st);
     zero(b->queue, sizeof(int));
     zero(B.redo_count, sizeof(int));
     {
