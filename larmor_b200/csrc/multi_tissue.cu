@@ -69,6 +69,9 @@ struct TissueDev {
     const double* iso;   // (m, ci)
     const double* wiso;  // (m, ci)
     const int* blocks;   // (nb, 2)
+    // The constants of the lane-per-voxel fractions (FracConstants), or null where they do not apply.
+    const double* fx;
+    int fx_rows;
 };
 
 // The signal a ridge NNLS fits, entry i of voxel v: s(v, i) itself (single tissue), or
@@ -100,7 +103,8 @@ __device__ __forceinline__ int64_t listed(const int* list, int64_t p) { return l
 // per step, a sector each; 32 samples ahead in registers) with the weights and the isotropic part
 // applied on the way. What bounds it: the tensor cores (13.4 kFMA per voxel and 44 columns). The
 // CUDA-core tiles below re-staged 16 measurements at a time behind two barriers and their loads'
-// latency: CORR_FIGURES They take what does not fit here (corr_tc_fits).
+// latency: 16.9 ms for the ten rounds and the high-resolution pass of 250,000 voxels, now 5.6 ms (3.9
+// and 1.2 ms for 8,191 voxels). They take what does not fit here (corr_tc_fits).
 
 constexpr int kCorrTcCols = 48, kCorrTcWarps = 16, kCorrTcLd = 52;  // 4 mod 16 doubles
 constexpr int kCorrTcMaxIso = 3, kCorrTcUnit = 8;
@@ -648,12 +652,23 @@ struct FracState {
     int fperm[kMaxGroups];
     double fr[kMaxGroups];
     double med[2];
+    uint16_t idx[kMaxColumns];  // the columns above the threshold, increasing
 };
 
-// Median of v[0..n), the mean of the two middle values for even n (cpp/src/sd/fractions.cpp:56-68),
-// by ranks: the element of stable rank r is the r-th smallest.
+// Median of v[0..n), the mean of the two middle values for even n (cpp/src/sd/fractions.cpp:56-68). A
+// non-negative vector with more zeros than half, as an NNLS solution is, has median 0; else by
+// ranks: the element of stable rank r is the r-th smallest (300 x 300 comparisons at high
+// resolution).
 __device__ __forceinline__ double warp_median(const double* v, int n, FracState& st, int lane) {
     const int hi = n / 2, lo = n % 2 ? n / 2 : n / 2 - 1;
+    int zeros = 0;
+    bool odd = false;
+    for (int i = lane; i < n; i += 32) {
+        zeros += v[i] == 0.0;
+        odd |= !(v[i] >= 0.0);
+    }
+    zeros = __reduce_add_sync(0xffffffffu, zeros);
+    if (!__any_sync(0xffffffffu, odd) && zeros > hi) return 0.0;
     for (int i = lane; i < n; i += 32) {
         const double vi = v[i];
         int rank = 0;
@@ -780,18 +795,28 @@ __device__ __forceinline__ bool small_nnls(const double (&G)[4][4], const double
 }
 
 // compute_fractions for one anisotropic column next to at most three isotropic ones and at most
-// 320 measurements: the column K th scaled to a maximum of 1 in registers, then C^T C, C^T s and
-// the columns' norm1 in one reduction, and the NNLS on those (small_nnls). False when that
-// needs the QR fit.
-__device__ __forceinline__ bool fractions_small(const TissueDev T, const double* sig, int gb, int ge, double tol,
-                                                const FracSlot sl, FracState& st, int lane) {
+// 320 measurements: the column K th scaled to a maximum of 1 in registers (over the columns listed
+// first, above the threshold), then C^T C, C^T s and the columns' norm1 in one reduction, and the NNLS
+// on those (small_nnls). False when that needs the QR fit.
+__device__ __forceinline__ bool fractions_small(const TissueDev T, const double* fod, const double* sig, int gb, int ge,
+                                                double threshold, double tol, FracState& st, int lane) {
     const int m = T.m, ci = T.ci, n = 1 + ci;
+    int kept = 0;
+    for (int j0 = gb; j0 < ge; j0 += 32) {
+        const int j = j0 + lane;
+        const double f = j < ge ? fod[j] : 0.0;
+        const bool in = j < ge && !(f < threshold) && f != 0.0;
+        const unsigned b = __ballot_sync(0xffffffffu, in);
+        if (in) st.idx[kept + __popc(b & ((1u << lane) - 1u))] = uint16_t(j);
+        kept += __popc(b);
+    }
+    __syncwarp();
     double col[kFastRowsPerLane];
 #pragma unroll
     for (int t = 0; t < kFastRowsPerLane; ++t) col[t] = 0.0;
-    for (int j = gb; j < ge; ++j) {
-        const double tj = sl.th[j];
-        if (tj == 0.0) continue;
+    for (int q = 0; q < kept; ++q) {
+        const int j = st.idx[q];
+        const double tj = fod[j];
         const double* kr = T.kt + size_t(j) * m;
 #pragma unroll
         for (int t = 0; t < kFastRowsPerLane; ++t) {
@@ -882,14 +907,14 @@ __device__ __forceinline__ void fractions(const TissueDev T, const double* fod, 
                                           double tol, const FracSlot sl, FracState& st, int lane) {
     const int m = T.m, ca = T.ca, ci = T.ci;
     const double threshold = warp_median(fod, ca, st, lane) * (1.0 - kMedianTie);
-    for (int j = lane; j < ca; j += 32) sl.th[j] = fod[j] < threshold ? 0.0 : fod[j];
-    __syncwarp();
     const int ng = per_block ? T.nb : 1;
     const int ncol = ng + ci;
     if (ng == 1 && ci <= 3 && m <= 32 * kFastRowsPerLane) {
         const int gb = per_block ? T.blocks[0] : 0, ge = per_block ? T.blocks[1] : ca;
-        if (fractions_small(T, sig, gb, ge, tol, sl, st, lane)) return;
+        if (fractions_small(T, fod, sig, gb, ge, threshold, tol, st, lane)) return;
     }
+    for (int j = lane; j < ca; j += 32) sl.th[j] = fod[j] < threshold ? 0.0 : fod[j];
+    __syncwarp();
     double colmax = 0.0;
     for (int g = 0; g < ng; ++g) {
         const int b = per_block ? T.blocks[2 * g] : 0, e = per_block ? T.blocks[2 * g + 1] : ca;
@@ -934,6 +959,200 @@ __device__ __forceinline__ void fractions(const TissueDev T, const double* fod, 
     warp_nnls_explicit(sl.cols, m, ncol, sig, tol, 3 * ncol, ns, lane);
     for (int g = lane; g < ncol; g += 32) st.fr[g] = sl.fu[g];
     __syncwarp();
+}
+
+// ---- fractions, a lane per voxel (low-resolution NNLS solutions) ----------------------------------
+//
+// A round's fractions need of the column K th only its maximum, its sum and its products with itself,
+// the isotropic columns and the signal. A non-negative K gives all but the first from small
+// constants, (th, K^T K th), (K^T iso)^T th and (K^T s)^T th, sums of non-negative terms; K^T s and
+// iso^T s do not change over the rounds and are taken once per fit. The maximum needs only the rows of K
+// that no other row bounds entry by entry (with a b0 among the measurements, that one row), and is
+// the same number, as the order of a row's sum is. Solutions have ~8 of 44 entries, so their median is 0 (else,
+// or for values that are not finite and non-negative, the warp takes the voxel by the general way).
+// So a voxel is ~200 FMAs on one lane, where a warp ranked 44 entries, built 280 rows and reduced
+// 18 sums: 28.1 ms for ten
+// rounds of 250,000 voxels, 2.0 ms for 8,191; now 3.4 and 1.9 ms (the latency of a lane's chain)
+
+constexpr int kFracCols = 48, kFracRows = 16, kFracList = 24, kFracWarps = 4;
+static_assert(kFracList >= kFracCols - kFracCols / 2 - 1, "the list holds every solution with median 0");
+
+// The constants of one kernel, packed: K^T K (c, c), K^T iso (c, ci), the column sums (c), the rows
+// that can hold the maximum (rows, c), iso^T iso (ci, ci), the isotropic columns' absolute sums (ci).
+struct FracConstants {
+    const double *gram, *ki, *ksum, *top, *ii, *isum;
+    __host__ __device__ FracConstants(const double* p, int c, int ci, int rows) {
+        gram = p;
+        ki = gram + c * c;
+        ksum = ki + c * ci;
+        top = ksum + c;
+        ii = top + rows * c;
+        isum = ii + ci * ci;
+    }
+    __host__ __device__ static int doubles(int c, int ci, int rows) {
+        return c * c + c * ci + c + rows * c + ci * ci + ci;
+    }
+};
+
+inline size_t frac_lane_smem(int doubles) {
+    return size_t(doubles) * sizeof(double) + size_t(kFracWarps) * 32 * kFracList * (sizeof(double) + 1);
+}
+
+// The fractions u of the solution x (c) with ks = [K^T s, iso^T s]; false when the general way is needed.
+__device__ __forceinline__ bool lane_fractions(const FracConstants& F, int m, int c, int ci, int rows,
+                                               const double* __restrict__ x, const double* __restrict__ ks,
+                                               double* vals, uint8_t* cols, double (&u)[4]) {
+    // The lane's list: entry q at [32 q].
+    int n = 0;
+    bool odd = false;
+    for (int j0 = 0; j0 < c; j0 += 8) {
+        double some[8];  // loaded together: each is its own trip to L2
+#pragma unroll
+        for (int q = 0; q < 8; ++q) some[q] = j0 + q < c ? x[j0 + q] : 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const double v = some[q];
+            if (v == 0.0) continue;
+            odd |= !(v > 0.0 && v < INFINITY);
+            if (n < kFracList) {
+                vals[32 * n] = v;
+                cols[32 * n] = uint8_t(j0 + q);
+            }
+            ++n;
+        }
+    }
+    if (odd || c - n <= c / 2) return false;
+    double largest = -INFINITY;
+    for (int r = 0; r < rows; ++r) {
+        double s = 0.0;
+        for (int q = 0; q < n; ++q) s = fma(F.top[r * c + cols[32 * q]], vals[32 * q], s);
+        largest = fmax(largest, s);
+    }
+    double cc = 0.0, cs = 0.0, sum = 0.0, ct[3] = {0.0, 0.0, 0.0};
+#pragma unroll 4
+    for (int q = 0; q < n; ++q) cs = fma(vals[32 * q], ks[cols[32 * q]], cs);
+    for (int q = 0; q < n; ++q) {
+        const double v = vals[32 * q];
+        const int j = cols[32 * q];
+        const double* row = F.gram + j * c;
+        double s = 0.0;
+        for (int p = 0; p < q; ++p) s = fma(row[cols[32 * p]], vals[32 * p], s);
+        cc = fma(v, fma(2.0, s, row[j] * v), cc);
+        sum = fma(v, F.ksum[j], sum);
+#pragma unroll
+        for (int t = 0; t < 3; ++t)
+            if (t < ci) ct[t] = fma(v, F.ki[j * ci + t], ct[t]);
+    }
+    if (largest > 0.0) {
+        cc = cc / largest / largest;
+        cs /= largest;
+        sum /= largest;
+#pragma unroll
+        for (int t = 0; t < 3; ++t) ct[t] /= largest;
+    }
+    double G[4][4], b[4], norm1 = sum;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        b[a] = a == 0 ? cs : a <= ci ? ks[c + a - 1] : 0.0;
+        if (a > 0 && a <= ci) norm1 = fmax(norm1, F.isum[a - 1]);
+#pragma unroll
+        for (int d = 0; d < 4; ++d) {
+            if (a == 0 || d == 0)
+                G[a][d] = a + d == 0 ? cc : ct[a + d > 3 ? 2 : a + d - 1];
+            else
+                G[a][d] = a <= ci && d <= ci ? F.ii[(a - 1) * ci + d - 1] : 0.0;
+        }
+    }
+    return small_nnls(G, b, 1 + ci, 10.0 * kEps64 * norm1 * double(max(m, 1 + ci)), 3 * (1 + ci), u);
+}
+
+// A round's state of one volume, as the fraction kernels update it.
+struct FracRound {
+    const double* s;       // (v, m) signals
+    const double* x;       // (v, ldx) low-resolution solutions
+    const double* ks;      // (v, c + ci)
+    double *fiso, *prev;   // (v, ci), (v, ci + 1)
+    int32_t* rounds;
+    int* next;             // the next round's list and its count
+    int* next_count;
+    int ldx, round, max_rounds;
+    double tol;
+};
+
+// The general way, out of line: its registers stay out of the lane-per-voxel kernels.
+__device__ __noinline__ void fractions_by_warp(const TissueDev& T, const double* fod, const double* sig,
+                                               const FracSlot& sl, FracState& st, int lane) {
+    fractions(T, fod, sig, false, -1.0, sl, st, lane);
+}
+
+// One warp's voxels, one per lane (-1: none): fractions, the convergence test and the next list
+// (lr_fractions_kernel).
+__device__ __forceinline__ void lane_fractions_unit(const TissueDev& T, const FracConstants& F, const FracRound& R,
+                                                    int64_t voxel, double* vals, uint8_t* cols, const FracSlot& sl,
+                                                    FracState& st, int lane) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int c = T.ca, ci = T.ci;
+    double u[4] = {0.0, 0.0, 0.0, 0.0};
+    bool ok = true;
+    if (voxel >= 0)
+        ok = lane_fractions(F, T.m, c, ci, T.fx_rows, R.x + voxel * R.ldx, R.ks + voxel * (c + ci), vals, cols, u);
+    __syncwarp();
+    for (unsigned left = __ballot_sync(kAll, !ok); left; left &= left - 1u) {
+        const int who = __ffs(left) - 1;
+        const int64_t w = __shfl_sync(kAll, voxel, who);
+        fractions_by_warp(T, R.x + w * R.ldx, R.s + w * T.m, sl, st, lane);
+        if (lane == who) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) u[j] = j <= ci ? st.fr[j] : 0.0;
+        }
+        __syncwarp();
+    }
+    bool goes_on = false;
+    if (voxel >= 0) {
+        // The first round has nothing to compare with (its previous fractions are infinite).
+        bool converged = R.round > 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (j > ci) continue;
+            double& before = R.prev[voxel * (ci + 1) + j];
+            if (R.round > 0) converged &= fabs(u[j] - before) < R.tol;
+            before = u[j];
+            if (j > 0) R.fiso[voxel * ci + j - 1] = u[j];
+        }
+        goes_on = !converged && R.round + 1 < R.max_rounds;
+        if (!goes_on) R.rounds[voxel] = R.round + 1;
+    }
+    const unsigned on = __ballot_sync(kAll, goes_on);
+    if (on) {
+        int base = 0;
+        if (lane == 0) base = atomicAdd(R.next_count, __popc(on));
+        base = __shfl_sync(kAll, base, 0);
+        if (goes_on) R.next[base + __popc(on & ((1u << lane) - 1u))] = int(voxel);
+    }
+    __syncwarp();
+}
+
+__global__ void __launch_bounds__(kFracWarps * 32) lane_fractions_kernel(
+    TissueDev T, FracRound R, const int* __restrict__ list, int64_t count, const int* __restrict__ count_dev,
+    double* __restrict__ workspace, size_t slot_size) {
+    if (count_dev) count = min(count, int64_t(*count_dev));
+    if (count <= int64_t(blockIdx.x) * 32) return;
+    extern __shared__ __align__(16) double fsm[];
+    __shared__ FracState states[kFracWarps];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n = FracConstants::doubles(T.ca, T.ci, T.fx_rows);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) fsm[i] = T.fx[i];
+    __syncthreads();
+    const FracConstants F(fsm, T.ca, T.ci, T.fx_rows);
+    double* vals = fsm + n + warp * 32 * kFracList + lane;
+    uint8_t* cols = reinterpret_cast<uint8_t*>(fsm + n + kFracWarps * 32 * kFracList) + warp * 32 * kFracList + lane;
+    const FracSlot sl =
+        carve_frac(workspace + (size_t(blockIdx.x) * kFracWarps + warp) * slot_size, T.m, T.ca, 1 + T.ci);
+    // Units of 32 voxels dealt to the CTAs first.
+    for (int64_t p0 = (blockIdx.x + int64_t(gridDim.x) * warp) * 32; p0 < count;
+         p0 += int64_t(gridDim.x) * kFracWarps * 32)
+        lane_fractions_unit(T, F, R, p0 + lane < count ? listed(list, p0 + lane) : -1, vals, cols, sl, states[warp],
+                            lane);
 }
 
 // One round's fractions of the listed voxels (cpp/src/sd/multi_tissue.cpp:100-125): f_iso(v)
@@ -1014,6 +1233,8 @@ struct MfodBatchJob {
     TissueDev lrt, hrt;
     const double* s;   // (v, m) S0-normalised signals
     const double* w;   // (m,) shell weights
+    const double* kx;  // [K, iso] of the low-resolution kernel, unweighted (m, ca + ci), where lrt.fx is set
+    int64_t ks_off;    // its first double in the batch's ks
     double* fods;      // (v, hr.c)
     double* fractions; // (v, hrt.nb + hrt.ci)
     int32_t* rounds;   // (v,) or null
@@ -1024,7 +1245,7 @@ struct MfodBatchJob {
 struct MfodBatchState {
     const MfodBatchJob* jobs;
     int n_jobs, ci, ldc, ldx;  // isotropic tissues; row strides of corr and of the low-resolution FODs
-    double *fiso, *prev, *corr, *xlr;
+    double *fiso, *prev, *corr, *xlr, *ks;
     int32_t* rounds;
     uint8_t* bad;
     int64_t* vfirst;   // (n_jobs + 1) this stage's first voxel ticket per volume
@@ -1225,6 +1446,69 @@ __global__ void __launch_bounds__(kHighWarps * 32, kHighCtas) batch_high_kernel(
     }
 }
 
+// [K^T s, iso^T s] of every voxel of the volumes whose fractions take a lane per voxel, once per fit.
+__global__ void __launch_bounds__(kCorrTcWarps * 32, 1) batch_ks_kernel(MfodBatchState B) {
+    extern __shared__ __align__(16) double csm[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col0 = blockIdx.y * kCorrTcCols;
+    const int64_t total = B.cfirst[B.n_jobs];
+    int cur = -1;
+    for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
+        const int j = ticket_job(B.cfirst, B.n_jobs, t);
+        const MfodBatchJob& J = B.jobs[j];
+        const int c = J.lrt.ca + J.lrt.ci;
+        if (J.lrt.fx == nullptr || col0 >= c) continue;
+        const SignalDev S{J.s, nullptr, nullptr, nullptr, J.lrt.m, 0};
+        if (j != cur) {
+            __syncthreads();
+            corr_tc_stage(csm, S, J.kx, c, col0);
+            cur = j;
+            __syncthreads();
+        }
+        const int64_t p = (t - B.cfirst[j]) * kCorrTcTicket + warp * kCorrTcUnit + (lane >> 2);
+        corr_tc_unit<-1>(csm, S, p < J.v ? p : -1, c, col0, B.ks + J.ks_off, c, lane);
+    }
+}
+
+// lane_fractions_kernel over those volumes' lists: a CTA takes a ticket of kLowTicket listed voxels.
+__global__ void __launch_bounds__(kFracWarps * 32) batch_lane_fractions_kernel(
+    MfodBatchState B, int doubles, const int* __restrict__ list, int round, int max_rounds, double fraction_tol,
+    int* __restrict__ next, int* next_counts, double* __restrict__ workspace, size_t slot_size) {
+    extern __shared__ __align__(16) double fsm[];
+    __shared__ FracState states[kFracWarps];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ci = B.ci;
+    double* vals = fsm + doubles + warp * 32 * kFracList + lane;
+    uint8_t* cols =
+        reinterpret_cast<uint8_t*>(fsm + doubles + kFracWarps * 32 * kFracList) + warp * 32 * kFracList + lane;
+    double* slot = workspace + (size_t(blockIdx.x) * kFracWarps + warp) * slot_size;
+    const int64_t total = B.qfirst[B.n_jobs];
+    int cur = -1;
+    for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
+        const int j = ticket_job(B.qfirst, B.n_jobs, t);
+        const MfodBatchJob& J = B.jobs[j];
+        const TissueDev T = J.lrt;
+        if (T.fx == nullptr) continue;
+        if (j != cur) {
+            __syncthreads();
+            const int n = FracConstants::doubles(T.ca, T.ci, T.fx_rows);
+            for (int i = threadIdx.x; i < n; i += blockDim.x) fsm[i] = T.fx[i];
+            cur = j;
+            __syncthreads();
+        }
+        const FracConstants F(fsm, T.ca, T.ci, T.fx_rows);
+        const FracSlot sl = carve_frac(slot, T.m, T.ca, 1 + ci);
+        const FracRound R{J.s, B.xlr + J.off * B.ldx, B.ks + J.ks_off, B.fiso + J.off * ci,
+                          B.prev + J.off * (ci + 1), B.rounds + J.off, next + J.off, next_counts + j, B.ldx, round,
+                          max_rounds, fraction_tol};
+        const int64_t p0 = (t - B.qfirst[j]) * kLowTicket;
+        const int64_t count = min(int64_t(kLowTicket), B.vfirst[j + 1] - B.vfirst[j] - p0);
+        for (int64_t q = warp * 32; q < count; q += kFracWarps * 32) {
+            const int64_t p = p0 + q + lane;
+            const int64_t voxel = q + lane < count ? (list ? int64_t(list[J.off + p]) : p) : -1;
+            lane_fractions_unit(T, F, R, voxel, vals, cols, sl, states[warp], lane);
+        }
+    }
+}
+
 // lr_fractions_kernel over every volume's list; the next round's list goes to each volume's
 // segment.
 __global__ void __launch_bounds__(kMtWarps * 32, 4) batch_lr_fractions_kernel(
@@ -1244,6 +1528,7 @@ __global__ void __launch_bounds__(kMtWarps * 32, 4) batch_lr_fractions_kernel(
         const BatchItem it = batch_item(B, list, p);
         const MfodBatchJob& J = B.jobs[it.job];
         const TissueDev T = J.lrt;
+        if (T.fx != nullptr) continue;  // batch_lane_fractions_kernel's
         const FracSlot sl = carve_frac(slot, T.m, T.ca, 1 + T.ci);
         const int64_t row = J.off + it.voxel;
         fractions(T, B.xlr + row * B.ldx, J.s + it.voxel * T.m, false, -1.0, sl, st, lane);
@@ -1469,12 +1754,66 @@ struct lar_deconv_kernel_s {
     lar::DeviceArray<double> kt, iso, wiso;
     lar::DeviceArray<float> kt32, iso32, wiso32;  // FP32 copies for the plain single-precision fit
     lar::DeviceArray<int> blocks;
+    // The lane-per-voxel fractions' constants and [K, iso] (m, ca + ci), where they apply.
+    lar::DeviceArray<double> fx, kx;
+    int fx_rows = 0;
     lar::TissueDev view() const {
-        return lar::TissueDev{int(m), int(ca), int(ci), int(nb), kt.ptr, iso.ptr, wiso.ptr, blocks.ptr};
+        return lar::TissueDev{int(m), int(ca), int(ci), int(nb), kt.ptr, iso.ptr, wiso.ptr, blocks.ptr, fx.ptr, fx_rows};
     }
 };
 
 using namespace lar;
+
+// The constants of a kernel's lane-per-voxel fractions (FracConstants) and its columns side by side;
+// left out for a kernel that is too wide, not finite and non-negative, or has many candidate rows.
+static void prepare_frac_constants(lar_deconv_kernel_s* h, const double* k, const double* iso) {
+    const int m = int(h->m), c = int(h->ca), ci = int(h->ci);
+    if (c > kFracCols || ci > 3 || !corr_tc_fits(m, 0)) return;
+    for (int64_t i = 0; i < int64_t(m) * c; ++i)
+        if (!(k[i] >= 0.0 && std::isfinite(k[i]))) return;
+    // The rows that no other row bounds.
+    std::vector<int> top;
+    for (int i = 0; i < m; ++i) {
+        auto bounds = [&](int a, int b) {  // row a >= row b everywhere
+            for (int j = 0; j < c; ++j)
+                if (k[size_t(a) * c + j] < k[size_t(b) * c + j]) return false;
+            return true;
+        };
+        bool out = false;
+        for (int t : top) out |= bounds(t, i);
+        if (out) continue;
+        top.erase(std::remove_if(top.begin(), top.end(), [&](int t) { return bounds(i, t); }), top.end());
+        top.push_back(i);
+        if (int(top.size()) > 4 * kFracRows) return;
+    }
+    if (int(top.size()) > kFracRows) return;
+    const int rows = int(top.size());
+    std::vector<double> p(size_t(FracConstants::doubles(c, ci, rows)), 0.0);
+    const FracConstants f(p.data(), c, ci, rows);
+    auto at = [&](const double* q, int i) -> double& { return p[size_t(q - p.data()) + size_t(i)]; };
+    for (int i = 0; i < m; ++i) {
+        const double* ki = k + size_t(i) * c;
+        for (int a = 0; a < c; ++a) {
+            for (int b = 0; b < c; ++b) at(f.gram, a * c + b) += ki[a] * ki[b];
+            for (int t = 0; t < ci; ++t) at(f.ki, a * ci + t) += ki[a] * iso[size_t(i) * ci + t];
+            at(f.ksum, a) += ki[a];
+        }
+        for (int t = 0; t < ci; ++t) {
+            for (int q = 0; q < ci; ++q) at(f.ii, t * ci + q) += iso[size_t(i) * ci + t] * iso[size_t(i) * ci + q];
+            at(f.isum, t) += std::fabs(iso[size_t(i) * ci + t]);
+        }
+    }
+    for (int r = 0; r < rows; ++r)
+        for (int j = 0; j < c; ++j) at(f.top, r * c + j) = k[size_t(top[size_t(r)]) * c + j];
+    h->fx.upload(p.data(), p.size());
+    h->fx_rows = rows;
+    std::vector<double> kx(size_t(m) * (c + ci));
+    for (int i = 0; i < m; ++i) {
+        for (int j = 0; j < c; ++j) kx[size_t(i) * (c + ci) + j] = k[size_t(i) * c + j];
+        for (int t = 0; t < ci; ++t) kx[size_t(i) * (c + ci) + c + t] = iso[size_t(i) * ci + t];
+    }
+    h->kx.upload(kx.data(), kx.size());
+}
 
 // The multi-tissue fit behind both entry points. device_rounds: enqueue every round with its
 // voxel count read on the device (as under stream capture) instead of reading each count back.
@@ -1516,7 +1855,11 @@ static int fit_multi_tissue(const double* signals, int64_t v, const double* weig
         // Voxels per pass: the per-voxel state of a pass (correlations, the low-resolution FOD,
         // f_iso and the previous fractions, two list entries, the round count and status) within
         // 4 GiB.
-        const size_t per_voxel = (size_t(std::max(c_lr, c_hr)) + size_t(c_lr) + 2 * size_t(ci) + 1) * sizeof(double) +
+        // (a lane per voxel for the fractions: K^T s and iso^T s too)
+        const bool lane_frac = !lr_drl && lrt.fx != nullptr;
+        const size_t per_voxel = (size_t(std::max(c_lr, c_hr)) + size_t(c_lr) + 2 * size_t(ci) + 1 +
+                                  (lane_frac ? size_t(c_lr + ci) : 0)) *
+                                     sizeof(double) +
                                  3 * sizeof(int) + 1;
         const int64_t n_max = std::min<int64_t>(v, std::max<int64_t>(4096, int64_t((size_t(4) << 30) / per_voxel)));
         const int64_t lr_slots = lr_drl ? 0 : resident_slots(lr_nnls.kernel, lr_smem, n_max, "sd.nnls.ctas_per_sm");
@@ -1533,7 +1876,10 @@ static int fit_multi_tissue(const double* signals, int64_t v, const double* weig
         const bool high = !hr_drl && hrs.normal_equations && c_hr > 64 && c_hr <= 320;
         const int64_t high_slots =
             high ? resident_slots(ridge_nnls_high_kernel, high_smem_bytes(), n_max, "sd.nnls.ctas_per_sm", kHighWarps) : 0;
-        const int64_t lf_slots = resident_slots(lr_fractions_kernel, 0, n_max, "sd.fractions.ctas_per_sm");
+        const size_t lane_smem = lane_frac ? frac_lane_smem(FracConstants::doubles(c_lr, ci, lrt.fx_rows)) : 0;
+        const int64_t lf_slots =
+            lane_frac ? resident_slots(lane_fractions_kernel, lane_smem, (n_max + 31) / 32, "sd.fractions.ctas_per_sm")
+                      : resident_slots(lr_fractions_kernel, 0, n_max, "sd.fractions.ctas_per_sm");
         const int64_t hf_slots = resident_slots(hr_fractions_kernel, 0, n_max, "sd.fractions.ctas_per_sm");
         const size_t lr_slot = nnls_slot_doubles(mi, lr_nnls.cap), hr_slot = nnls_slot_doubles(mi, hr_nnls.cap);
         const size_t lf_slot = frac_slot_doubles(mi, c_lr, 1 + ci), hf_slot = frac_slot_doubles(mi, c_hr, nf);
@@ -1545,7 +1891,7 @@ static int fit_multi_tissue(const double* signals, int64_t v, const double* weig
                             // [4] the voxels to refit by the one-warp NNLS
             int* list[2];
             int* redo;
-            double *fiso, *prev, *corr, *xlr, *slots;
+            double *fiso, *prev, *corr, *xlr, *ks, *slots;
             int32_t* rounds;
             uint8_t* bad;
         };
@@ -1559,6 +1905,7 @@ static int fit_multi_tissue(const double* signals, int64_t v, const double* weig
             p.prev = cv.take<double>(size_t(n_max) * (ci + 1));
             p.corr = cv.take<double>(size_t(n_max) * std::max(c_lr, c_hr));
             p.xlr = cv.take<double>(size_t(n_max) * c_lr);
+            p.ks = cv.take<double>(lane_frac ? size_t(n_max) * (c_lr + ci) : 0);
             p.rounds = cv.take<int32_t>(size_t(n_max));
             p.bad = cv.take<uint8_t>(size_t(n_max));
             p.slots = cv.take<double>(slot_doubles);
@@ -1595,6 +1942,11 @@ static int fit_multi_tissue(const double* signals, int64_t v, const double* weig
             cuda_check(cudaMemsetAsync(P.rounds, 0, size_t(n) * sizeof(int32_t), st), "cudaMemsetAsync");
             cuda_check(cudaMemsetAsync(P.bad, 0, size_t(n), st), "cudaMemsetAsync");
             const SignalDev lr_sig{sig, dweights, lrt.wiso, P.fiso, mi, ci};
+            if (lane_frac && max_rounds > 0) {
+                const RidgeDev kx{mi, c_lr + ci, 0.0, 0.0, 0, lr->kx.ptr, nullptr};
+                launch_correlate(SignalDev{sig, nullptr, nullptr, nullptr, mi, 0}, nullptr, n, nullptr, kx, P.ks,
+                                 c_lr + ci, st);
+            }
             // The first round takes every voxel; later rounds the list the previous one wrote,
             // with its count read back on the host (or, under capture, on the device).
             const int* cur = nullptr;
@@ -1633,8 +1985,16 @@ static int fit_multi_tissue(const double* signals, int64_t v, const double* weig
                         lr_slot);
                     cuda_check(cudaGetLastError(), "ridge_nnls_kernel launch");
                 }
-                reset_queue();
-                {
+                if (lane_frac) {
+                    LaunchScope scope("lane_fractions_kernel", st);
+                    const FracRound fr{sig, P.xlr, P.ks, P.fiso, P.prev, P.rounds, nxt, nxt_count, c_lr, round,
+                                       max_rounds, fraction_tol};
+                    const unsigned grid = unsigned(std::min<int64_t>((count + 31) / 32, lf_slots / kFracWarps));
+                    lane_fractions_kernel<<<grid, kFracWarps * 32, lane_smem, st>>>(lrt, fr, cur, count, cur_count,
+                                                                                   P.slots, lf_slot);
+                    cuda_check(cudaGetLastError(), "lane_fractions_kernel launch");
+                } else {
+                    reset_queue();
                     LaunchScope scope("lr_fractions_kernel", st);
                     lr_fractions_kernel<<<blocks(lf_slots, count), kMtWarps * 32, 0, st>>>(
                         lrt, sig, P.xlr, c_lr, cur, count, cur_count, round, max_rounds, fraction_tol, P.fiso, P.prev,
@@ -1718,6 +2078,10 @@ struct MfodBatch {
     ~MfodBatch() {
         if (scratch) cudaFree(scratch);
     }
+    int64_t ks_doubles = 0;  // of the volumes whose fractions take a lane per voxel
+    int ks_m = 0, fx_doubles = 0;  // their most measurements and constants
+    bool lane_all = true;          // they are all of them
+    int64_t lane_slots = 0;
     int tc_m = 0;         // the most measurements of the volumes the tensor-core correlations take
     bool tc_all = true;   // they take every volume
     // A stage's correlations: the tensor-core kernel's volumes, then the others.
@@ -1795,6 +2159,15 @@ void mfod_batch_add(MfodBatch* b, const double* signals, int64_t v, const double
     j.fractions = fractions;
     j.rounds = rounds;
     j.status = status;
+    j.kx = lr->kx.ptr;
+    j.ks_off = b->ks_doubles;
+    if (j.lrt.fx != nullptr) {
+        b->ks_doubles += v * (lr->ca + lr->ci);
+        b->ks_m = std::max(b->ks_m, int(m));
+        b->fx_doubles = std::max(b->fx_doubles, FracConstants::doubles(int(lr->ca), int(lr->ci), lr->fx_rows));
+    } else {
+        b->lane_all = false;
+    }
     b->jobs.push_back(j);
     b->weights.emplace_back(weights, weights + m);
     b->voxels += v;
@@ -1826,7 +2199,10 @@ void mfod_batch_finalize(MfodBatch* b) {
     b->lr_slots = resident_slots(batch_redo_kernel<1, 2, false>, b->lr_smem, V, "sd.nnls.ctas_per_sm");
     b->hr_smem = nnls_smem_bytes(b->c_hr_max, kCholCap) * kMtWarps;
     b->hr_slots = resident_slots(batch_redo_kernel<kCholCap / 32, 10, true>, b->hr_smem, V, "sd.nnls.ctas_per_sm");
-    b->lf_slots = resident_slots(batch_lr_fractions_kernel, 0, V, "sd.fractions.ctas_per_sm");
+    b->lf_slots = b->lane_all ? 0 : resident_slots(batch_lr_fractions_kernel, 0, V, "sd.fractions.ctas_per_sm");
+    b->lane_slots = b->fx_doubles ? resident_slots(batch_lane_fractions_kernel, frac_lane_smem(b->fx_doubles),
+                                                   (V + 31) / 32, "sd.fractions.ctas_per_sm")
+                                  : 0;
     b->hf_slots = resident_slots(batch_hr_fractions_kernel, 0, V, "sd.fractions.ctas_per_sm");
     b->lr_slot = nnls_slot_doubles(mi, 32);
     b->hr_slot = nnls_slot_doubles(mi, kCholCap);
@@ -1834,7 +2210,7 @@ void mfod_batch_finalize(MfodBatch* b) {
     b->hf_slot = frac_slot_doubles(mi, b->c_hr_max, b->nf_max);
     const size_t slot_doubles =
         std::max({size_t(b->lr_slots) * b->lr_slot, size_t(b->hr_slots) * b->hr_slot,
-                  size_t(b->lf_slots) * b->lf_slot, size_t(b->hf_slots) * b->hf_slot});
+                  size_t(std::max(b->lf_slots, b->lane_slots)) * b->lf_slot, size_t(b->hf_slots) * b->hf_slot});
     auto carve_all = [&](Carver& cv) {
         MfodBatchState s{};
         s.jobs = b->d_jobs.ptr;
@@ -1846,6 +2222,7 @@ void mfod_batch_finalize(MfodBatch* b) {
         s.prev = cv.take<double>(size_t(V) * (ci + 1));
         s.corr = cv.take<double>(size_t(V) * ldc);
         s.xlr = cv.take<double>(size_t(V) * ldx);
+        s.ks = cv.take<double>(size_t(b->ks_doubles));
         s.rounds = cv.take<int32_t>(size_t(V));
         s.bad = cv.take<uint8_t>(size_t(V));
         s.vfirst = cv.take<int64_t>(size_t(nj) + 1);
@@ -1899,6 +2276,15 @@ void mfod_batch_run(MfodBatch* b, cudaStream_t st) {
             batch_plan_kernel<<<1, 32, 0, st>>>(B, cur_counts);
             launched("batch_plan_kernel launch");
         }
+        if (round == 0 && b->fx_doubles > 0) {
+            const size_t smem = corr_tc_smem(b->ks_m, 0);
+            cuda_check(cudaFuncSetAttribute(batch_ks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
+                       "cudaFuncSetAttribute");
+            LaunchScope scope("batch_ks_kernel", st);
+            const unsigned gy = unsigned((b->c_lr_max + ci + kCorrTcCols - 1) / kCorrTcCols);
+            batch_ks_kernel<<<dim3(unsigned(sm_count()) / gy, gy), kCorrTcWarps * 32, smem, st>>>(B);
+            launched("batch_ks_kernel launch");
+        }
         b->correlate<false>(cur, corr_grid, st);
         zero(b->queue, sizeof(int));
         zero(nxt_counts, size_t(nj) * sizeof(int));
@@ -1915,8 +2301,15 @@ void mfod_batch_run(MfodBatch* b, cudaStream_t st) {
                 B, b->c_lr_max, b->queue, b->slots, b->lr_slot);
             launched("batch_redo_kernel launch");
         }
-        zero(b->queue, sizeof(int));
-        {
+        if (b->fx_doubles > 0) {
+            LaunchScope scope("batch_lane_fractions_kernel", st);
+            batch_lane_fractions_kernel<<<unsigned(b->lane_slots / kFracWarps), kFracWarps * 32,
+                                          frac_lane_smem(b->fx_doubles), st>>>(
+                B, b->fx_doubles, cur, round, b->max_rounds, b->fraction_tol, nxt, nxt_counts, b->slots, b->lf_slot);
+            launched("batch_lane_fractions_kernel launch");
+        }
+        if (!b->lane_all) {
+            zero(b->queue, sizeof(int));
             LaunchScope scope("batch_lr_fractions_kernel", st);
             batch_lr_fractions_kernel<<<blocks(b->lf_slots, V), kMtWarps * 32, 0, st>>>(
                 B, cur, round, b->max_rounds, b->fraction_tol, nxt, nxt_counts, b->queue, b->slots, b->lf_slot);
@@ -2137,6 +2530,7 @@ int lar_deconv_kernel_create(const double* k_aniso, int64_t m, int64_t ca, const
         std::vector<int> bl(size_t(2 * nb));
         for (int64_t b = 0; b < 2 * nb; ++b) bl[size_t(b)] = int(blocks[b]);
         h->blocks.upload(bl.data(), bl.size());
+        prepare_frac_constants(h.get(), k_aniso, iso.data());
         *out = h.release();
     });
 }

@@ -51,6 +51,36 @@ def test_lean_nnls_matches_the_oracle(cuda, oracle, c_lr, c_hr, v, sparse):
         assert ((fods > 0).sum(axis=1) > 32).any()  # some voxels outgrow the lean factor
 
 
+# Kernels within [0, 1] whose maximum can lie in `top` rows only (row r is 1 but for one entry): the
+# lane-per-voxel fractions take up to 16 such rows and solutions that are mostly zero; 17 rows, more
+# columns, four isotropic tissues or dense solutions go the general way.
+@pytest.mark.parametrize("top, c_lr, v, sparse, ci", [
+    (1, 44, 1, True, 2), (1, 1, 33, True, 1), (2, 47, 64, True, 3), (16, 48, 31, True, 2), (17, 40, 20, True, 2),
+    (1, 49, 20, True, 2), (1, 20, 40, True, 0), (1, 20, 40, True, 4), (1, 40, 70, False, 2)])
+def test_fractions_of_bounded_kernels(cuda, oracle, top, c_lr, v, sparse, ci):
+    from larmor_b200 import _core
+
+    rng = np.random.default_rng(100 * top + c_lr)
+    k_lr, k_hr = (rng.uniform(0.0, 1.0, (M, c)) ** 3 for c in (c_lr, 100))
+    k_lr[:top] = 1.0
+    for r in range(1, top):
+        k_lr[r, r % c_lr] = 1.0 + 0.01 * r
+        k_lr[r, (r + 1) % c_lr] = 0.5
+    k_lr, k_hr = np.ascontiguousarray(k_lr), np.ascontiguousarray(k_hr)
+    iso = np.ascontiguousarray(np.exp(-np.linspace(0, 1, M)[:, None] * (1.0 + 2.0 * np.arange(ci))))
+    x = rng.uniform(0.0, 1.0, (v, c_lr)) * (rng.uniform(size=(v, c_lr)) < (0.15 if sparse else 0.95))
+    s = np.ascontiguousarray(np.maximum(
+        x @ k_lr.T / c_lr + rng.uniform(0.0, 0.2, (v, ci)) @ iso.T + 0.01 * rng.standard_normal((v, M)), 0.0))
+    empty = ci == 0
+    lr, hr = (_core.DeconvKernel(k, None if empty else iso, None if empty else iso, [(0, k.shape[1])])
+              for k in (k_lr, k_hr))
+    fods, fractions = _core.fit_multi_tissue(s, np.ones(M), lr, _core.FodSolver.l2nnls(k_lr, 0.0, 1e-6), hr,
+                                             _core.FodSolver.l2nnls(k_hr, 0.1, 1e-6), 20, 1e-7, 1e-2, 1)
+    rf, rfr = _oracle(oracle, k_lr, k_hr, iso, s)
+    assert np.abs(fods - rf).max() <= 1e-8 * np.abs(rf).max()
+    assert np.abs(fractions - rfr).max() <= 1e-8
+
+
 def test_a_nan_voxel_leaves_the_others_alone(cuda):
     k_lr, k_hr, iso, s = _case(3, 44, 100, 50)
     plain, plain_fr = _device(k_lr, k_hr, iso, s)
