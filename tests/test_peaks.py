@@ -508,3 +508,77 @@ def test_gpu_isotropic_fod_merges_every_start(cuda, oracle, peaks_fixture):
     np.testing.assert_array_equal(np.isnan(amps), np.isnan(ra))
     np.testing.assert_allclose(dirs, rd, rtol=0, atol=1e-12)
     np.testing.assert_allclose(amps, ra, rtol=1e-12)
+
+
+def _crossings(n: int) -> np.ndarray:
+    """n voxels of two crossing fibres, some along or near the z axis, where a climb meets a pole."""
+    rng = np.random.default_rng(71)
+    out = []
+    for k in range(n):
+        a, b = _unit(rng.normal(size=3)), _unit(rng.normal(size=3))
+        if k % 3 == 0:
+            tilt, turn = (0.0, 0.02, 0.1)[k // 3 % 3], rng.uniform(0, 2 * math.pi)
+            a = _unit([math.sin(tilt) * math.cos(turn), math.sin(tilt) * math.sin(turn), math.cos(tilt)])
+        out.append(_fibre_sh(a) + rng.uniform(0, 1.2) * _fibre_sh(b))
+    return np.stack(out)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("full", [False, True])
+@pytest.mark.parametrize("copies", [1, 2])
+@pytest.mark.parametrize("n", [1, 16, 37])
+def test_gpu_search_shares_opposite_climbs(cuda, oracle, peaks_fixture, n, copies, full):
+    """Opposite maxima of an even series share a climb, on a sphere whose amplitudes fit a block's shared memory
+    and on one of twice the vertices that does not, with the whole and a partial group of voxels. Climbs of one peak
+    whose amplitudes tie may leave either: both ended by a step below 1e-4, which for a tie within
+    rounding is the last of a quadratic convergence, so within 2 * 8 * 1e-8. A climb that steps from a
+    pole and back with the capped step leaves that cycle by its rounding: voxels whose peaks the oracle itself moves
+    when the starts move by 1e-15 are not compared."""
+    from larmor_b200 import _core
+    from larmor_b200.sd.sh import build_basis_matrix
+    from larmor_b200.sd.sphere import get_theta_phi
+
+    v, nb = peaks_fixture["vertices"], peaks_fixture["neighbours"]
+    if copies == 2:  # a second icosphere, turned about the z axis
+        c, s = math.cos(0.1), math.sin(0.1)
+        v = np.concatenate([v, v @ np.array([[c, s, 0.0], [-s, c, 0.0], [0.0, 0.0, 1.0]])])
+        nb = np.concatenate([nb, nb + 642])
+    theta, phi = get_theta_phi(v)
+    shs = _crossings(n)
+    if full:
+        shs = np.stack([_to_full(sh, LMAX) for sh in shs])
+    on = shs @ build_basis_matrix(theta, phi, LMAX, full=full).T
+    want_d, want_a = oracle.peaks_chunk(shs, LMAX, on, v, nb, 4, 0.1, 0.0, full=full)
+    moved_d, moved_a = oracle.peaks_chunk(shs, LMAX, on, v + 1e-15, nb, 4, 0.1, 0.0, full=full)
+    got_d, got_a = _core.peaks_chunk(shs, LMAX, on, v, nb, 4, 0.1, 0.0, 1, full=full)
+    np.testing.assert_array_equal(np.isnan(got_a), np.isnan(want_a))
+    stable = np.isclose(moved_a, want_a, rtol=1e-12, atol=0, equal_nan=True).all(axis=1)
+    assert np.all(np.flatnonzero(~stable) % 3 == 0)  # a fibre near the z axis
+    np.testing.assert_allclose(got_a[stable], want_a[stable], rtol=1e-12)
+    for gd, wd in zip(got_d[stable], want_d[stable]):
+        # The two lobes that a symmetric fibre has in a full series have one amplitude: either may come first.
+        found = np.isfinite(wd[:, 0])
+        nearest = np.argmax(wd[found] @ gd[found].T, axis=1)
+        assert sorted(nearest) == list(range(int(found.sum())))
+        np.testing.assert_allclose(gd[found][nearest], wd[found], rtol=0, atol=1.6e-7)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ca", [1, 15, 16, 17, 28, 29, 45, 48])
+@pytest.mark.parametrize("rows", [1, 15, 130])
+def test_gpu_expansion_on_many_directions(cuda, ca, rows):
+    """A short series on many directions: the product within the rounding of its sums, at the edges of its
+    tiles and slices, from a column slice."""
+    import torch
+
+    from larmor_b200 import _core
+
+    rng = np.random.default_rng(ca)
+    for ncoef in (4 * ca, 4 * ca + 3, 642):
+        matrix = rng.normal(size=(ncoef, ca))
+        wide = rng.normal(size=(rows, ca + 3))
+        got = _core.project_sh_device(_core.ShProjector(matrix), torch.from_numpy(wide).cuda()[:, 2 : ca + 2],
+                                      exact_integral=False).cpu().numpy()
+        a = wide[:, 2 : ca + 2]
+        bound = 2 * (ca + 1) * 2.0**-53 * (np.abs(a) @ np.abs(matrix).T)
+        assert np.all(np.abs(got - a @ matrix.T) <= bound)
