@@ -7,20 +7,27 @@
 // u = 1 - strength (1 - f^8 / (f^8 + nu^8)), with strength = max(1 - 4 std(s), 0). A voxel
 // stops when its amplitudes change in total by no more than 1e-4 of its largest signal value.
 //
-// Mapping: a CTA of 8 warps takes 8 RT voxels at a time (32 up to 320 directions, 8 up to 640)
+// Mapping: a CTA of 8 warps takes 8 RT voxels at a time (32 up to 320 directions, 16 up to 640)
 // and keeps their FODs F (8 RT, c) and K^T s (8 RT, c) in shared memory for all their
 // iterations. An iteration is one product F K^T K on the FP64 tensor cores: mma.sync m8n8k4
 // over the RT 8-voxel row tiles and the 8-direction column tiles, which the warps take
-// round-robin. K^T K (c x c, 720 KB at c = 300) stays in L2 and streams through each CTA once
-// per iteration for its voxels, 8 rows at a time, into a double-buffered shared-memory stage by
-// cp.async while the tensor cores work on the previous 8 rows. The rows of F, K^T s and the
-// stage are padded, so the fragment loads of a warp fall in distinct banks. The update is the
-// epilogue, on the accumulators, after a barrier, since every warp reads all of F. Each voxel's
-// change is reduced in a fixed order, so the stopping test does not depend on the schedule.
-// Converged voxels keep their FOD while the tile's others iterate.
+// round-robin. K^T K (c x c, 720 KB at c = 300) stays in L2. A warp's columns are no other warp's, so it
+// reads them straight into its fragments, one to three groups of eight k ahead of their use and the
+// first before the update, and the warps meet only around the update: through a shared-memory stage, with
+// two barriers per eight k, the tensor cores stood still most of the time. The two k-steps of a group take
+// its even and its odd k, so that a lane's two operands lie side by side in a row of K^T K and of F (16-byte
+// loads). K^T s is the same product of the signals with K^T. The update is the epilogue, on the
+// accumulators, after a barrier, since every warp reads all of F. Each voxel's change is reduced in
+// a fixed order, so the stopping test does not depend on the schedule. Converged voxels keep their
+// FOD while the tile's others iterate.
 //
-// Up to 64 directions the whole K^T K (at most 36 KB) is loaded once per CTA instead, and an
-// iteration needs one barrier; the CTA then fits in half an SM.
+// What bounds it: the FP64 pipe. 100,003 voxels, 300 directions, 200 iterations: 133 ms, of which the
+// products take 97 at the tensor cores' rate and 8 more for the columns past the 38th tile (through the
+// stage: 261 ms). With 32 voxels to a CTA and 8 warps nothing hides the update behind another tile's
+// products: two CTAs would need K^T K's traffic twice.
+//
+// Up to 64 directions the whole K^T K (at most 36 KB) is loaded once per CTA instead
+// (drl_resident_kernel), and the CTA then fits in half an SM.
 //
 // The multi-tissue rounds (GRL, cpp/src/sd/multi_tissue.cpp:40-95) run the same solve on a list
 // of voxels whose signal is the anisotropic part max(s w - W_iso f_iso, 0) of the round.
@@ -37,35 +44,22 @@ namespace lar {
 namespace {
 
 constexpr int kDrlWarps = 8;
-constexpr int kDrlChunk = 8;   // rows of K^T K per stage (two k-steps), one per warp
-// The two tilings: RT 8-voxel row tiles per CTA, MAXCT column tiles per warp, for
-// c <= 8 * kDrlWarps * MAXCT directions.
+constexpr int kGroup = 8;  // k values of a group: two k-steps
+// RT 8-voxel row tiles per CTA, up to MAXCT column tiles per warp, for c <= 8 * kDrlWarps * MAXCT directions.
 constexpr int kNarrowRt = 4, kNarrowCt = 5;   // 32 voxels, c <= 320
-constexpr int kWideRt = 1, kWideCt = 10;      // 8 voxels, c <= 640
+constexpr int kWideRt = 2, kWideCt = 10;      // 16 voxels, c <= 640
 constexpr int kNarrowMaxC = 8 * kDrlWarps * kNarrowCt;
 constexpr int kWideMaxC = 8 * kDrlWarps * kWideCt;
 // Up to 64 directions (the low-resolution kernels of the multi-tissue rounds) all of K^T K stays
 // in shared memory for the CTA's life: 32 voxels, one column tile per warp, two CTAs per SM.
 constexpr int kResidentMaxC = 8 * kDrlWarps;
 
-// Row strides (doubles) of F and K^T s, and of the K^T K stage, for cp columns: the padding puts
-// the 8 rows of an A fragment, and the 4 rows of a B fragment, in different banks.
+// Row strides (doubles) for cp columns, in the resident kernel of F and K^T s, and of K^T K: the padding puts
+// the 8 rows of an A fragment, and the 4 rows of a B fragment, in different banks. In the streaming kernel of
+// F and K^T s: 8 more than a multiple of 16, so that two rows' 64 bytes of a fragment are in different banks.
 __host__ __device__ inline int drl_ldf(int cp) { return cp + 4; }
 __host__ __device__ inline int drl_ldg(int cp) { return cp + 8; }
-
-__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
-    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src));
-}
-__device__ __forceinline__ void cp_async16(double* dst, const double* src) {
-    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N));
-}
+__host__ __device__ inline int drl_lds(int cp) { return cp % 16 == 8 ? cp : cp + 8; }
 
 __device__ __forceinline__ double power_8(double x) {
     const double x2 = x * x, x4 = x2 * x2;
@@ -88,98 +82,150 @@ __device__ __forceinline__ double signal_at(const DrlSignal& S, int64_t voxel, i
     return fmax(ws - r, 0.0);
 }
 
+// The voxels of a tile from list entry p0, each one's damping strength (1 - 4 x the sample standard
+// deviation, at least 0) and stopping threshold (1e-4 x its largest non-NaN signal value).
+template <int ROWS>
+struct DrlTile {
+    double part[kDrlWarps][ROWS];
+    double strength[ROWS], threshold[ROWS];
+    int active[ROWS];
+    int64_t vox[ROWS];
+};
+
+template <int ROWS>
+__device__ __forceinline__ void open_tile(DrlTile<ROWS>& t, const DrlSignal& S, int m, const int* __restrict__ list,
+                                          int64_t p0, int64_t count) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid < ROWS) t.vox[tid] = p0 + tid < count ? (list ? int64_t(list[p0 + tid]) : p0 + tid) : -1;
+    __syncthreads();
+    for (int r = warp; r < ROWS; r += kDrlWarps) {
+        const int64_t voxel = t.vox[r];
+        if (voxel < 0) {
+            if (lane == 0) {
+                t.active[r] = 0;
+                t.strength[r] = t.threshold[r] = 0.0;
+            }
+            continue;
+        }
+        double sum = 0.0, mx = -CUDART_INF;
+        bool any = false;
+        for (int i = lane; i < m; i += 32) {
+            const double si = signal_at(S, voxel, i);
+            sum += si;
+            if (!isnan(si)) {
+                mx = any ? fmax(mx, si) : si;
+                any = true;
+            }
+        }
+        const double mean = warp_sum(sum) / m;
+        double ss = 0.0;
+        for (int i = lane; i < m; i += 32) {
+            const double si = signal_at(S, voxel, i);
+            ss += (si - mean) * (si - mean);
+        }
+        ss = warp_sum(ss);
+        const bool all_nan = !__any_sync(0xffffffffu, any);
+        mx = warp_max(any ? mx : -CUDART_INF);
+        if (lane == 0) {
+            t.strength[r] = fmax(1.0 - 4.0 * sqrt(ss / double(m - 1)), 0.0);
+            t.threshold[r] = 1e-4 * (all_nan ? CUDART_NAN : mx);
+            t.active[r] = 1;
+        }
+    }
+}
+
+// a / b by Newton's iteration on the hardware's approximate reciprocal and one step on the quotient, without
+// the branches of the general division, so that a lane's quotients overlap (the 100,003 voxels below took
+// 149 ms with them). For |b| well inside the range of the exponent: (f^8 + nu^8) (p + 1e-16) is, with
+// f >= 1e-6 from the first update on.
+__device__ __forceinline__ double quotient(double a, double b) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
+    r = fma(r, fma(-b, r, 1.0), r);
+    r = fma(r, fma(-b, r, 1.0), r);
+    const double q = a * r;
+    return fma(r, fma(-b, q, a), q);
+}
+
+// The update's relative step as it is written, for a start and a nu so small that the quotient's range may end.
+__device__ __noinline__ double plain_step(double f8, double nu8, double strength, double ks, double pred) {
+    return (1.0 - strength * (1.0 - f8 / (f8 + nu8))) * ((ks - pred) / (pred + 1e-16));
+}
+
+// The damped update of the still-active voxels from the prediction acc (column tile t of the warp in
+// acc[.][t]), each one's total change into part, and whether any voxel is still active. The damping
+// 1 - strength (1 - f^8 / (f^8 + nu^8)) and the ratio (K^T s - p) / (p + 1e-16) share one division.
+template <int RT, int CT>
+__device__ __forceinline__ bool update_tile(DrlTile<8 * RT>& tile, const double (&acc)[RT][CT][2], double* F,
+                                            const double* KS, int ld, int c, double nu8, bool plain) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+    for (int rt = 0; rt < RT; ++rt) {
+        const int r = 8 * rt + (lane >> 2);
+        double change = 0.0;
+        if (tile.active[r]) {
+            const double off = (1.0 - tile.strength[r]) * nu8;
+#pragma unroll
+            for (int t = 0; t < CT; ++t) {
+                const int d = 8 * (warp + kDrlWarps * t) + 2 * (lane & 3);
+                double* at = F + r * ld + min(d, c - 1) / 2 * 2;
+                const double2 f = *reinterpret_cast<const double2*>(at);
+                const double2 ks = *reinterpret_cast<const double2*>(KS + (at - F));
+                double to[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const double fh = h ? f.y : f.x, f8 = power_8(fh), pred = acc[rt][t][h];
+                    double step = quotient((f8 + off) * ((h ? ks.y : ks.x) - pred), (f8 + nu8) * (pred + 1e-16));
+                    if (plain) step = plain_step(f8, nu8, tile.strength[r], h ? ks.y : ks.x, pred);
+                    to[h] = fmax(fh * (1.0 + step), 1e-6);
+                    if (d + h < c) change += fabs(to[h] - fh);
+                }
+                if (d < c) at[0] = to[0];
+                if (d + 1 < c) at[1] = to[1];
+            }
+        }
+        change += __shfl_xor_sync(0xffffffffu, change, 1);
+        change += __shfl_xor_sync(0xffffffffu, change, 2);
+        if ((lane & 3) == 0) tile.part[warp][r] = change;
+    }
+    __syncthreads();
+    int alive = 0;
+    if (tid < 8 * RT && tile.active[tid]) {
+        double total = 0.0;
+        for (int w = 0; w < kDrlWarps; ++w) total += tile.part[w][tid];
+        alive = !(total <= tile.threshold[tid]);
+        tile.active[tid] = alive;
+    }
+    return __syncthreads_or(alive);
+}
+
 // x(list[p], :) = the dRL FOD of voxel list[p] for p < count (min(count, *count_dev) when
 // count_dev is given); no list: voxel p itself.
-template <int RT, int MAXCT, bool RESIDENT>
-__global__ void __launch_bounds__(kDrlWarps * 32, RESIDENT ? 2 : 1)
-    drl_kernel(DrlDev P, DrlSignal S, const int* __restrict__ list, int64_t count, const int* __restrict__ count_dev,
-               double* __restrict__ x, int64_t ldx) {
-    constexpr int kRows = 8 * RT;
+__global__ void __launch_bounds__(kDrlWarps * 32, 2)
+    drl_resident_kernel(DrlDev P, DrlSignal S, const int* __restrict__ list, int64_t count,
+                        const int* __restrict__ count_dev, double* __restrict__ x, int64_t ldx) {
+    constexpr int RT = kNarrowRt, kRows = 8 * RT;
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ double part[kDrlWarps][kRows];
-    __shared__ double strength[kRows], threshold[kRows];
-    __shared__ int active[kRows];
-    __shared__ int64_t vox[kRows];
-    __shared__ int n_active;
+    __shared__ DrlTile<kRows> tile;
     if (count_dev) count = min(count, int64_t(*count_dev));
-    const int c = P.c, m = P.m, cp = (c + 7) / 8 * 8, n_ct = cp / 8, ldf = drl_ldf(cp), ldg = drl_ldg(cp);
+    const int c = P.c, m = P.m, cp = (c + 7) / 8 * 8, ldf = drl_ldf(cp), ldg = drl_ldg(cp);
     double* F = reinterpret_cast<double*>(smem);  // (kRows, ldf)
     double* KS = F + kRows * ldf;                 // (kRows, ldf)
-    double* GS = KS + kRows * ldf;                // (2, kDrlChunk, ldg): the K^T K stage; resident: (cp, ldg)
+    double* GS = KS + kRows * ldf;                // (cp, ldg)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const double nu8 = power_8(P.nu);
-    if constexpr (RESIDENT) {
-        // All of K^T K, zero past c (made visible by the barrier at the first tile's start).
-        for (int e = threadIdx.x; e < cp * ldg; e += blockDim.x) {
-            const int k = e / ldg, d = e - k * ldg;
-            GS[e] = (k < c && d < c) ? P.gram[size_t(k) * c + d] : 0.0;
-        }
-    } else {
-        // The stage's columns past c stay 0.
-        for (int e = threadIdx.x; e < 2 * kDrlChunk * ldg; e += blockDim.x)
-            if (e % ldg >= c) GS[e] = 0.0;
+    const bool plain = !(nu8 + power_8(P.init) > 1e-200);
+    // All of K^T K, zero past c (made visible by the barrier at the first tile's start).
+    for (int e = threadIdx.x; e < cp * ldg; e += blockDim.x) {
+        const int k = e / ldg, d = e - k * ldg;
+        GS[e] = (k < c && d < c) ? P.gram[size_t(k) * c + d] : 0.0;
     }
-    const int n_chunks = cp / kDrlChunk;
-    // Rows [8 q, 8 q + 8) of K^T K into stage buffer b, one row per 32 threads: cp.async of 16
-    // bytes when the rows are 16-byte aligned (c even; the stage's row stride is a multiple of 16
-    // bytes), else of 8; zeros for the rows past c.
-    const bool wide = c % 2 == 0;
-    auto stage = [&](int q, int b) {
-        const int r = threadIdx.x >> 5, k = q * kDrlChunk + r;
-        double* dst = GS + (b * kDrlChunk + r) * ldg;
-        const double* src = P.gram + size_t(k) * c;
-        if (k >= c) {
-            for (int d = lane; d < c; d += 32) dst[d] = 0.0;
-        } else if (wide) {
-            for (int d = 2 * lane; d < c; d += 64) cp_async16(dst + d, src + d);
-        } else {
-            for (int d = lane; d < c; d += 32) cp_async8(dst + d, src + d);
-        }
-        cp_async_commit();
-    };
     for (int64_t p0 = int64_t(blockIdx.x) * kRows; p0 < count; p0 += int64_t(gridDim.x) * kRows) {
-        if (tid < kRows) vox[tid] = p0 + tid < count ? (list ? int64_t(list[p0 + tid]) : p0 + tid) : -1;
-        __syncthreads();
-        // Each voxel's damping strength (1 - 4 x the sample standard deviation, at least 0) and
-        // stopping threshold (1e-4 x its largest non-NaN signal value).
-        for (int r = warp; r < kRows; r += kDrlWarps) {
-            const int64_t voxel = vox[r];
-            if (voxel < 0) {
-                if (lane == 0) {
-                    active[r] = 0;
-                    strength[r] = threshold[r] = 0.0;
-                }
-                continue;
-            }
-            double sum = 0.0, mx = -CUDART_INF;
-            bool any = false;
-            for (int i = lane; i < m; i += 32) {
-                const double si = signal_at(S, voxel, i);
-                sum += si;
-                if (!isnan(si)) {
-                    mx = any ? fmax(mx, si) : si;
-                    any = true;
-                }
-            }
-            const double mean = warp_sum(sum) / m;
-            double ss = 0.0;
-            for (int i = lane; i < m; i += 32) {
-                const double si = signal_at(S, voxel, i);
-                ss += (si - mean) * (si - mean);
-            }
-            ss = warp_sum(ss);
-            const bool all_nan = !__any_sync(0xffffffffu, any);
-            mx = warp_max(any ? mx : -CUDART_INF);
-            if (lane == 0) {
-                strength[r] = fmax(1.0 - 4.0 * sqrt(ss / double(m - 1)), 0.0);
-                threshold[r] = 1e-4 * (all_nan ? CUDART_NAN : mx);
-                active[r] = 1;
-            }
-        }
+        open_tile(tile, S, m, list, p0, count);
         // K^T s and the start.
         for (int e = tid; e < kRows * ldf; e += blockDim.x) {
             const int r = e / ldf, d = e - r * ldf;
-            const int64_t voxel = vox[r];
+            const int64_t voxel = tile.vox[r];
             const bool real = voxel >= 0 && d < c;
             double ks = 0.0;
             if (real) {
@@ -191,118 +237,167 @@ __global__ void __launch_bounds__(kDrlWarps * 32, RESIDENT ? 2 : 1)
         }
         __syncthreads();
         for (int it = 0; it < P.n_iter; ++it) {
-            if (tid == 0) {
-                int a = 0;
-                for (int r = 0; r < kRows; ++r) a += active[r];
-                n_active = a;
-            }
-            __syncthreads();
-            if (n_active == 0) break;
             // The prediction K^T K f of every voxel of the tile (K^T K is symmetric: its column
             // block is read as rows).
-            double acc[RT][MAXCT][2];
+            double acc[RT][1][2];
 #pragma unroll
-            for (int rt = 0; rt < RT; ++rt)
+            for (int rt = 0; rt < RT; ++rt) acc[rt][0][0] = acc[rt][0][1] = 0.0;
+            if (8 * warp < cp)
+                for (int k0 = 0; k0 < cp; k0 += 4) {
+                    const int kk = k0 + (lane & 3);
+                    const double b = GS[kk * ldg + 8 * warp + (lane >> 2)];
 #pragma unroll
-                for (int t = 0; t < MAXCT; ++t) acc[rt][t][0] = acc[rt][t][1] = 0.0;
-            if constexpr (RESIDENT) {
-                const int ct = warp;
-                if (ct < n_ct) {
-                    for (int k0 = 0; k0 < cp; k0 += 4) {
-                        const int kk = k0 + (lane & 3);
-                        const double b = GS[kk * ldg + 8 * ct + (lane >> 2)];
-#pragma unroll
-                        for (int rt = 0; rt < RT; ++rt)
-                            mma_f64(acc[rt][0][0], acc[rt][0][1], F[(8 * rt + (lane >> 2)) * ldf + kk], b);
-                    }
+                    for (int rt = 0; rt < RT; ++rt)
+                        mma_f64(acc[rt][0][0], acc[rt][0][1], F[(8 * rt + (lane >> 2)) * ldf + kk], b);
                 }
-                // The update overwrites F: every warp is done reading it first.
-                __syncthreads();
-            } else {
-                stage(0, 0);
-                for (int q = 0; q < n_chunks; ++q) {
-                    if (q + 1 < n_chunks) {
-                        stage(q + 1, (q + 1) & 1);
-                        cp_async_wait<1>();
-                    } else {
-                        cp_async_wait<0>();
-                    }
-                    __syncthreads();
-                    const double* g = GS + (q & 1) * kDrlChunk * ldg;
-#pragma unroll
-                    for (int ks = 0; ks < kDrlChunk; ks += 4) {
-                        const int kk = q * kDrlChunk + ks + (lane & 3);
-                        const double* grow = g + (ks + (lane & 3)) * ldg + (lane >> 2);
-                        double a[RT];
-#pragma unroll
-                        for (int rt = 0; rt < RT; ++rt) a[rt] = F[(8 * rt + (lane >> 2)) * ldf + kk];
-#pragma unroll
-                        for (int t = 0; t < MAXCT; ++t) {
-                            const int ct = warp + kDrlWarps * t;
-                            if (ct < n_ct) {
-                                const double b = grow[8 * ct];
-#pragma unroll
-                                for (int rt = 0; rt < RT; ++rt) mma_f64(acc[rt][t][0], acc[rt][t][1], a[rt], b);
-                            }
-                        }
-                    }
-                    // The next stage overwrites this buffer: every warp is done with it first.
-                    __syncthreads();
-                }
-            }
-            // The damped update of the still-active voxels, and each one's total change.
-            double change[RT];
-#pragma unroll
-            for (int rt = 0; rt < RT; ++rt) change[rt] = 0.0;
-#pragma unroll
-            for (int t = 0; t < MAXCT; ++t) {
-                const int ct = warp + kDrlWarps * t;
-                if (ct >= n_ct) continue;
-#pragma unroll
-                for (int rt = 0; rt < RT; ++rt) {
-                    const int r = 8 * rt + (lane >> 2);
-                    if (!active[r]) continue;
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int d = 8 * ct + 2 * (lane & 3) + h;
-                        if (d >= c) continue;
-                        const double f = F[r * ldf + d], f8 = power_8(f);
-                        const double damping = 1.0 - strength[r] * (1.0 - f8 / (f8 + nu8));
-                        const double pred = acc[rt][t][h];
-                        const double ratio = (KS[r * ldf + d] - pred) / (pred + 1e-16);
-                        const double updated = fmax(f * (1.0 + damping * ratio), 1e-6);
-                        F[r * ldf + d] = updated;
-                        change[rt] += fabs(updated - f);
-                    }
-                }
-            }
-#pragma unroll
-            for (int rt = 0; rt < RT; ++rt) {
-                change[rt] += __shfl_xor_sync(0xffffffffu, change[rt], 1);
-                change[rt] += __shfl_xor_sync(0xffffffffu, change[rt], 2);
-                if ((lane & 3) == 0) part[warp][8 * rt + (lane >> 2)] = change[rt];
-            }
+            // The update overwrites F: every warp is done reading it first.
             __syncthreads();
-            if (tid < kRows && active[tid]) {
-                double total = 0.0;
-                for (int w = 0; w < kDrlWarps; ++w) total += part[w][tid];
-                if (total <= threshold[tid]) active[tid] = 0;
-            }
-            __syncthreads();
+            if (!update_tile<RT, 1>(tile, acc, F, KS, ldf, c, nu8, plain)) break;
         }
         for (int e = tid; e < kRows * ldf; e += blockDim.x) {
             const int r = e / ldf, d = e - r * ldf;
-            const int64_t voxel = vox[r];
+            const int64_t voxel = tile.vox[r];
             if (voxel >= 0 && d < c) x[voxel * ldx + d] = F[e];
         }
         __syncthreads();
     }
 }
 
-template <int RT, int MAXCT, bool RESIDENT>
-void launch_variant(const DrlDev& P, const DrlSignal& S, const int* list, int64_t count, const int* count_dev,
-                    double* x, int64_t ldx, cudaStream_t st, const char* name) {
-    auto kernel = drl_kernel<RT, MAXCT, RESIDENT>;
+// Columns 8 (warp + 8 t) + {0..7}, t < CT, of A B^T for a tile's rows A (8 RT, k) in shared memory and B
+// (n, k) row-major in global memory: B's fragments through registers, DEPTH groups of eight k in flight.
+template <int RT, int CT>
+struct StreamedProduct {
+    static constexpr int DEPTH = CT >= 4 ? 2 : 4;
+    double2 b[DEPTH][CT];
+    const double* row[CT];  // of this lane's column in tile t, at its first k
+    int k;                  // k values, and this lane's next group is at k0
+    bool wide;              // rows of B start on 16 bytes
+
+    __device__ __forceinline__ void open(const double* __restrict__ B, int64_t ldb, int n, int from, int count) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        k = count;
+        wide = ldb % 2 == 0 && from % 2 == 0 && (reinterpret_cast<uintptr_t>(B) & 15) == 0;
+#pragma unroll
+        for (int t = 0; t < CT; ++t)  // a column past the last reads the last, and no one its product
+            row[t] = B + int64_t(min(8 * (warp + kDrlWarps * t) + (lane >> 2), n - 1)) * ldb + from + 2 * (lane & 3);
+#pragma unroll
+        for (int u = 0; u < DEPTH; ++u) fetch(u, u * kGroup);
+    }
+
+    __device__ __forceinline__ void fetch(int u, int k0) {
+        if (k0 >= k) return;
+        const int at = k0 + 2 * (threadIdx.x & 3);
+        if (wide && k0 + kGroup <= k) {
+#pragma unroll
+            for (int t = 0; t < CT; ++t) b[u][t] = __ldcg(reinterpret_cast<const double2*>(row[t] + k0));
+        } else {
+#pragma unroll
+            for (int t = 0; t < CT; ++t)
+                b[u][t] = make_double2(at < k ? __ldcg(row[t] + k0) : 0.0, at + 1 < k ? __ldcg(row[t] + k0 + 1) : 0.0);
+        }
+    }
+
+    // acc += the product; A has zeros from column k to the end of its last group.
+    __device__ __forceinline__ void run(double (&acc)[RT][CT][2], const double* A, int ld) {
+        const int lane = threadIdx.x & 31;
+        const double* mine = A + (lane >> 2) * ld + 2 * (lane & 3);
+        for (int k0 = 0; k0 < k; k0 += DEPTH * kGroup) {
+#pragma unroll
+            for (int u = 0; u < DEPTH; ++u) {
+                const int at = k0 + u * kGroup;
+                if (at < k) {
+                    double2 a[RT];
+#pragma unroll
+                    for (int rt = 0; rt < RT; ++rt) a[rt] = *reinterpret_cast<const double2*>(mine + 8 * rt * ld + at);
+#pragma unroll
+                    for (int t = 0; t < CT; ++t)
+#pragma unroll
+                        for (int rt = 0; rt < RT; ++rt) mma_f64(acc[rt][t][0], acc[rt][t][1], a[rt].x, b[u][t].x);
+#pragma unroll
+                    for (int t = 0; t < CT; ++t)
+#pragma unroll
+                        for (int rt = 0; rt < RT; ++rt) mma_f64(acc[rt][t][0], acc[rt][t][1], a[rt].y, b[u][t].y);
+                    fetch(u, at + DEPTH * kGroup);
+                }
+            }
+        }
+    }
+};
+
+template <int RT, int CT>
+__global__ void __launch_bounds__(kDrlWarps * 32, 1)
+    drl_kernel(DrlDev P, DrlSignal S, const int* __restrict__ list, int64_t count, const int* __restrict__ count_dev,
+               double* __restrict__ x, int64_t ldx) {
+    constexpr int kRows = 8 * RT;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ DrlTile<kRows> tile;
+    if (count_dev) count = min(count, int64_t(*count_dev));
+    const int c = P.c, m = P.m, cp = (c + 7) / 8 * 8, ld = drl_lds(cp);
+    double* F = reinterpret_cast<double*>(smem);  // (kRows, ld)
+    double* KS = F + kRows * ld;                  // (kRows, ld)
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const double nu8 = power_8(P.nu);
+    const bool plain = !(nu8 + power_8(P.init) > 1e-200);
+    StreamedProduct<RT, CT> product;
+    double acc[RT][CT][2];
+    auto clear = [&] {
+#pragma unroll
+        for (int rt = 0; rt < RT; ++rt)
+#pragma unroll
+            for (int t = 0; t < CT; ++t) acc[rt][t][0] = acc[rt][t][1] = 0.0;
+    };
+    for (int64_t p0 = int64_t(blockIdx.x) * kRows; p0 < count; p0 += int64_t(gridDim.x) * kRows) {
+        open_tile(tile, S, m, list, p0, count);
+        // K^T s: the signals in F, cp measurements at a time.
+        clear();
+        for (int from = 0; from < m; from += cp) {
+            const int here = min(cp, m - from);
+            product.open(P.k_t, m, c, from, here);
+            for (int e = tid; e < kRows * cp; e += blockDim.x) {
+                const int r = e / cp, i = e - r * cp;
+                const int64_t voxel = tile.vox[r];
+                F[r * ld + i] = voxel >= 0 && i < here ? signal_at(S, voxel, from + i) : 0.0;
+            }
+            __syncthreads();
+            product.run(acc, F, ld);
+            __syncthreads();
+        }
+#pragma unroll
+        for (int rt = 0; rt < RT; ++rt)
+#pragma unroll
+            for (int t = 0; t < CT; ++t) {
+                const int d = 8 * (warp + kDrlWarps * t) + 2 * (lane & 3);
+                if (d < cp)
+                    *reinterpret_cast<double2*>(KS + (8 * rt + (lane >> 2)) * ld + d) =
+                        make_double2(acc[rt][t][0], acc[rt][t][1]);
+            }
+        for (int e = tid; e < kRows * cp; e += blockDim.x) {
+            const int r = e / cp, d = e - r * cp;
+            F[r * ld + d] = tile.vox[r] >= 0 && d < c ? P.init : 0.0;
+        }
+        if (P.n_iter > 0) product.open(P.gram, c, c, 0, c);
+        __syncthreads();
+        for (int it = 0; it < P.n_iter; ++it) {
+            // The prediction K^T K f of every voxel of the tile.
+            clear();
+            product.run(acc, F, ld);
+            if (it + 1 < P.n_iter) product.open(P.gram, c, c, 0, c);
+            // The update overwrites F: every warp is done reading it first.
+            __syncthreads();
+            if (!update_tile<RT, CT>(tile, acc, F, KS, ld, c, nu8, plain)) break;
+        }
+        for (int e = tid; e < kRows * cp; e += blockDim.x) {
+            const int r = e / cp, d = e - r * cp;
+            const int64_t voxel = tile.vox[r];
+            if (voxel >= 0 && d < c) x[voxel * ldx + d] = F[r * ld + d];
+        }
+        __syncthreads();
+    }
+}
+
+template <int RT, typename Kernel>
+void launch_variant(Kernel kernel, const DrlDev& P, const DrlSignal& S, const int* list, int64_t count,
+                    const int* count_dev, double* x, int64_t ldx, cudaStream_t st, const char* name) {
     const size_t smem = drl_smem_bytes(P.c);
     cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
                "cudaFuncSetAttribute");
@@ -323,7 +418,7 @@ size_t drl_smem_bytes(int c) {
     const int cp = (c + 7) / 8 * 8;
     if (c <= kResidentMaxC) return (2 * size_t(8 * kNarrowRt) * drl_ldf(cp) + size_t(cp) * drl_ldg(cp)) * sizeof(double);
     const size_t rows = c <= kNarrowMaxC ? 8 * kNarrowRt : 8 * kWideRt;
-    return (2 * rows * drl_ldf(cp) + 2 * size_t(kDrlChunk) * drl_ldg(cp)) * sizeof(double);
+    return 2 * rows * drl_lds(cp) * sizeof(double);
 }
 
 bool drl_fits(int c) { return c >= 1 && c <= kWideMaxC; }
@@ -336,11 +431,19 @@ void launch_drl_listed(const DrlDev& P, const DrlSignal& S, const int* list, int
         return;
     }
     if (P.c <= kResidentMaxC)
-        launch_variant<kNarrowRt, 1, true>(P, S, list, count, count_dev, x, ldx, st, "drl_kernel_resident");
-    else if (P.c <= kNarrowMaxC)
-        launch_variant<kNarrowRt, kNarrowCt, false>(P, S, list, count, count_dev, x, ldx, st, "drl_kernel");
-    else
-        launch_variant<kWideRt, kWideCt, false>(P, S, list, count, count_dev, x, ldx, st, "drl_kernel_wide");
+        launch_variant<kNarrowRt>(drl_resident_kernel, P, S, list, count, count_dev, x, ldx, st, "drl_kernel_resident");
+    else if (P.c <= kNarrowMaxC) {
+        // As many column tiles per warp as c needs: the products of a warp's columns past c are wasted.
+        const int ct = (P.c + 8 * kDrlWarps - 1) / (8 * kDrlWarps);
+        launch_variant<kNarrowRt>(ct == 2   ? drl_kernel<kNarrowRt, 2>
+                                  : ct == 3 ? drl_kernel<kNarrowRt, 3>
+                                  : ct == 4 ? drl_kernel<kNarrowRt, 4>
+                                            : drl_kernel<kNarrowRt, kNarrowCt>,
+                                  P, S, list, count, count_dev, x, ldx, st, "drl_kernel");
+    } else {
+        launch_variant<kWideRt>(P.c <= 8 * kDrlWarps * 7 ? drl_kernel<kWideRt, 7> : drl_kernel<kWideRt, kWideCt>, P, S,
+                                list, count, count_dev, x, ldx, st, "drl_kernel_wide");
+    }
 }
 
 void launch_drl(const DrlDev& P, const double* signals, int64_t v, double* fods, cudaStream_t st) {

@@ -231,3 +231,21 @@ def test_tensor_core_drl_refuses_sizes_it_does_not_take(cuda, drl_fixture):
         solver.set_precision("tf32x3")
     with pytest.raises(ValueError, match="precision must be"):
         solver.set_precision("fp16")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize(("n_meas", "n_dirs", "n_vox"),
+                         [(7, 65, 1), (65, 66, 33), (300, 128, 32), (131, 193, 31), (90, 257, 33), (641, 320, 5),
+                          (34, 321, 17), (90, 449, 16), (31, 640, 15)])
+@pytest.mark.parametrize(("nu", "init"), [(0.02, 0.01), (0.0, 1e-30)])
+def test_gpu_drl_at_the_edges_of_its_tiles(cuda, oracle, n_meas, n_dirs, n_vox, nu, init):
+    """The column tiles per warp, the voxel tile, directions and measurements that are odd or more than one pass
+    takes, and a start whose eighth power is out of the short division's range. Non-negative products, so
+    an iteration's relative error grows by a few roundings of sums of n_dirs terms: within the other sizes' 1e-9."""
+    rng = np.random.default_rng(n_dirs)
+    k = np.abs(rng.normal(size=(n_meas, n_dirs))) + 0.1
+    signals = np.abs(rng.normal(size=(n_vox, n_meas))) / 10
+    k_t, k_t_k = _products(k)
+    got = _device_drl(signals, k, nu, 20, init)
+    ref = oracle.drl(signals, k_t, k_t_k, nu, 20, init, n_threads=4)
+    np.testing.assert_allclose(got, ref, rtol=1e-9, atol=0)
