@@ -277,3 +277,29 @@ def test_csd_model_fits_a_volume_like_the_oracle(cuda, oracle, csd_fixture):
     scale = np.abs(ref).max(axis=1, keepdims=True)
     assert np.quantile((np.abs(got[finite] - ref) / scale).max(axis=1), 0.99) <= 2e-7
     assert (fit.fods[0][~mask] == 0).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("c", [1, 8, 15, 16, 17, 32, 33, 45, 48, 49])
+@pytest.mark.parametrize(("k", "n"), [(1, 1), (31, 5), (160, 149), (161, 37), (300, 1000), (1100, 20)])
+def test_gpu_solve_at_the_edges_of_its_tiles(cuda, oracle, c, k, n):
+    """Random problems around the tile rows, the constraint words and the size of C that shared memory takes,
+    with and without unconstrained directions. Two backward-stable solves of a system of condition kappa differ by
+    a small multiple of c eps kappa, and by the rounding of M^T s, whose m terms may cancel, through the
+    smallest eigenvalue; a voxel whose set differs in a step by rounding would differ by far more."""
+    from larmor_b200 import _core
+
+    rng = np.random.default_rng(1000 * c + k)
+    m = max(20, c // 2)
+    initial, forward = rng.normal(size=(max(1, c // 3), m)) / m, rng.normal(size=(m, c))
+    constraint = rng.normal(size=(k, c))
+    signals = rng.normal(size=(n, m)) * rng.choice([1.0, 0.05], size=(n, 1))
+    args = (initial, forward, constraint, 1.0, 0.1, 12)
+    fods, conv = _core.fit_csd(signals, *args, 1)
+    ref, rconv = oracle.fit_csd(signals, *args, n_threads=4)
+    np.testing.assert_array_equal(conv, rconv)
+    gram = forward.T @ forward + np.eye(c)
+    kappa = np.linalg.norm(gram + constraint.T @ constraint, 2) / np.linalg.eigvalsh(gram)[0]
+    bound = 16 * c * 2.0**-53 * kappa * np.linalg.norm(ref, axis=1)
+    bound += 2 * m * 2.0**-53 * np.linalg.norm(np.abs(signals) @ np.abs(forward), axis=1) / np.linalg.eigvalsh(gram)[0]
+    assert np.all(np.linalg.norm(fods - ref, axis=1) <= bound)
