@@ -31,6 +31,19 @@ void clear_timed() {
 
 void set_error(const std::string& message) { last_error = message; }
 
+void raise_smem_limit(const void* kernel, size_t bytes) {
+    static std::mutex mutex;
+    static std::map<std::pair<int, const void*>, size_t> granted;
+    int device = 0;
+    cuda_check(cudaGetDevice(&device), "cudaGetDevice");
+    std::lock_guard<std::mutex> lock(mutex);
+    size_t& most = granted[{device, kernel}];
+    if (bytes <= most) return;
+    cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)),
+               "cudaFuncSetAttribute");
+    most = bytes;
+}
+
 namespace {
 std::mutex settings_mutex;
 std::map<std::string, int64_t> settings;

@@ -83,6 +83,16 @@ struct LaunchScope {
     cudaEvent_t start = nullptr;
 };
 
+// Lets launches of the kernel on this device take `bytes` of dynamic shared memory. The permission is only ever
+// raised: it belongs to the kernel, not to a launch, and another thread's smaller call would take it from under
+// this one's.
+void raise_smem_limit(const void* kernel, size_t bytes);
+
+template <class Kernel>
+void allow_smem(Kernel* kernel, size_t bytes) {
+    raise_smem_limit(reinterpret_cast<const void*>(kernel), bytes);
+}
+
 // Launch settings (lar_set_launch_setting): 0 when a setting is unset, which keeps the
 // library's own choice. A tuner sets them; results never depend on them.
 int64_t launch_setting(const char* name);

@@ -1170,9 +1170,7 @@ constexpr size_t kCSmem = kCWarps * sizeof(WarpShared);
 template <class Src>
 void allow_smem() {
     static_assert(kCSmem <= 200 * 1024, "the re-fit's shared state outgrows an SM");
-    cuda_check(cudaFuncSetAttribute(constrained_fit_kernel<Src>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(kCSmem)),
-               "cudaFuncSetAttribute");
+    allow_smem(constrained_fit_kernel<Src>, kCSmem);
 }
 
 // The shared-memory re-fit is used while a warp's state stays within this many bytes (at least
@@ -1196,8 +1194,7 @@ int global_resident_warps() {
 
 template <class Kernel>
 void allow_refit_smem(Kernel kernel, size_t bytes) {
-    cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)),
-               "cudaFuncSetAttribute");
+    allow_smem(kernel, bytes);
 }
 
 // Where the fast re-fit runs: DKI's constraints and a table whose rows fit a warp's state.
@@ -1227,8 +1224,7 @@ void launch_batch_refit(const DkiBatchJob* jobs, int n_jobs, int fast_jobs, int 
                         int weighted, int* queue, double* workspace, int slots, size_t slot_doubles,
                         cudaStream_t stream) {
     const int blocks = std::max(1, slots / kCWarps);
-    cuda_check(cudaFuncSetAttribute(batch_refit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kCSmem)),
-               "cudaFuncSetAttribute");
+    allow_smem(batch_refit_kernel, kCSmem);
     cuda_check(cudaMemsetAsync(queue, 0, 2 * sizeof(int), stream), "cudaMemsetAsync");
     if (fast_jobs > 0) {
         const int n = std::min(n_max, kFastMaxRows);

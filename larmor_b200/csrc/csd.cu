@@ -468,8 +468,7 @@ bool launch_tiles(const CsdDev& P, const double* signals, int64_t v, double* fod
                   cudaStream_t st) {
     const size_t smem = TileShape<T>::bytes(P.k);
     if (P.k > 1024 || smem > 220 * 1024) return false;  // (a set is a word per lane)
-    cuda_check(cudaFuncSetAttribute(csd_tiles_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
-               "cudaFuncSetAttribute");
+    allow_smem(csd_tiles_kernel<T>, smem);
     int per_sm = 0;
     cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, csd_tiles_kernel<T>, kTileWarps * 32, smem),
                "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
@@ -557,8 +556,7 @@ int lar_fit_csd(lar_csd csd, const double* signals, int64_t v, double* fods, uin
         const int warps = int(std::max<size_t>(1, std::min<size_t>(4, (200 * 1024) / per_warp)));
         const size_t smem = per_warp * warps;
         auto kernel = csd_kernel;
-        cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
-                   "cudaFuncSetAttribute");
+        allow_smem(kernel, smem);
         int per_sm = 0;
         cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, smem),
                    "cudaOccupancyMaxActiveBlocksPerMultiprocessor");

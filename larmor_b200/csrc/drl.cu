@@ -399,8 +399,7 @@ template <int RT, typename Kernel>
 void launch_variant(Kernel kernel, const DrlDev& P, const DrlSignal& S, const int* list, int64_t count,
                     const int* count_dev, double* x, int64_t ldx, cudaStream_t st, const char* name) {
     const size_t smem = drl_smem_bytes(P.c);
-    cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
-               "cudaFuncSetAttribute");
+    allow_smem(kernel, smem);
     int per_sm = 0;
     cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kDrlWarps * 32, smem),
                "cudaOccupancyMaxActiveBlocksPerMultiprocessor");

@@ -526,8 +526,7 @@ void launch_drl_tc(const DrlDev& P, const float* gtc, const DrlSignal& S, const 
     require(drl_tc_fits(P.c), "the tensor-core dRL takes 65 to 320 directions");
     const size_t smem = drl_tc_smem_bytes(P.c);
     require(smem <= 227 * 1024, "the tensor-core dRL's shared memory outgrows an SM");
-    cuda_check(cudaFuncSetAttribute(drl_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
-               "cudaFuncSetAttribute");
+    allow_smem(drl_tc_kernel, smem);
     const int64_t tiles = (count + kTcN - 1) / kTcN;
     const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(tiles, sm_count()));
     LaunchScope scope("drl_tc_kernel", st);

@@ -346,8 +346,7 @@ inline int small_block(int n, int raw_bytes, size_t per_value) {
 template <class Kernel>
 void set_smem(Kernel kernel, size_t bytes) {
     require(bytes <= 227 * 1024, "the design has too many measurements for the shared-memory fit");
-    cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)),
-               "cudaFuncSetAttribute");
+    allow_smem(kernel, bytes);
 }
 
 // Scratch layout for a constrained fit of v voxels: [count, two queues] ints, voxel ids, scaled

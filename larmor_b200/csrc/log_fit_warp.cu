@@ -547,8 +547,7 @@ int64_t warp_fit_residency(const WarpLayout<T>& lay) {
     const size_t smem = lay.bytes(WARPS);
     if (smem > 227 * 1024) return 0;
     auto kernel = fit_log_warp_kernel<T, DKI, Src, WARPS>;
-    cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
-               "cudaFuncSetAttribute");
+    allow_smem(kernel, smem);
     int per_sm = 0;
     cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, WARPS * 32, smem),
                "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
@@ -635,8 +634,7 @@ void launch_batch_log_warp_impl(const DkiBatchJob* jobs, const int64_t* first, i
                                 int64_t tickets, int weighted, int max_rw, double tol, int* queue,
                                 const BatchViolators& violators, cudaStream_t stream) {
     auto kernel = batch_log_warp_kernel<WARPS>;
-    cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
-               "cudaFuncSetAttribute");
+    allow_smem(kernel, smem);
     int per_sm = 0;
     cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, WARPS * 32, smem),
                "cudaOccupancyMaxActiveBlocksPerMultiprocessor");

@@ -1196,8 +1196,7 @@ int lar_fit_lsi(lar_lsi_design design, const double* signals, int64_t v, int onl
         // Constraint columns per lane: 10 up to 320 constraints (302 with the 300-direction grid),
         // else kColsPerLane.
         auto kernel = h.k <= 320 ? lsi_kernel<10> : lsi_kernel<kColsPerLane>;
-        cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
-                   "cudaFuncSetAttribute");
+        allow_smem(kernel, smem);
         int per_sm = 1;  // the marked voxels are few: one CTA per SM looks for them
         if (!grouped)
             cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kLsiWarps * 32, smem),
@@ -1225,10 +1224,8 @@ int lar_fit_lsi(lar_lsi_design design, const double* signals, int64_t v, int onl
         if (grouped) {
             int* redo = reinterpret_cast<int*>(base + 256);
             launch_rows_product(signals, v, D.m, D.qt, D.n, x, st);
-            cuda_check(cudaFuncSetAttribute(plan.main, cudaFuncAttributeMaxDynamicSharedMemorySize, int(plan.main_smem)),
-                       "cudaFuncSetAttribute");
-            cuda_check(cudaFuncSetAttribute(plan.qr, cudaFuncAttributeMaxDynamicSharedMemorySize, int(plan.qr_smem)),
-                       "cudaFuncSetAttribute");
+            allow_smem(plan.main, plan.main_smem);
+            allow_smem(plan.qr, plan.qr_smem);
             // One CTA per SM (its shared memory); a small call spreads its voxels over the SMs.
             const unsigned grid = unsigned(std::min<int64_t>(v, sm_count()));
             {

@@ -1586,8 +1586,7 @@ __global__ void __launch_bounds__(kMtWarps * 32, 4) batch_hr_fractions_kernel(Mf
 template <class Kernel>
 int64_t resident_slots(Kernel kernel, size_t smem, int64_t items, const char* setting, int warps = kMtWarps) {
     require(smem <= 200 * 1024, "the kernel has too many columns for the shared-memory solver");
-    cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
-               "cudaFuncSetAttribute");
+    allow_smem(kernel, smem);
     int per_sm = 0;
     cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, smem),
                "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
@@ -1633,8 +1632,7 @@ inline void launch_correlate(const SignalDev& S, const int* list, int64_t count,
         const unsigned gx = unsigned(std::max<int64_t>(1, std::min<int64_t>(units, sm_count() / gy)));
         const size_t smem = corr_tc_smem(R.m, S.w ? S.ci : 0);
         auto run = [&](auto kernel) {
-            cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
-                       "cudaFuncSetAttribute");
+            allow_smem(kernel, smem);
             LaunchScope scope("correlate_kernel", st);
             kernel<<<dim3(gx, gy), kCorrTcWarps * 32, smem, st>>>(S, list, count, count_dev, R.k, R.c, corr, ldc);
             cuda_check(cudaGetLastError(), "correlate_tc_kernel launch");
@@ -2093,8 +2091,7 @@ struct MfodBatch {
             const unsigned gy = unsigned((c_max + kCorrTcCols - 1) / kCorrTcCols);
             const unsigned gx = std::max(1u, unsigned(sm_count()) / gy);
             auto run = [&](auto kernel) {
-                cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
-                           "cudaFuncSetAttribute");
+                allow_smem(kernel, smem);
                 LaunchScope scope("batch_correlate_kernel", st);
                 kernel<<<dim3(gx, gy), kCorrTcWarps * 32, smem, st>>>(B, list);
                 cuda_check(cudaGetLastError(), "batch_correlate_tc_kernel launch");
@@ -2278,8 +2275,7 @@ void mfod_batch_run(MfodBatch* b, cudaStream_t st) {
         }
         if (round == 0 && b->fx_doubles > 0) {
             const size_t smem = corr_tc_smem(b->ks_m, 0);
-            cuda_check(cudaFuncSetAttribute(batch_ks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
-                       "cudaFuncSetAttribute");
+            allow_smem(batch_ks_kernel, smem);
             LaunchScope scope("batch_ks_kernel", st);
             const unsigned gy = unsigned((b->c_lr_max + ci + kCorrTcCols - 1) / kCorrTcCols);
             batch_ks_kernel<<<dim3(unsigned(sm_count()) / gy, gy), kCorrTcWarps * 32, smem, st>>>(B);

@@ -881,9 +881,7 @@ int lar_find_peaks(lar_peak_sphere sphere, const double* coeffs, int64_t n, int6
             LaunchScope scope("peak_count_kernel", st);
             if (tile_fits(nv)) {
                 const size_t smem = tile_bytes(nv);
-                cuda_check(cudaFuncSetAttribute(peak_count_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                int(smem)),
-                           "cudaFuncSetAttribute");
+                allow_smem(peak_count_tile_kernel, smem);
                 peak_count_tile_kernel<<<unsigned((n + kTileVoxels - 1) / kTileVoxels), kTileThreads, smem, st>>>(
                     on_sphere, n, lds, sphere->neighbours.ptr, antipodes, nv, counts, masks);
             } else {
@@ -927,8 +925,7 @@ int lar_find_peaks(lar_peak_sphere sphere, const double* coeffs, int64_t n, int6
                                                : (lcap == 12 ? climb_pool_kernel<12, false> : climb_pool_kernel<20, false>));
             const size_t smem = staged ? size_t(4 * kStagedDim * kColumnLd) * sizeof(double) : 0;
             if (staged)
-                cuda_check(cudaFuncSetAttribute(climber, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
-                           "cudaFuncSetAttribute");
+                allow_smem(climber, smem);
             int per_sm = 0;
             cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, climber, 128, smem),
                        "cudaOccupancyMaxActiveBlocksPerMultiprocessor");

@@ -591,8 +591,7 @@ void launch_plain_lsi(const PlainLsi& D, const float* signals, int64_t v, float*
     require(D.n <= kPlainLsiMaxParameters && D.k <= kPlainLsiMaxConstraints,
             "the plain FP32 LSI fit takes at most 63 parameters and 512 constraints");
     const size_t smem = plain_lsi_warp_bytes(D.k) * kPlainWarps;
-    cuda_check(cudaFuncSetAttribute(plain_lsi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
-               "cudaFuncSetAttribute");
+    allow_smem(plain_lsi_kernel, smem);
     int per_sm = 0;
     cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, plain_lsi_kernel, kPlainWarps * 32, smem),
                "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
@@ -610,8 +609,7 @@ void launch_plain_fp32(const PlainStage& lr, const PlainStage& hr, const float* 
     const int ng = std::max(1, hr.nb);
     const size_t smem = plain_warp_bytes(lr.m, std::max(lr.c, hr.c), ng) * kPlainWarps;
     require(smem <= 200 * 1024, "the plain FP32 fit's per-warp state does not fit in shared memory");
-    cuda_check(cudaFuncSetAttribute(plain_fp32_mfod_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
-               "cudaFuncSetAttribute");
+    allow_smem(plain_fp32_mfod_kernel, smem);
     int per_sm = 0;
     cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, plain_fp32_mfod_kernel, kPlainWarps * 32, smem),
                "cudaOccupancyMaxActiveBlocksPerMultiprocessor");

@@ -153,8 +153,7 @@ void launch_expand(const double* in, int64_t v, int64_t lda, int ca, const doubl
     const int slices = (ncoef + most - 1) / most;
     const int width = ((ncoef + slices - 1) / slices + 7) / 8 * 8;
     const size_t smem = size_t(4 * KS) * (width + 4) * sizeof(double);
-    cuda_check(cudaFuncSetAttribute(expand_sh_kernel<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
-               "cudaFuncSetAttribute");
+    allow_smem(expand_sh_kernel<KS>, smem);
     const int64_t blocks = (v + 16 * kExpandWarps - 1) / (16 * kExpandWarps);
     const unsigned gx = unsigned(std::max<int64_t>(1, std::min<int64_t>(blocks, 2 * sm_count() / slices)));
     LaunchScope scope("project_sh_kernel", st);
