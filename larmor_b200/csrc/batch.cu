@@ -145,16 +145,17 @@ int lar_batch_finalize(lar_batch batch) {
         require(batch != nullptr, "batch must not be NULL");
         require(!batch->finalized, "the batch is already finalized");
         lar_batch_s& b = *batch;
-        // DTI: tickets of kDtiBatchBlock voxels.
+        // DTI: tickets of dti_ticket_voxels.
         std::vector<int64_t> voxels;
-        for (const auto& j : b.dti) {
-            voxels.push_back(j.v);
-            b.dti_nmax = std::max(b.dti_nmax, j.d.n);
-        }
+        for (const auto& j : b.dti) b.dti_nmax = std::max(b.dti_nmax, j.d.n);
         if (!b.dti.empty()) {
             require(batch_dti_smem(b.dti_nmax) <= 227 * 1024,
                     "a DTI table of the batch has too many measurements for the shared-memory fit");
-            const auto first = ticket_starts(voxels, kDtiBatchBlock);
+            std::vector<int64_t> first(1, 0);
+            for (const auto& j : b.dti) {
+                const int64_t block = dti_ticket_voxels(j.v, j.d.n);
+                first.push_back(first.back() + (j.v + block - 1) / block);
+            }
             b.dti_tickets = first.back();
             upload_vector(b.d_dti, b.dti);
             upload_vector(b.dti_first, first);

@@ -69,12 +69,13 @@ struct BatchViolators {
 };
 
 // Voxels per ticket of the family stages.
-constexpr int kDtiBatchBlock = 32;   // one CTA of the DTI fit (thread per voxel)
+constexpr int kDtiBatchThreads = 64;  // one CTA of the DTI fit
 constexpr int kDkiVoxelsPerWarp = 4;  // a ticket of the DKI log fit: 4 voxels per warp of its CTA
 constexpr int kMapsBatchVoxels = 128;
 
 // Launch shapes and shared memory of the family stages (sized for the largest table).
 size_t batch_dti_smem(int n_max);
+int dti_ticket_voxels(int64_t v, int n);  // of one ticket of a volume of v voxels on n measurements
 // Warps per CTA of the DKI log fit (12, 8 or 4; 0: the largest table does not fit) and its
 // shared memory.
 int batch_log_warp_warps(int n_max, int p);

@@ -8,10 +8,10 @@
 // pseudo-inverse, the products Z[n][ab] = X_na X_nb of the normal matrix, constraints) is small
 // and shared by every voxel: each CTA stages it once into shared memory.
 //
-// DTI (p = 7): one thread per voxel. Each thread accumulates its 28 normal-matrix entries and
-// 7 right-hand sides in registers over the measurements (design operands are warp-uniform
-// shared-memory broadcasts), solves the 7 x 7 system by LU with partial pivoting in registers,
-// and finishes with the tensor's eigen-decomposition (cyclic Jacobi) and the DTI maps.
+// DTI (p = 7): two to eight neighbouring lanes per voxel (small_lanes). A lane accumulates the 28
+// normal-matrix entries and 7 right-hand sides in registers over its share of the measurements, a
+// butterfly sums the lanes' shares, each lane solves the 7 x 7 system by L D L^T in registers, and the first
+// finishes with the tensor's eigen-decomposition (cyclic Jacobi) and the DTI maps.
 
 #include <cmath>
 #include <cstdio>
@@ -69,219 +69,315 @@ __device__ __forceinline__ bool all_finite(const T (&v)[P]) {
     return ok;
 }
 
-// ---- the small-p thread-per-voxel IRLS --------------------------------------------------
+// ---- the IRLS of the 7-column design ------------------------------------------------------
 
-template <class T, int P>
-struct SmallFit {
-    static constexpr int PP = P * (P + 1) / 2;
-    // Shared memory: x, z, pinv^T (T), the CTA's log signals (T), its raw rows.
-    static size_t bytes(int n, int block, int raw_bytes) {
-        return size_t(n) * (2 * P + PP) * sizeof(T) + size_t(n) * block * sizeof(T) +
-               size_t(n) * block * raw_bytes + 16;
+constexpr int kSmallThreads = 64;
+constexpr int kSmallCtas = 6;  // an SM's, by registers: with eight the fit spills (79,912 voxels: 277 us against 274)
+
+// Lanes per voxel of a fit of v voxels on n measurements. More lanes shorten a voxel's serial chain, while each
+// adds its part of the sums' butterfly (35 values) and repeats the solve. Measured, microseconds with 8, 4 and 2
+// lanes (one lane before: 115 to 139 up to 24,000 voxels of 31 measurements, 339 at 79,912):
+//   n = 31, v = 2,003: 42, 53, 75; 5,000: 53, 55, 76; 8,000: 76, 59, 76; 16,000: 113, 95, 98; 79,912: 464, 317, 274
+//   n = 94, v = 16,000: 204, 217, 219; 79,912: 801, 680, 700.   n = 134, v = 79,912: 906, 903, 971.
+__host__ __device__ inline int small_lanes(int64_t v, int n) { return v <= 5000 ? 8 : (v <= 10000 || n >= 80 ? 4 : 2); }
+
+// Row strides in shared memory: of x and pinv^T (7 entries in whole 16-byte loads, eight rows of which
+// fall in distinct banks), and of the log signals of `voxels` voxels.
+template <class T>
+__host__ __device__ constexpr int row_ld() { return sizeof(T) == 8 ? 10 : 12; }
+__host__ __device__ constexpr int voxel_ld(int voxels) { return voxels + 1; }
+
+template <class T>
+size_t small_bytes(int n, int voxels) {
+    return size_t(n) * (2 * row_ld<T>() + voxel_ld(voxels)) * sizeof(T);
+}
+
+// The first 8 entries of a row.
+__device__ __forceinline__ void load_row(const double* row, double (&x)[8]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const double2 two = reinterpret_cast<const double2*>(row)[i];
+        x[2 * i] = two.x;
+        x[2 * i + 1] = two.y;
     }
-};
+}
+__device__ __forceinline__ void load_row(const float* row, float (&x)[8]) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const float4 four = reinterpret_cast<const float4*>(row)[i];
+        x[4 * i] = four.x;
+        x[4 * i + 1] = four.y;
+        x[4 * i + 2] = four.z;
+        x[4 * i + 3] = four.w;
+    }
+}
 
 // Packed index of (a, b), a <= b, in the upper triangle stored row by row.
 __host__ __device__ constexpr int packed(int a, int b, int p) { return a * p - a * (a - 1) / 2 + (b - a); }
+
+__host__ __device__ constexpr int packed_row(int k, int p) {
+    int a = 0;
+    while (k >= packed(a + 1, a + 1, p)) ++a;
+    return a;
+}
+__host__ __device__ constexpr int packed_column(int k, int p) {
+    return k - packed(packed_row(k, p), packed_row(k, p), p) + packed_row(k, p);
+}
 
 // Solves the symmetric system g x = b (g packed, P x P) in place in b by L D L^T. Returns false
 // when a pivot is exactly zero, the weighted normal equations being singular (weights that
 // underflow to zero on most measurements), as the reference's zero LU pivot test does
 // (cpp/src/dwi/log_fit.cpp:128-133).
+// Every index is fixed at compile time by loops from 0 with a test: loops from j + 1 were not unrolled, and
+// the matrix lay in local memory, written and read in each iteration (half a gigabyte at 79,912 voxels).
 template <class T, int P>
 __device__ __forceinline__ bool ldlt_solve(T (&g)[P * (P + 1) / 2], T (&b)[P]) {
-    // In place: g(j, j) <- d_j, g(j, i) (j < i) <- L(i, j).
+    // In place: g(j, j) <- 1 / d_j, g(j, i) (j < i) <- L(i, j); behind column j its update is taken from the rest.
     bool ok = true;
 #pragma unroll
     for (int j = 0; j < P; ++j) {
-        T d = g[packed(j, j, P)];
-#pragma unroll
-        for (int k = 0; k < j; ++k) {
-            const T l = g[packed(k, j, P)];
-            d = fma(-l * g[packed(k, k, P)], l, d);
-        }
+        const T d = g[packed(j, j, P)];
         ok &= (d != T(0));
-        g[packed(j, j, P)] = d;
         const T inv = T(1) / d;
+        T l[P];
 #pragma unroll
-        for (int i = j + 1; i < P; ++i) {
-            T s = g[packed(j, i, P)];
+        for (int i = 0; i < P; ++i)
+            if (i > j) {
+                l[i] = g[packed(j, i, P)] * inv;
+                b[i] = fma(-l[i], b[j], b[i]);
+            }
 #pragma unroll
-            for (int k = 0; k < j; ++k) s = fma(-g[packed(k, i, P)] * g[packed(k, k, P)], g[packed(k, j, P)], s);
-            g[packed(j, i, P)] = s * inv;
-        }
+        for (int i = 0; i < P; ++i)
+#pragma unroll
+            for (int k = 0; k < P; ++k)
+                if (i > j && k >= i) g[packed(i, k, P)] = fma(-l[i], g[packed(j, k, P)], g[packed(i, k, P)]);
+#pragma unroll
+        for (int i = 0; i < P; ++i)
+            if (i > j) g[packed(j, i, P)] = l[i];
+        b[j] *= inv;
     }
     if (!ok) return false;
 #pragma unroll
-    for (int i = 0; i < P; ++i)
-#pragma unroll
-        for (int k = 0; k < i; ++k) b[i] = fma(-g[packed(k, i, P)], b[k], b[i]);
-#pragma unroll
-    for (int i = 0; i < P; ++i) b[i] = b[i] / g[packed(i, i, P)];
-#pragma unroll
     for (int i = P - 1; i >= 0; --i)
 #pragma unroll
-        for (int k = i + 1; k < P; ++k) b[i] = fma(-g[packed(i, k, P)], b[k], b[i]);
+        for (int k = 0; k < P; ++k)
+            if (k > i) b[i] = fma(-g[packed(i, k, P)], b[k], b[i]);
     return true;
 }
 
-// Fits one voxel from its log signals ys[j * stride] and leaves its scaled parameters in p;
-// returns the number of weighted fits. Follows reweighted_fit (cpp/src/dwi/log_fit.cpp:114-147)
-// from the ordinary fit pinv y (:251).
-template <class T, int P>
-__device__ __forceinline__ int fit_voxel_small(const T* __restrict__ xs, const T* __restrict__ zs,
-                                               const T* __restrict__ pinvt, int n,
-                                               const T* __restrict__ ys, int stride, bool weighted,
-                                               int max_rw, T tol, T (&p)[P]) {
-    constexpr int PP = P * (P + 1) / 2;
-    T ord[P];
+// The sum and the maximum over the G lanes of a voxel, the same bits in each (mask: those lanes).
+template <int G, class T, int N>
+__device__ __forceinline__ void lanes_sum(T (&v)[N], unsigned mask) {
 #pragma unroll
-    for (int a = 0; a < P; ++a) ord[a] = T(0);
-#pragma unroll 2
-    for (int j = 0; j < n; ++j) {
-        const T y = ys[j * stride];
+    for (int o = 1; o < G; o *= 2)
 #pragma unroll
-        for (int a = 0; a < P; ++a) ord[a] = fma(pinvt[j * P + a], y, ord[a]);
-    }
+        for (int i = 0; i < N; ++i) v[i] += __shfl_xor_sync(mask, v[i], o);
+}
+template <int G, class T>
+__device__ __forceinline__ T lanes_max(T v, unsigned mask) {
 #pragma unroll
-    for (int a = 0; a < P; ++a) p[a] = ord[a];
-    if (!weighted || !all_finite(ord)) return 0;
+    for (int o = 1; o < G; o *= 2) v = fmax(v, __shfl_xor_sync(mask, v, o));
+    return v;
+}
 
-    T mx = -INFINITY;
+// Fits one voxel from its log signals ys[j * stride], lane g of its G, and leaves its scaled parameters in p
+// (the same in every lane); returns the number of weighted fits. Follows reweighted_fit
+// (cpp/src/dwi/log_fit.cpp:114-147) from the ordinary fit pinv y (:251).
+// What bounds it: the latencies of a measurement's chain (a product, an exponential, the sums) with twelve warps
+// in an SM, and the lanes that wait for their warp's slowest voxel: 44% of the FP64 pipe at 79,912 voxels.
+template <class T, int G>
+__device__ __forceinline__ int fit_voxel_small(const T* __restrict__ xs, const T* __restrict__ pinvt, int n,
+                                               const T* __restrict__ ys, int stride, bool weighted, int max_rw, T tol,
+                                               T (&p)[7]) {
+    constexpr int P = 7, PP = 28, LD = row_ld<T>();
+    const int g = int(threadIdx.x) % G;
+    const unsigned mask = ((1u << G) - 1u) << (threadIdx.x % 32 - g);
+    auto ordinary = [&] {
+        T sum[P];
+#pragma unroll
+        for (int a = 0; a < P; ++a) sum[a] = T(0);
 #pragma unroll 2
-    for (int j = 0; j < n; ++j) {
+        for (int j = g; j < n; j += G) {
+            const T y = ys[j * stride];
+            T row[8];
+            load_row(pinvt + j * LD, row);
+#pragma unroll
+            for (int a = 0; a < P; ++a) sum[a] = fma(row[a], y, sum[a]);
+        }
+        lanes_sum<G>(sum, mask);
+#pragma unroll
+        for (int a = 0; a < P; ++a) p[a] = sum[a];
+    };
+    auto predict = [](const T (&x)[8], const T (&q)[P]) {
         T pred = T(0);
 #pragma unroll
-        for (int a = 0; a < P; ++a) pred = fma(xs[j * P + a], p[a], pred);
-        mx = fmax(mx, pred);
+        for (int a = 0; a < P; ++a) pred = fma(x[a], q[a], pred);
+        return pred;
+    };
+    ordinary();
+    if (!weighted || !all_finite(p)) return 0;
+    T mx = -INFINITY;
+#pragma unroll 2
+    for (int j = g; j < n; j += G) {
+        T x[8];
+        load_row(xs + j * LD, x);
+        mx = fmax(mx, predict(x, p));
     }
+    mx = lanes_max<G>(mx, mask);
     int it = 0;
     for (; it < max_rw; ++it) {
-        T g[PP], r[P];
+        T m[PP], r[P];
 #pragma unroll
-        for (int k = 0; k < PP; ++k) g[k] = T(0);
+        for (int k = 0; k < PP; ++k) m[k] = T(0);
 #pragma unroll
         for (int a = 0; a < P; ++a) r[a] = T(0);
 #pragma unroll 2
-        for (int j = 0; j < n; ++j) {
-            T pred = T(0);
+        for (int j = g; j < n; j += G) {
+            T x[8];
+            load_row(xs + j * LD, x);
+            const T w = dev_exp<T>(T(2) * (predict(x, p) - mx));
+            const T y = ys[j * stride];
+            // The products x_a x_b come from the row itself: a table of them was four times the loads.
+            T wx[P];
 #pragma unroll
-            for (int a = 0; a < P; ++a) pred = fma(xs[j * P + a], p[a], pred);
-            const T w = dev_exp<T>(T(2) * (pred - mx));
-            const T wy = w * ys[j * stride];
+            for (int a = 0; a < P; ++a) {
+                wx[a] = w * x[a];
+                r[a] = fma(wx[a], y, r[a]);
+            }
 #pragma unroll
-            for (int k = 0; k < PP; ++k) g[k] = fma(w, zs[j * PP + k], g[k]);
-#pragma unroll
-            for (int a = 0; a < P; ++a) r[a] = fma(wy, xs[j * P + a], r[a]);
+            for (int k = 0; k < PP; ++k) m[k] = fma(wx[packed_row(k, P)], x[packed_column(k, P)], m[k]);
         }
-        if (!ldlt_solve<T, P>(g, r) || !all_finite(r)) {
-#pragma unroll
-            for (int a = 0; a < P; ++a) p[a] = ord[a];
+        lanes_sum<G>(m, mask);
+        lanes_sum<G>(r, mask);
+        if (!ldlt_solve<T, P>(m, r) || !all_finite(r)) {
+            ordinary();
             return it + 1;
         }
         T change = T(0), mx_next = -INFINITY;
 #pragma unroll 2
-        for (int j = 0; j < n; ++j) {
-            T po = T(0), pn = T(0);
-#pragma unroll
-            for (int a = 0; a < P; ++a) {
-                po = fma(xs[j * P + a], p[a], po);
-                pn = fma(xs[j * P + a], r[a], pn);
-            }
+        for (int j = g; j < n; j += G) {
+            T x[8];
+            load_row(xs + j * LD, x);
+            const T po = predict(x, p), pn = predict(x, r);
             change = fmax(change, fabs(pn - po));
             mx_next = fmax(mx_next, pn);
         }
+        change = lanes_max<G>(change, mask);
+        mx = lanes_max<G>(mx_next, mask);
 #pragma unroll
         for (int a = 0; a < P; ++a) p[a] = r[a];
-        mx = mx_next;
         if (!(change > tol)) return it + 1;
     }
     return it;
 }
 
-// Stages x (n, p), z (n, pp) and pinv^T (n, p) into shared memory; returns the end.
-template <class T, int P>
+// Stages x and pinv^T (n, p) into shared memory; returns the end.
+template <class T>
 __device__ __forceinline__ T* stage_design(const LogDesignDevice<T>& d, T* sm) {
-    constexpr int PP = P * (P + 1) / 2;
-    const int n = d.n;
-    for (int i = threadIdx.x; i < n * P; i += blockDim.x) sm[i] = d.x[i];
-    for (int i = threadIdx.x; i < n * PP; i += blockDim.x) sm[n * P + i] = d.z[i];
-    for (int i = threadIdx.x; i < n * P; i += blockDim.x) sm[n * (P + PP) + i] = d.pinvt[i];
-    return sm + n * (2 * P + PP);
+    constexpr int P = 7, LD = row_ld<T>();
+    for (int i = threadIdx.x; i < d.n * 8; i += blockDim.x) {
+        const int j = i / 8, a = i % 8;
+        sm[j * LD + a] = a < P ? d.x[j * P + a] : T(0);
+        sm[(d.n + j) * LD + a] = a < P ? d.pinvt[j * P + a] : T(0);
+    }
+    return sm + 2 * d.n * LD;
 }
 
-template <class T, int P, int BLOCK, class Src>
-__global__ void __launch_bounds__(BLOCK) fit_log_small_kernel(LogDesignDevice<T> d, Src src, int64_t v,
-                                                              int weighted, int max_rw, T tol,
-                                                              double* __restrict__ params,
-                                                              uint8_t* __restrict__ broke,
-                                                              int32_t* __restrict__ iterations) {
+// The log signals of `count` voxels from `first`, measurement-major, the loads along the rows.
+template <class T, class Src>
+__device__ __forceinline__ void stage_signals(const Src& src, int64_t first, int count, int n, T* ys, int ld) {
+    for (int i = threadIdx.x; i < count * n; i += blockDim.x) {
+        const int local = i / n;
+        ys[(i - local * n) * ld + local] = src.template entry<T>(first + local, first * n + i);
+    }
+}
+
+template <class T, int G, class Src>
+__global__ void __launch_bounds__(kSmallThreads, kSmallCtas) fit_log_small_kernel(LogDesignDevice<T> d, Src src, int64_t v,
+                                                                     int weighted, int max_rw, T tol,
+                                                                     double* __restrict__ params,
+                                                                     uint8_t* __restrict__ broke,
+                                                                     int32_t* __restrict__ iterations) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* sm = reinterpret_cast<T*>(smem_raw);
-    constexpr int PP = P * (P + 1) / 2;
-    const int n = d.n;
-    T* ys = stage_design<T, P>(d, sm);
-    unsigned char* raw = reinterpret_cast<unsigned char*>(ys + n * BLOCK);
-    const int64_t first = int64_t(blockIdx.x) * BLOCK;
-    const int count = int(v - first < int64_t(BLOCK) ? v - first : int64_t(BLOCK));
-    src.template stage<T, BLOCK>(first, count, raw, ys);
+    const int n = d.n, voxels = blockDim.x / G, ld = voxel_ld(voxels), local = threadIdx.x / G;
+    T* ys = stage_design<T>(d, sm);
+    const int64_t first = int64_t(blockIdx.x) * voxels;
+    const int count = int(v - first < int64_t(voxels) ? v - first : int64_t(voxels));
+    stage_signals<T>(src, first, count, n, ys, ld);
     __syncthreads();
-    if (threadIdx.x >= count) return;
-    const int64_t voxel = first + threadIdx.x;
-    T p[P];
-    const int it = fit_voxel_small<T, P>(sm, sm + n * P, sm + n * (P + PP), n, ys + threadIdx.x, BLOCK,
-                                         weighted != 0, max_rw, tol, p);
+    if (local >= count) return;
+    const int64_t voxel = first + local;
+    T p[7];
+    const int it = fit_voxel_small<T, G>(sm, sm + n * row_ld<T>(), n, ys + local, ld, weighted != 0, max_rw, tol, p);
+    if (threadIdx.x % G) return;
 #pragma unroll
-    for (int a = 0; a < P; ++a) params[voxel * P + a] = double(p[a]) / d.scales64[a];
+    for (int a = 0; a < 7; ++a) params[voxel * 7 + a] = double(p[a]) / d.scales64[a];
     broke[voxel] = 0;
     if (iterations) iterations[voxel] = it;
 }
 
-template <class T, int BLOCK>
-__global__ void __launch_bounds__(BLOCK) fit_dti_maps_kernel(LogDesignDevice<T> d, FlooredSource src,
-                                                             int64_t v, int weighted, int max_rw, T tol,
-                                                             float* __restrict__ maps,
-                                                             uint8_t* __restrict__ npd,
-                                                             double* __restrict__ params) {
-    constexpr int P = 7, PP = 28;
+template <class T, int G>
+__global__ void __launch_bounds__(kSmallThreads, kSmallCtas) fit_dti_maps_kernel(LogDesignDevice<T> d, FlooredSource src,
+                                                                    int64_t v, int weighted, int max_rw, T tol,
+                                                                    float* __restrict__ maps,
+                                                                    uint8_t* __restrict__ npd,
+                                                                    double* __restrict__ params) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* sm = reinterpret_cast<T*>(smem_raw);
-    const int n = d.n;
-    T* ys = stage_design<T, P>(d, sm);
-    unsigned char* raw = reinterpret_cast<unsigned char*>(ys + n * BLOCK);
-    const int64_t first = int64_t(blockIdx.x) * BLOCK;
-    const int count = int(v - first < int64_t(BLOCK) ? v - first : int64_t(BLOCK));
-    src.template stage<T, BLOCK>(first, count, raw, ys);
+    const int n = d.n, voxels = blockDim.x / G, ld = voxel_ld(voxels), local = threadIdx.x / G;
+    T* ys = stage_design<T>(d, sm);
+    const int64_t first = int64_t(blockIdx.x) * voxels;
+    const int count = int(v - first < int64_t(voxels) ? v - first : int64_t(voxels));
+    stage_signals<T>(src, first, count, n, ys, ld);
     __syncthreads();
-    if (threadIdx.x >= count) return;
-    const int64_t voxel = first + threadIdx.x;
-    T p[P];
-    fit_voxel_small<T, P>(sm, sm + n * P, sm + n * (P + PP), n, ys + threadIdx.x, BLOCK, weighted != 0,
-                          max_rw, tol, p);
+    if (local >= count) return;
+    const int64_t voxel = first + local;
+    T p[7];
+    fit_voxel_small<T, G>(sm, sm + n * row_ld<T>(), n, ys + local, ld, weighted != 0, max_rw, tol, p);
+    if (threadIdx.x % G) return;
     T dt[6];
 #pragma unroll
     for (int a = 0; a < 6; ++a) dt[a] = p[a + 1] / d.scales[a + 1];
     if (params) {
 #pragma unroll
-        for (int a = 0; a < P; ++a) params[voxel * P + a] = double(p[a]) / d.scales64[a];
+        for (int a = 0; a < 7; ++a) params[voxel * 7 + a] = double(p[a]) / d.scales64[a];
     }
     dti_maps<T>(dt, voxel, v, maps, npd);
 }
 
 // The DTI family of a batch (batch.cuh): a persistent grid whose CTAs take tickets of
-// kDtiBatchBlock voxels of one volume from a device counter across every DTI volume; a CTA
+// dti_ticket_voxels(v, n) voxels of one volume from a device counter across every DTI volume; a CTA
 // restages the design when its ticket moves to another volume. Per voxel the same fit and maps
 // as fit_dti_maps_kernel (FP64).
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) batch_dti_kernel(const DtiBatchJob* __restrict__ jobs,
-                                                          const int64_t* __restrict__ first, int n_jobs,
-                                                          int weighted, int max_rw, double tol,
-                                                          int* __restrict__ queue) {
-    using T = double;
-    constexpr int P = 7;
+template <int G>
+__device__ __noinline__ void batch_dti_ticket(const DtiBatchJob& job, int64_t ticket, int weighted, int max_rw,
+                                              double tol, double* sm) {
+    const int n = job.d.n, local = threadIdx.x / G;
+    constexpr int kVoxels = kDtiBatchThreads / G, kLd = voxel_ld(kVoxels), LD = row_ld<double>();
+    double* ys = sm + 2 * n * LD;
+    const int64_t first = ticket * kVoxels;
+    const int count = int(job.v - first < int64_t(kVoxels) ? job.v - first : int64_t(kVoxels));
+    stage_signals<double>(FlooredSource{job.s, job.floor, n}, first, count, n, ys, kLd);
+    __syncthreads();
+    if (local < count) {
+        double p[7];
+        fit_voxel_small<double, G>(sm, sm + n * LD, n, ys + local, kLd, weighted != 0, max_rw, tol, p);
+        if (threadIdx.x % G == 0) {
+            double dt[6];
+#pragma unroll
+            for (int a = 0; a < 6; ++a) dt[a] = p[a + 1] / job.d.scales[a + 1];
+            dti_maps<double>(dt, first + local, job.v, job.maps, job.npd);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kDtiBatchThreads, kSmallCtas * kSmallThreads / kDtiBatchThreads)
+    batch_dti_kernel(const DtiBatchJob* __restrict__ jobs, const int64_t* __restrict__ first, int n_jobs, int weighted,
+                     int max_rw, double tol, int* __restrict__ queue) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ long long ticket;
-    T* sm = reinterpret_cast<T*>(smem_raw);
+    double* sm = reinterpret_cast<double*>(smem_raw);
     const int64_t total = first[n_jobs];
     int cur = -1;
     for (;;) {
@@ -291,29 +387,14 @@ __global__ void __launch_bounds__(BLOCK) batch_dti_kernel(const DtiBatchJob* __r
         if (t >= total) break;
         const int j = ticket_job(first, n_jobs, t);
         const DtiBatchJob& job = jobs[j];
-        const LogDesignDevice<T> d = job.d;
-        const int n = d.n;
-        T* ys = sm + n * (2 * P + P * (P + 1) / 2);
         if (j != cur) {
-            stage_design<T, P>(d, sm);
+            stage_design<double>(job.d, sm);
             cur = j;
         }
-        unsigned char* raw = reinterpret_cast<unsigned char*>(ys + n * BLOCK);
-        const int64_t v = job.v;
-        const int64_t block_first = (t - first[j]) * BLOCK;
-        const int count = int(v - block_first < int64_t(BLOCK) ? v - block_first : int64_t(BLOCK));
-        const FlooredSource src{job.s, job.floor, n};
-        src.template stage<T, BLOCK>(block_first, count, raw, ys);
-        __syncthreads();
-        if (threadIdx.x < count) {
-            const int64_t voxel = block_first + threadIdx.x;
-            T p[P];
-            fit_voxel_small<T, P>(sm, sm + n * P, sm + n * (P + P * (P + 1) / 2), n, ys + threadIdx.x, BLOCK,
-                                  weighted != 0, max_rw, T(tol), p);
-            T dt[6];
-#pragma unroll
-            for (int a = 0; a < 6; ++a) dt[a] = p[a + 1] / d.scales[a + 1];
-            dti_maps<T>(dt, voxel, v, job.maps, job.npd);
+        switch (small_lanes(job.v, job.d.n)) {
+            case 8: batch_dti_ticket<8>(job, t - first[j], weighted, max_rw, tol, sm); break;
+            case 4: batch_dti_ticket<4>(job, t - first[j], weighted, max_rw, tol, sm); break;
+            default: batch_dti_ticket<2>(job, t - first[j], weighted, max_rw, tol, sm);
         }
         __syncthreads();
     }
@@ -326,21 +407,14 @@ const LogDesignDevice<double>& device_view<double>(const lar_log_design_s* h) { 
 template <>
 const LogDesignDevice<float>& device_view<float>(const lar_log_design_s* h) { return h->d32; }
 
-// Voxels per CTA of the shared-memory fits: 64, or 32 / 16 when the design and a CTA's signals
-// of 64 voxels do not fit in shared memory (tables of more than about 200 measurements).
-inline int small_block(int n, int raw_bytes, size_t per_value) {
-    auto fits = [&](int block) {
-        return size_t(n) * (2 * 7 + 28) * per_value + size_t(n) * block * per_value + size_t(n) * block * raw_bytes +
-                   16 <= 227 * 1024;
-    };
+// Threads per CTA of the shared-memory fits: those of 64 voxels or kSmallThreads, or fewer when the design and
+// the CTA's signals do not fit in shared memory (tables of more than about 300 measurements).
+template <class T>
+int small_threads(int n, int lanes) {
     const int64_t want = launch_setting("dti.voxels_per_cta");
-    if ((want == 16 || want == 32 || want == 64) && fits(int(want))) return int(want);
-    for (int block : {64, 32, 16}) {
-        const size_t bytes = size_t(n) * (2 * 7 + 28) * per_value + size_t(n) * block * per_value +
-                             size_t(n) * block * raw_bytes + 16;
-        if (bytes <= 227 * 1024) return block;
-    }
-    return 16;
+    int threads = std::min<int>(kSmallThreads, (want == 16 || want == 32 || want == 64 ? int(want) : 64) * lanes);
+    while (threads > 16 && small_bytes<T>(n, threads / lanes) > 227 * 1024) threads /= 2;
+    return threads;
 }
 
 template <class Kernel>
@@ -409,19 +483,20 @@ void launch_fit(lar_log_design_s* h, const double* log_s, int64_t v, int weighte
     const int p = int(h->host.p);
     LogSource src{log_s, h->host.n};
     if (p == 7 && h->host.m == 0) {
-        auto run = [&](auto kernel, int block) {
-            const size_t sm = SmallFit<T, 7>::bytes(d.n, block, LogSource::raw_bytes);
+        auto run = [&](auto kernel, int lanes) {
+            const int threads = small_threads<T>(d.n, lanes), voxels = threads / lanes;
+            const size_t sm = small_bytes<T>(d.n, voxels);
             set_smem(kernel, sm);
-            const int64_t grid = (v + block - 1) / block;
+            const int64_t grid = (v + voxels - 1) / voxels;
             LaunchScope scope("fit_log_small_kernel", stream);
-            kernel<<<unsigned(grid), block, sm, stream>>>(d, src, v, weighted, max_rw, T(tol), params, broke,
-                                                          iterations);
+            kernel<<<unsigned(grid), threads, sm, stream>>>(d, src, v, weighted, max_rw, T(tol), params, broke,
+                                                            iterations);
             cuda_check(cudaGetLastError(), "fit_log_small_kernel launch");
         };
-        const int block = small_block(d.n, LogSource::raw_bytes, sizeof(T));
-        if (block == 64) run(fit_log_small_kernel<T, 7, 64, LogSource>, 64);
-        else if (block == 32) run(fit_log_small_kernel<T, 7, 32, LogSource>, 32);
-        else run(fit_log_small_kernel<T, 7, 16, LogSource>, 16);
+        const int lanes = small_lanes(v, d.n);
+        if (lanes == 8) run(fit_log_small_kernel<T, 8, LogSource>, 8);
+        else if (lanes == 4) run(fit_log_small_kernel<T, 4, LogSource>, 4);
+        else run(fit_log_small_kernel<T, 2, LogSource>, 2);
         return;
     }
     launch_general<T>(h, src, v, weighted, max_rw, tol, params, broke, iterations, stream);
@@ -433,37 +508,40 @@ void launch_dti_maps(const lar_log_design_s* h, const float* s, const double* fl
                      double* params, cudaStream_t stream) {
     const auto& d = device_view<T>(h);
     FlooredSource src{s, floor, h->host.n};
-    auto run = [&](auto kernel, int block) {
-        const size_t sm = SmallFit<T, 7>::bytes(d.n, block, FlooredSource::raw_bytes);
+    auto run = [&](auto kernel, int lanes) {
+        const int threads = small_threads<T>(d.n, lanes), voxels = threads / lanes;
+        const size_t sm = small_bytes<T>(d.n, voxels);
         set_smem(kernel, sm);
-        const int64_t grid = (v + block - 1) / block;
+        const int64_t grid = (v + voxels - 1) / voxels;
         LaunchScope scope("fit_dti_maps_kernel", stream);
-        kernel<<<unsigned(grid), block, sm, stream>>>(d, src, v, weighted, max_rw, T(tol), maps, npd, params);
+        kernel<<<unsigned(grid), threads, sm, stream>>>(d, src, v, weighted, max_rw, T(tol), maps, npd, params);
         cuda_check(cudaGetLastError(), "fit_dti_maps_kernel launch");
     };
-    const int block = small_block(d.n, FlooredSource::raw_bytes, sizeof(T));
-    if (block == 64) run(fit_dti_maps_kernel<T, 64>, 64);
-    else if (block == 32) run(fit_dti_maps_kernel<T, 32>, 32);
-    else run(fit_dti_maps_kernel<T, 16>, 16);
+    const int lanes = small_lanes(v, d.n);
+    if (lanes == 8) run(fit_dti_maps_kernel<T, 8>, 8);
+    else if (lanes == 4) run(fit_dti_maps_kernel<T, 4>, 4);
+    else run(fit_dti_maps_kernel<T, 2>, 2);
 }
 
 }  // namespace
 
-size_t batch_dti_smem(int n_max) { return SmallFit<double, 7>::bytes(n_max, kDtiBatchBlock, FlooredSource::raw_bytes); }
+size_t batch_dti_smem(int n_max) { return small_bytes<double>(n_max, kDtiBatchThreads / 2); }
+
+int dti_ticket_voxels(int64_t v, int n) { return kDtiBatchThreads / small_lanes(v, n); }
 
 void launch_batch_dti(const DtiBatchJob* jobs, const int64_t* first, int n_jobs, int n_max, int64_t tickets,
                       int weighted, int max_rw, double tol, int* queue, cudaStream_t stream) {
     if (n_jobs == 0 || tickets == 0) return;
-    auto kernel = batch_dti_kernel<kDtiBatchBlock>;
+    auto kernel = batch_dti_kernel;
     const size_t sm = batch_dti_smem(n_max);
     set_smem(kernel, sm);
     int per_sm = 0;
-    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kDtiBatchBlock, sm),
+    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kDtiBatchThreads, sm),
                "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
     const int64_t grid = std::min<int64_t>(tickets, int64_t(sm_count()) * std::max(per_sm, 1));
     cuda_check(cudaMemsetAsync(queue, 0, sizeof(unsigned long long), stream), "cudaMemsetAsync");
     LaunchScope scope("batch_dti_kernel", stream);
-    kernel<<<unsigned(grid), kDtiBatchBlock, sm, stream>>>(jobs, first, n_jobs, weighted, max_rw, tol, queue);
+    kernel<<<unsigned(grid), kDtiBatchThreads, sm, stream>>>(jobs, first, n_jobs, weighted, max_rw, tol, queue);
     cuda_check(cudaGetLastError(), "batch_dti_kernel launch");
 }
 

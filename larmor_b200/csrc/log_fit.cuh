@@ -61,16 +61,10 @@ struct LogSource {
     __device__ __forceinline__ void warp_stage(int64_t voxel, T* ys, int lane) const {
         for (int j = lane; j < n; j += 32) ys[j] = T(log_s[voxel * n + j]);
     }
-    static constexpr int raw_bytes = 8;
-    template <class T, int BLOCK>
-    __device__ __forceinline__ void stage(int64_t first, int count, unsigned char* raw, T* ys) const {
-        const double* src = log_s + first * n;
-        double* dst = reinterpret_cast<double*>(raw);
-        const int total = count * int(n);
-        for (int i = threadIdx.x; i < total; i += BLOCK) dst[i] = src[i];
-        __syncthreads();
-        if (threadIdx.x < count)
-            for (int j = 0; j < n; ++j) ys[j * BLOCK + threadIdx.x] = T(dst[threadIdx.x * n + j]);
+    // y_i, i counting the (v, n) rows' entries.
+    template <class T>
+    __device__ __forceinline__ T entry(int64_t, int64_t i) const {
+        return T(log_s[i]);
     }
 };
 
@@ -88,21 +82,10 @@ struct FlooredSource {
             ys[j] = (isfinite(x) && x > 0.0f) ? dev_log<T>(T(x)) : lf;
         }
     }
-    static constexpr int raw_bytes = 4;
-    template <class T, int BLOCK>
-    __device__ __forceinline__ void stage(int64_t first, int count, unsigned char* raw, T* ys) const {
-        const float* src = s + first * n;
-        float* dst = reinterpret_cast<float*>(raw);
-        const int total = count * int(n);
-        for (int i = threadIdx.x; i < total; i += BLOCK) dst[i] = src[i];
-        __syncthreads();
-        if (threadIdx.x < count) {
-            const T log_floor = dev_log<T>(T(floor[first + threadIdx.x]));
-            for (int j = 0; j < n; ++j) {
-                const float v = dst[threadIdx.x * n + j];
-                ys[j * BLOCK + threadIdx.x] = (isfinite(v) && v > 0.0f) ? dev_log<T>(T(v)) : log_floor;
-            }
-        }
+    template <class T>
+    __device__ __forceinline__ T entry(int64_t voxel, int64_t i) const {
+        const float x = s[i];
+        return dev_log<T>((isfinite(x) && x > 0.0f) ? T(x) : T(floor[voxel]));
     }
 };
 

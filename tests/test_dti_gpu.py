@@ -134,3 +134,29 @@ def test_large_tables_use_smaller_ctas_and_match_the_oracle(cuda, oracle, shells
     ref, _ = oracle.fit_log_signal(design, None, log_s, True)
     sc = np.linalg.norm(design, axis=0)
     np.testing.assert_allclose(params * sc, ref * sc, rtol=0, atol=1e-10)
+
+
+@pytest.mark.parametrize(("v", "n"), [(1, 31), (9, 12), (5000, 31), (5001, 13), (10000, 31), (10001, 31), (10001, 79),
+                                      (10001, 80), (300, 134)])
+def test_lanes_per_voxel_match_the_oracle(cuda, oracle, v, n):
+    """Each number of lanes per voxel at the sizes where the next one takes over, with shares of the
+    measurements that are even and not; the same bound as the other tables' (FP64, sums in another order)."""
+    from larmor_b200 import _core
+    from larmor_b200.dwi.dti import dti_design
+    from larmor_b200.synthetic import random_rotations, unit_directions
+    from larmor_b200.types import GradientTable
+
+    rng = np.random.default_rng(1000 * n + v)
+    g = GradientTable(np.concatenate([np.zeros(2), np.full(n - 2, 1000.0)]),
+                      np.vstack([np.zeros((2, 3)), unit_directions(rng, n - 2)]))
+    design = dti_design(g)
+    rot = random_rotations(rng, v)
+    ev = np.stack([rng.uniform(1.2e-3, 2e-3, v), *(2 * [rng.uniform(0.2e-3, 0.6e-3, v)])], axis=1)
+    tensors = np.einsum("vij,vj,vkj->vik", rot, ev, rot)
+    s = 1000.0 * np.exp(-g.bvals[None, :] * np.einsum("ni,vij,nj->vn", g.bvecs, tensors, g.bvecs))
+    log_s = np.ascontiguousarray(np.log(np.abs(s + rng.normal(0, 20.0, s.shape) + 1j * rng.normal(0, 20.0, s.shape))))
+    params, broke = _core.fit_log_signal(design, np.zeros((0, 7)), log_s, True, 20, 1e-6, 1)
+    ref, _ = oracle.fit_log_signal(design, None, log_s, True)
+    assert not broke.any()
+    sc = np.linalg.norm(design, axis=0)
+    np.testing.assert_allclose(params * sc, ref * sc, rtol=0, atol=1e-10)
