@@ -391,7 +391,7 @@ class DkiWorkload:
     """Config 2: constrained DKI WLLS on the 96x96x60 volume (199,768 voxels, 6 b0 + 2 x 64)."""
 
     name = "dki_wlls_96x96x60"
-    kernels = ("fit_log_warp_kernel", "constrained_fit_kernel", "dki_maps_kernel")
+    kernels = ("fit_log_warp_kernel", "fast_refit_kernel", "dki_maps_kernel")
     has_fp32 = True
     # 134 float32 samples + S0 and floor (double) in; 36 float32 maps + npd + broke out.
     bytes_per_voxel = 4 * 134 + 16 + 36 * 4 + 2
@@ -449,7 +449,7 @@ class DkiWorkload:
         n_viol = self.handle.violators()
         inputs = 4 * 134 + 16
         return {"fit_log_warp_kernel": self.v * (inputs + 22 * 8 + 1),
-                "constrained_fit_kernel": n_viol * (inputs + 2 * 22 * 8),
+                "fast_refit_kernel": n_viol * (inputs + 2 * 22 * 8),
                 "dki_maps_kernel": self.v * (22 * 8 + 36 * 4 + 1)}
 
     def step_e2e(self):
@@ -508,8 +508,8 @@ class MfodWorkload(_SdWorkloadBase):
     (float64 signals in, new FOD and fraction arrays out)."""
 
     name = "mfod_3tissue_110x110x70"
-    kernels = ("correlate_kernel", "ridge_nnls_low_kernel", "ridge_nnls_kernel<1,2>", "lr_fractions_kernel",
-               "ridge_nnls_high_kernel", "ridge_nnls_kernel<8,10>", "hr_fractions_kernel")
+    kernels = ("correlate_kernel", "ridge_nnls_low_kernel", "ridge_nnls_kernel<1,2>", "lane_fractions_kernel",
+               "lr_fractions_kernel", "ridge_nnls_high_kernel", "ridge_nnls_kernel<8,10>", "hr_fractions_kernel")
     has_fp32 = True
     fraction_tol = 1e-7
     # The plain FP32 fit takes seconds per step: a few timed steps bound the run.
@@ -588,13 +588,13 @@ class MfodWorkload(_SdWorkloadBase):
         self.d_rounds = rounds
         vr = int(rounds.sum().item())
         m, c_lr, c_hr = 280, self.k_lr.ca, self.k_hr.ca
-        # The low-resolution NNLS runs two voxels per warp and the high-resolution one a first
-        # pass with a 32-column factor; the full-factor kernels refit only the few voxels handed
-        # back (counted with the first kernels').
+        # The full-factor NNLS and the warp-per-voxel fractions refit only the few voxels that the
+        # first kernels hand back (counted with those).
         return {"correlate_kernel": vr * 8 * (m + c_lr) + self.v * 8 * (m + c_hr),
                 "ridge_nnls_low_kernel": vr * 8 * 2 * c_lr,
                 "ridge_nnls_kernel<1,2>": 0,
-                "lr_fractions_kernel": vr * 8 * (c_lr + m + 3),
+                "lane_fractions_kernel": vr * 8 * (c_lr + m + 3),
+                "lr_fractions_kernel": 0,
                 "ridge_nnls_high_kernel": self.v * 8 * 2 * c_hr,
                 "ridge_nnls_kernel<8,10>": 0,
                 "hr_fractions_kernel": self.v * 8 * (c_hr + m + 3)}
@@ -671,7 +671,7 @@ class MsmtWorkload(_SdWorkloadBase):
     constraints (300 directions + 2) per voxel."""
 
     name = "msmt_csd_lsi_110x110x70"
-    kernels = ("lsi_kernel",)
+    kernels = ("lsi_group_kernel", "rows_product_kernel", "lsi_group_qr_kernel", "lsi_kernel")
     has_fp32 = True
     fp32_steps = 1
     fp32_what = ("lar_fit_lsi_plain_fp32: one warp per voxel runs the LSI steps in FP32, the Cholesky factor of the "
@@ -712,7 +712,8 @@ class MsmtWorkload(_SdWorkloadBase):
 
     def kernel_bytes(self) -> dict:
         """Algorithmic DRAM bytes of one step: 280 signals in, 47 coefficients and a flag out."""
-        return {"lsi_kernel": self.bytes_per_voxel * self.v}
+        return {"lsi_group_kernel": self.bytes_per_voxel * self.v, "rows_product_kernel": self.bytes_per_voxel * self.v,
+                "lsi_group_qr_kernel": 0, "lsi_kernel": 0}
 
     def step_e2e(self):
         self.d_signals.copy_(self.h_signals, non_blocking=True)
@@ -773,14 +774,15 @@ def _job_kernel_bytes(job) -> dict:
     if job.kind == "dki":
         viol = int(job.out["broke"].sum().item())  # the voxels whose fit broke a constraint
         return {"fit_log_warp_kernel": v * (4 * n + 16 + 22 * 8 + 1),
-                "constrained_fit_kernel": viol * (4 * n + 16 + 2 * 22 * 8),
+                "fast_refit_kernel": viol * (4 * n + 16 + 2 * 22 * 8),
                 "dki_maps_kernel": v * (22 * 8 + 36 * 4 + 1)}
     vr = int(job.out["rounds"].sum().item())
     c_lr, c_hr = job.handles["k_lr"].ca, job.handles["k_hr"].ca
     return {"correlate_kernel": vr * 8 * (n + c_lr) + v * 8 * (n + c_hr),
             "ridge_nnls_low_kernel": vr * 8 * 2 * c_lr,
             "ridge_nnls_kernel<1,2>": 0,
-            "lr_fractions_kernel": vr * 8 * (c_lr + n + 3),
+            "lane_fractions_kernel": vr * 8 * (c_lr + n + 3),
+            "lr_fractions_kernel": 0,
             "ridge_nnls_high_kernel": v * 8 * 2 * c_hr,
             "ridge_nnls_kernel<8,10>": 0,
             "hr_fractions_kernel": v * 8 * (c_hr + n + 3)}
@@ -789,9 +791,10 @@ def _job_kernel_bytes(job) -> dict:
 # The kernels of the per-family work queues and the single-volume kernels whose per-voxel work
 # they do (the same algorithmic bytes).
 QUEUE_KERNELS = {"batch_dti_kernel": "fit_dti_maps_kernel", "batch_log_warp_kernel": "fit_log_warp_kernel",
-                 "batch_refit_kernel": "constrained_fit_kernel", "batch_dki_maps_kernel": "dki_maps_kernel",
+                 "batch_fast_refit_kernel": "fast_refit_kernel", "batch_refit_kernel": None, "batch_dki_maps_kernel": "dki_maps_kernel",
                  "batch_plan_kernel": None, "batch_correlate_kernel": "correlate_kernel",
                  "batch_low_kernel": "ridge_nnls_low_kernel", "batch_redo_kernel<1,2>": "ridge_nnls_kernel<1,2>",
+                 "batch_ks_kernel": None, "batch_lane_fractions_kernel": "lane_fractions_kernel",
                  "batch_lr_fractions_kernel": "lr_fractions_kernel",
                  "batch_high_kernel": "ridge_nnls_high_kernel",
                  "batch_redo_kernel<8,10>": "ridge_nnls_kernel<8,10>",
@@ -1263,9 +1266,9 @@ class PeaksWorkload:
         each voxel's 45 coefficients (shared by its climbs);
         the merge reads the results and writes 12 outputs."""
         c = self.climbs()
-        return {"project_sh_kernel": self.v * 8 * (45 + 642), "peak_count_kernel": self.v * (8 * 642 + 4),
+        return {"project_sh_kernel": self.v * 8 * (45 + 642), "peak_count_kernel": self.v * (8 * 642 + 4 * 21 + 4),
                 "scan_blocks_kernel": self.v * 12, "scan_sums_kernel": 0,
-                "peak_fill_kernel": self.v * 8 * 642 + 8 * c,
+                "peak_fill_kernel": self.v * (4 * 21 + 12) + 8 * c,
                 "climb_pool_kernel": self.v * 8 * 45 + c * (8 + 32), "peak_merge_kernel": c * 32 + self.v * (12 * 8 + 12)}
 
     def step_e2e(self):
