@@ -7,7 +7,8 @@
 // u = 1 - strength (1 - f^8 / (f^8 + nu^8)), with strength = max(1 - 4 std(s), 0). A voxel
 // stops when its amplitudes change in total by no more than 1e-4 of its largest signal value.
 //
-// Mapping: a CTA of 8 warps takes 8 RT voxels at a time (32 up to 320 directions, 16 up to 640)
+// Mapping: a CTA of 8 warps takes 8 RT voxels at a time (32 up to 320 directions, 16 up to 640; fewer in a
+// list's last wave, launch_narrow)
 // and keeps their FODs F (8 RT, c) and K^T s (8 RT, c) in shared memory for all their
 // iterations. An iteration is one product F K^T K on the FP64 tensor cores: mma.sync m8n8k4
 // over the RT 8-voxel row tiles and the 8-direction column tiles, which the warps take
@@ -21,7 +22,7 @@
 // a fixed order, so the stopping test does not depend on the schedule. Converged voxels keep their
 // FOD while the tile's others iterate.
 //
-// What bounds it: the FP64 pipe. 100,003 voxels, 300 directions, 200 iterations: 133 ms, of which the
+// What bounds it: the FP64 pipe. 100,003 voxels, 300 directions, 200 iterations: 130 ms, of which the
 // products take 97 at the tensor cores' rate and 8 more for the columns past the 38th tile (through the
 // stage: 261 ms). With 32 voxels to a CTA and 8 warps nothing hides the update behind another tile's
 // products: two CTAs would need K^T K's traffic twice.
@@ -397,8 +398,7 @@ __global__ void __launch_bounds__(kDrlWarps * 32, 1)
 
 template <int RT, typename Kernel>
 void launch_variant(Kernel kernel, const DrlDev& P, const DrlSignal& S, const int* list, int64_t count,
-                    const int* count_dev, double* x, int64_t ldx, cudaStream_t st, const char* name) {
-    const size_t smem = drl_smem_bytes(P.c);
+                    const int* count_dev, double* x, int64_t ldx, cudaStream_t st, const char* name, size_t smem) {
     allow_smem(kernel, smem);
     int per_sm = 0;
     cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kDrlWarps * 32, smem),
@@ -409,6 +409,48 @@ void launch_variant(Kernel kernel, const DrlDev& P, const DrlSignal& S, const in
     LaunchScope scope(name, st);
     kernel<<<unsigned(blocks), kDrlWarps * 32, smem, st>>>(P, S, list, count, count_dev, x, ldx);
     cuda_check(cudaGetLastError(), "drl_kernel launch");
+}
+
+// The streaming kernel with RT row tiles and as many column tiles per warp as c needs: the products of a warp's
+// columns past c are wasted.
+template <int RT>
+void launch_streamed(const DrlDev& P, const DrlSignal& S, const int* list, int64_t count, const int* count_dev,
+                     double* x, int64_t ldx, cudaStream_t st) {
+    const int ct = (P.c + 8 * kDrlWarps - 1) / (8 * kDrlWarps);
+    const size_t smem = 2 * size_t(8 * RT) * drl_lds((P.c + 7) / 8 * 8) * sizeof(double);
+    launch_variant<RT>(ct <= 2   ? drl_kernel<RT, 2>
+                       : ct == 3 ? drl_kernel<RT, 3>
+                       : ct == 4 ? drl_kernel<RT, 4>
+                                 : drl_kernel<RT, kNarrowCt>,
+                       P, S, list, count, count_dev, x, ldx, st, "drl_kernel", smem);
+}
+
+// Up to 320 directions: whole waves of 32-voxel tiles, a CTA on every SM, then what is left of the list in tiles
+// small enough to be one wave too. A tile's time is nearly its rows', so a wave of few 32-voxel
+// tiles takes as long as a full one (300 directions, 200 iterations: 6.1 ms for any number of 32-voxel tiles up to
+// a wave; 2.6 ms for 1,184 voxels and 3.5 for 2,368 in the smaller ones, whose warps read all of K^T K for
+// fewer products). A count on the device is not known here.
+void launch_narrow(const DrlDev& P, const DrlSignal& S, const int* list, int64_t count, const int* count_dev, double* x,
+                   int64_t ldx, cudaStream_t st) {
+    const int64_t wave = int64_t(sm_count()) * 8;
+    const int64_t rest = count_dev != nullptr ? count : count % (4 * wave), whole = count - rest;
+    if (count_dev != nullptr || rest > 2 * wave || rest == 0) {
+        launch_streamed<4>(P, S, list, count, count_dev, x, ldx, st);
+        return;
+    }
+    if (whole > 0) launch_streamed<4>(P, S, list, whole, nullptr, x, ldx, st);
+    DrlSignal after = S;
+    if (list != nullptr) {
+        list += whole;
+    } else {
+        after.s += whole * S.m;
+        if (S.fiso != nullptr) after.fiso += whole * S.ci;
+        x += whole * ldx;
+    }
+    if (rest > wave)
+        launch_streamed<2>(P, after, list, rest, nullptr, x, ldx, st);
+    else
+        launch_streamed<1>(P, after, list, rest, nullptr, x, ldx, st);
 }
 
 }  // namespace
@@ -430,19 +472,13 @@ void launch_drl_listed(const DrlDev& P, const DrlSignal& S, const int* list, int
         return;
     }
     if (P.c <= kResidentMaxC)
-        launch_variant<kNarrowRt>(drl_resident_kernel, P, S, list, count, count_dev, x, ldx, st, "drl_kernel_resident");
-    else if (P.c <= kNarrowMaxC) {
-        // As many column tiles per warp as c needs: the products of a warp's columns past c are wasted.
-        const int ct = (P.c + 8 * kDrlWarps - 1) / (8 * kDrlWarps);
-        launch_variant<kNarrowRt>(ct == 2   ? drl_kernel<kNarrowRt, 2>
-                                  : ct == 3 ? drl_kernel<kNarrowRt, 3>
-                                  : ct == 4 ? drl_kernel<kNarrowRt, 4>
-                                            : drl_kernel<kNarrowRt, kNarrowCt>,
-                                  P, S, list, count, count_dev, x, ldx, st, "drl_kernel");
-    } else {
+        launch_variant<kNarrowRt>(drl_resident_kernel, P, S, list, count, count_dev, x, ldx, st, "drl_kernel_resident",
+                                  drl_smem_bytes(P.c));
+    else if (P.c <= kNarrowMaxC)
+        launch_narrow(P, S, list, count, count_dev, x, ldx, st);
+    else
         launch_variant<kWideRt>(P.c <= 8 * kDrlWarps * 7 ? drl_kernel<kWideRt, 7> : drl_kernel<kWideRt, kWideCt>, P, S,
-                                list, count, count_dev, x, ldx, st, "drl_kernel_wide");
-    }
+                                list, count, count_dev, x, ldx, st, "drl_kernel_wide", drl_smem_bytes(P.c));
 }
 
 void launch_drl(const DrlDev& P, const double* signals, int64_t v, double* fods, cudaStream_t st) {

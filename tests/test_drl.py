@@ -249,3 +249,18 @@ def test_gpu_drl_at_the_edges_of_its_tiles(cuda, oracle, n_meas, n_dirs, n_vox, 
     got = _device_drl(signals, k, nu, 20, init)
     ref = oracle.drl(signals, k_t, k_t_k, nu, 20, init, n_threads=4)
     np.testing.assert_allclose(got, ref, rtol=1e-9, atol=0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize(("n_dirs", "n_vox"), [(66, 1190), (193, 2400), (300, 1184), (300, 2368), (300, 4740),
+                                               (300, 6000), (257, 9480)])
+def test_gpu_drl_whole_waves_and_the_rest(cuda, oracle, n_dirs, n_vox):
+    """Lists of whole waves of the largest tile, of a rest for each smaller one, and of both; the same bound as at
+    the tiles' edges."""
+    rng = np.random.default_rng(n_dirs + n_vox)
+    k = np.abs(rng.normal(size=(30, n_dirs))) + 0.1
+    signals = np.abs(rng.normal(size=(n_vox, 30))) / 10
+    k_t, k_t_k = _products(k)
+    got = _device_drl(signals, k, 0.02, 6, 0.01)
+    ref = oracle.drl(signals, k_t, k_t_k, 0.02, 6, 0.01, n_threads=8)
+    np.testing.assert_allclose(got, ref, rtol=1e-9, atol=0)
