@@ -14,7 +14,7 @@
 // T -= X X^T behind it; only the 8x8 diagonal tiles are eliminated lane by lane, giving their inverse
 // factors, which the two triangular solves use as well. What bounds it: the C_S^T C_S products and the
 // latencies of the diagonal tiles: 500,040 voxels, 45 coefficients, 300 constraints, 4.6 solves each of 134
-// constrained rows, 46.6 ms, of which the products take 26 at the tensor cores' rate (as csd_kernel does it
+// constrained rows, 44.7 ms, of which the products take 26 at the tensor cores' rate (as csd_kernel does it
 // below: 138 ms).
 //
 // For larger systems (csd_kernel) the system is packed in the warp's shared memory (lower
@@ -36,7 +36,7 @@ namespace {
 constexpr int kCsdStage = 8;   // constraint rows staged per pass of the system build (two k-steps of 4)
 constexpr int kCsdBatch = 8;   // tiles accumulated at once for larger systems
 constexpr int kTileRows = 6;   // most tile rows of csd_tiles_kernel: c <= 48 (lmax <= 8)
-constexpr int kTileWarps = 12;
+constexpr int kTileWarps = 16;  // (44.7 ms at the size below; 12 warps of 168 registers: 46.6, 14: 50)
 
 struct CsdDev {
     const double* initial_t;     // (m, c0)
@@ -110,7 +110,7 @@ __device__ __forceinline__ double row_sum(double v) {
 
 // The inverse Cholesky factor of the symmetric 8x8 tile (a0, a1) in its place: Gaussian elimination of
 // [A | I] without the square roots, whose rows are scaled at the end. Not inlined: six copies overran the
-// instruction cache (54.4 ms against 46.6).
+// instruction cache (54.4 ms against 46.6 with twelve warps).
 __device__ __noinline__ double2 invert_diagonal(double a0, double a1, int lane) {
     const int r = lane >> 2, p = lane & 3;
     double e0 = r == 2 * p ? 1.0 : 0.0, e1 = r == 2 * p + 1 ? 1.0 : 0.0, d = 1.0;
