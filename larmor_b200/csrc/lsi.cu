@@ -451,18 +451,19 @@ struct Place {
 // g.part (two entries per lane, na <= 64), with the barrier that makes it visible.
 template <int NW>
 __device__ __forceinline__ void group_sum(const GroupVoxel& g, int cap, int na, const Place<NW>& at, double (&a)[2]) {
-    if constexpr (NW == 1) return;
+    if constexpr (NW > 1) {
 #pragma unroll
-    for (int t = 0; t < 2; ++t)
-        if (at.lane + 32 * t < na) g.part[at.wig * cap + at.lane + 32 * t] = a[t];
-    at.sync();
+        for (int t = 0; t < 2; ++t)
+            if (at.lane + 32 * t < na) g.part[at.wig * cap + at.lane + 32 * t] = a[t];
+        at.sync();
 #pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        if (at.lane + 32 * t >= na) continue;
-        double s = g.part[at.lane + 32 * t];
+        for (int t = 0; t < 2; ++t) {
+            if (at.lane + 32 * t >= na) continue;
+            double s = g.part[at.lane + 32 * t];
 #pragma unroll
-        for (int q = 1; q < NW; ++q) s += g.part[q * cap + at.lane + 32 * t];
-        a[t] = s;
+            for (int q = 1; q < NW; ++q) s += g.part[q * cap + at.lane + 32 * t];
+            a[t] = s;
+        }
     }
 }
 
