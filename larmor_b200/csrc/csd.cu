@@ -17,7 +17,7 @@
 // constrained rows, 44.7 ms, of which the products take 26 at the tensor cores' rate (as csd_kernel does it
 // below: 138 ms).
 //
-// For larger systems (csd_kernel) the system is packed in the warp's shared memory (lower
+// For larger systems and constraint sets (csd_kernel) the system is packed in the warp's shared memory (lower
 // triangle, row-major). Each iteration rebuilds it as the Gram matrix plus C_S^T C_S on the tensor cores, rows
 // staged eight at a time in shared memory. A left-looking Cholesky factorisation (one row per lane) and two
 // column-oriented triangular solves follow. The amplitudes C f read C^T, so that the lanes (one
@@ -34,7 +34,7 @@ namespace lar {
 namespace {
 
 constexpr int kCsdStage = 8;   // constraint rows staged per pass of the system build (two k-steps of 4)
-constexpr int kCsdBatch = 8;   // tiles accumulated at once for larger systems
+constexpr int kCsdBatch = 8;   // tiles accumulated at once by build_batched
 constexpr int kTileRows = 6;   // most tile rows of csd_tiles_kernel: c <= 48 (lmax <= 8)
 constexpr int kTileWarps = 16;  // (44.7 ms at the size below; 12 warps of 168 registers: 46.6, 14: 50)
 
@@ -297,7 +297,44 @@ __global__ void __launch_bounds__(kTileWarps * 32, 1)
     }
 }
 
-// H = gram + C_S^T C_S for larger c: the lower tiles kCsdBatch at a time, the rows staged again
+// H = gram + C_S^T C_S in T tile rows, all their lower tiles accumulated over one pass of the constrained rows.
+template <int T>
+__device__ __forceinline__ void build_once(const CsdDev& P, const uint16_t* cur, int n_cur, double* rows, double* H,
+                                        int lane) {
+    constexpr int cp = 8 * T;
+    double acc[T * (T + 1) / 2][2];
+#pragma unroll
+    for (int t = 0; t < T * (T + 1) / 2; ++t) acc[t][0] = acc[t][1] = 0.0;
+    for (int q0 = 0; q0 < n_cur; q0 += kCsdStage) {
+        stage_rows(P, cur, n_cur, q0, rows, cp, lane);
+#pragma unroll
+        for (int kk = 0; kk < kCsdStage; kk += 4) {
+            const double* rk = rows + (kk + (lane & 3)) * cp + (lane >> 2);
+            double v[T];
+#pragma unroll
+            for (int b = 0; b < T; ++b) v[b] = rk[8 * b];
+#pragma unroll
+            for (int bi = 0; bi < T; ++bi)
+#pragma unroll
+                for (int bj = 0; bj <= bi; ++bj) mma_f64(acc[tile_of(bi, bj)][0], acc[tile_of(bi, bj)][1], v[bi], v[bj]);
+        }
+    }
+    const int c = P.c;
+#pragma unroll
+    for (int bi = 0; bi < T; ++bi)
+#pragma unroll
+        for (int bj = 0; bj <= bi; ++bj)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int i = 8 * bi + (lane >> 2), j = 8 * bj + 2 * (lane & 3) + h;
+                if (i < c && j <= i) {
+                    const int e = i * (i + 1) / 2 + j;
+                    H[e] = P.gram[e] + acc[tile_of(bi, bj)][h];
+                }
+            }
+}
+
+// H = gram + C_S^T C_S for any c: the lower tiles kCsdBatch at a time, the rows staged again
 // for each batch.
 __device__ __noinline__ void build_batched(const CsdDev& P, const uint16_t* cur, int n_cur, double* rows, double* H,
                                            int lane) {
@@ -342,6 +379,8 @@ __device__ __noinline__ void build_batched(const CsdDev& P, const uint16_t* cur,
     }
 }
 
+// TILES: the system's tile rows, built by build_once, or 0 for build_batched.
+template <int TILES>
 __global__ void csd_kernel(CsdDev P, const double* __restrict__ signals, int64_t v, double* __restrict__ fods,
                            uint8_t* __restrict__ converged_out) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -400,7 +439,10 @@ __global__ void csd_kernel(CsdDev P, const double* __restrict__ signals, int64_t
             // The system: the Gram matrix plus C_S^T C_S, the constrained rows' product on the
             // tensor cores over the rows staged kCsdStage at a time (zero-padded to whole tiles
             // and k-steps).
-            build_batched(P, cur, n_cur, rows, H, lane);
+            if constexpr (TILES > 0)
+                build_once<TILES>(P, cur, n_cur, rows, H, lane);
+            else
+                build_batched(P, cur, n_cur, rows, H, lane);
             __syncwarp();
             // Left-looking Cholesky, packed in place: column j's entries from the finished
             // columns, one row per lane; lane 0 holds the diagonal.
@@ -555,7 +597,12 @@ int lar_fit_csd(lar_csd csd, const double* signals, int64_t v, double* fods, uin
         const size_t per_warp = csd_warp_bytes(csd->c, csd->k);
         const int warps = int(std::max<size_t>(1, std::min<size_t>(4, (200 * 1024) / per_warp)));
         const size_t smem = per_warp * warps;
-        auto kernel = csd_kernel;
+        // Systems of four to six tile rows whose constraints are too many for the CTA's shared memory (past some
+        // 475 directions at 45 coefficients): one pass of the rows, where the batches would stage them two or three
+        // times (20,000 voxels, 642 directions: 45 coefficients XX against 32.9 ms, 28: XX against XX). With fewer tile
+        // rows one batch is one pass; with more the accumulators would not fit.
+        const int tiles = padded8(csd->c) / 8;
+        auto kernel = tiles == 4 ? csd_kernel<4> : tiles == 5 ? csd_kernel<5> : tiles == 6 ? csd_kernel<6> : csd_kernel<0>;
         allow_smem(kernel, smem);
         int per_sm = 0;
         cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, smem),

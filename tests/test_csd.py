@@ -303,3 +303,28 @@ def test_gpu_solve_at_the_edges_of_its_tiles(cuda, oracle, c, k, n):
     bound = 16 * c * 2.0**-53 * kappa * np.linalg.norm(ref, axis=1)
     bound += 2 * m * 2.0**-53 * np.linalg.norm(np.abs(signals) @ np.abs(forward), axis=1) / np.linalg.eigvalsh(gram)[0]
     assert np.all(np.linalg.norm(fods - ref, axis=1) <= bound)
+
+
+@pytest.mark.gpu
+def test_gpu_large_direction_sets_build_their_systems_in_one_pass(cuda):
+    """More directions than shared memory takes: up to 48 coefficients the constrained rows go through the products
+    once for all tiles, as they do below that size. 56 coefficients take four passes; 48 took three (0.7 of their
+    time with a pass the largest part) and take one (about 0.3)."""
+    from larmor_b200 import _core
+
+    torch = cuda
+    ms = {}
+    for c in (48, 56):
+        rng = np.random.default_rng(c)
+        problem = _core.CsdProblem(rng.normal(size=(15, 60)) / 60, rng.normal(size=(60, c)),
+                                   rng.normal(size=(700, c)), 1.0, 0.1, 3)
+        signals = torch.from_numpy(rng.normal(size=(5000, 60))).cuda()
+        times = []
+        for _ in range(4):
+            _core.kernel_timing(True)
+            _core.fit_csd_device(problem, signals)
+            torch.cuda.synchronize()
+            times.append(_core.kernel_time("csd_kernel")[0])
+            _core.kernel_timing(False)
+        ms[c] = min(times)
+    assert ms[48] <= 0.5 * ms[56], ms
