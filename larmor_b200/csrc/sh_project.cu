@@ -145,16 +145,19 @@ __global__ void __launch_bounds__(kExpandWarps * 32, 2) expand_sh_kernel(const d
     }
 }
 
-// Launches expand_sh_kernel<KS> with slices of at most ~100 KB, so that two CTAs share an SM.
+// Launches expand_sh_kernel<KS> with slices of at most ~100 KB, so that two CTAs share an SM, and narrower ones
+// for few rows, so that they are spread over the SMs: what a CTA stages and its warps' chains of products
+// get shorter with the slice.
 template <int KS>
 void launch_expand(const double* in, int64_t v, int64_t lda, int ca, const double* pt, int ncoef, double* out,
                    int64_t ldo, cudaStream_t st) {
     const int most = (100 * 1024 / (4 * KS * 8) - 4) / 8 * 8;
-    const int slices = (ncoef + most - 1) / most;
+    const int64_t blocks = (v + 16 * kExpandWarps - 1) / (16 * kExpandWarps);
+    const int slices = int(std::max<int64_t>((ncoef + most - 1) / most,
+                                             std::min<int64_t>((ncoef + 7) / 8, 2 * sm_count() / blocks)));
     const int width = ((ncoef + slices - 1) / slices + 7) / 8 * 8;
     const size_t smem = size_t(4 * KS) * (width + 4) * sizeof(double);
     allow_smem(expand_sh_kernel<KS>, smem);
-    const int64_t blocks = (v + 16 * kExpandWarps - 1) / (16 * kExpandWarps);
     const unsigned gx = unsigned(std::max<int64_t>(1, std::min<int64_t>(blocks, 2 * sm_count() / slices)));
     LaunchScope scope("project_sh_kernel", st);
     expand_sh_kernel<KS><<<dim3(gx, unsigned((ncoef + width - 1) / width)), kExpandWarps * 32, smem, st>>>(
@@ -207,7 +210,8 @@ int lar_project_sh(lar_sh_projector projector, const double* amplitudes, int64_t
         // fewer outputs than four times the inputs a warp's loads of them are no longer few beside its products.
         if (!exact_integral && ca <= 48 && nc >= 4 * ca) {
             const double* pt = projector->pt.ptr;
-            if (ca <= 16) launch_expand<4>(amplitudes, v, lda, ca, pt, nc, out, ldo, st);
+            if (ca <= 8) launch_expand<2>(amplitudes, v, lda, ca, pt, nc, out, ldo, st);
+            else if (ca <= 16) launch_expand<4>(amplitudes, v, lda, ca, pt, nc, out, ldo, st);
             else if (ca <= 28) launch_expand<7>(amplitudes, v, lda, ca, pt, nc, out, ldo, st);
             else launch_expand<12>(amplitudes, v, lda, ca, pt, nc, out, ldo, st);
             return;
