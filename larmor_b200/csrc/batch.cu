@@ -67,7 +67,7 @@ struct lar_batch_s {
     DeviceArray<DtiBatchJob> d_dti;
     DeviceArray<int64_t> dti_first;
     int64_t dti_tickets = 0;
-    int dti_nmax = 0;
+    size_t dti_smem = 0;
     // DKI
     LogFitSettings dki_fit;
     std::vector<DkiBatchJob> dki;
@@ -147,13 +147,13 @@ int lar_batch_finalize(lar_batch batch) {
         lar_batch_s& b = *batch;
         // DTI: tickets of dti_ticket_voxels.
         std::vector<int64_t> voxels;
-        for (const auto& j : b.dti) b.dti_nmax = std::max(b.dti_nmax, j.d.n);
+        for (const auto& j : b.dti) b.dti_smem = std::max(b.dti_smem, batch_dti_smem(j.v, j.d.n, b.dti_fit.weighted != 0));
         if (!b.dti.empty()) {
-            require(batch_dti_smem(b.dti_nmax) <= 227 * 1024,
+            require(b.dti_smem <= 227 * 1024,
                     "a DTI table of the batch has too many measurements for the shared-memory fit");
             std::vector<int64_t> first(1, 0);
             for (const auto& j : b.dti) {
-                const int64_t block = dti_ticket_voxels(j.v, j.d.n);
+                const int64_t block = dti_ticket_voxels(j.v, j.d.n, b.dti_fit.weighted != 0);
                 first.push_back(first.back() + (j.v + block - 1) / block);
             }
             b.dti_tickets = first.back();
@@ -223,7 +223,7 @@ int lar_batch_run(lar_batch batch, int families, void* stream) {
         lar_batch_s& b = *batch;
         auto st = static_cast<cudaStream_t>(stream);
         if ((families & LAR_BATCH_DTI) && !b.dti.empty())
-            launch_batch_dti(b.d_dti.ptr, b.dti_first.ptr, int(b.dti.size()), b.dti_nmax, b.dti_tickets,
+            launch_batch_dti(b.d_dti.ptr, b.dti_first.ptr, int(b.dti.size()), b.dti_smem, b.dti_tickets,
                              b.dti_fit.weighted, b.dti_fit.max_rw, b.dti_fit.tol, b.counters, st);
         if ((families & LAR_BATCH_DKI) && !b.dki.empty()) {
             cuda_check(cudaMemsetAsync(b.violators.count, 0, sizeof(int), st), "cudaMemsetAsync");

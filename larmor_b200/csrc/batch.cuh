@@ -74,13 +74,13 @@ constexpr int kDkiVoxelsPerWarp = 4;  // a ticket of the DKI log fit: 4 voxels p
 constexpr int kMapsBatchVoxels = 128;
 
 // Launch shapes and shared memory of the family stages (sized for the largest table).
-size_t batch_dti_smem(int n_max);
-int dti_ticket_voxels(int64_t v, int n);  // of one ticket of a volume of v voxels on n measurements
+size_t batch_dti_smem(int64_t v, int n, bool weighted);  // of a ticket of a volume of v voxels on n measurements
+int dti_ticket_voxels(int64_t v, int n, bool weighted);  // its voxels
 // Warps per CTA of the DKI log fit (12, 8 or 4; 0: the largest table does not fit) and its
 // shared memory.
 int batch_log_warp_warps(int n_max, int p);
 size_t batch_log_warp_smem(int n_max, int p, int warps);
-void launch_batch_dti(const DtiBatchJob* jobs, const int64_t* first, int n_jobs, int n_max, int64_t tickets,
+void launch_batch_dti(const DtiBatchJob* jobs, const int64_t* first, int n_jobs, size_t smem, int64_t tickets,
                       int weighted, int max_rw, double tol, int* queue, cudaStream_t stream);
 void launch_batch_log_warp(const DkiBatchJob* jobs, const int64_t* first, int n_jobs, int n_max, int p, int warps,
                            int64_t tickets, int weighted, int max_rw, double tol, int* queue,

@@ -8,9 +8,9 @@
 // pseudo-inverse, the products Z[n][ab] = X_na X_nb of the normal matrix, constraints) is small
 // and shared by every voxel: each CTA stages it once into shared memory.
 //
-// DTI (p = 7): two to eight neighbouring lanes per voxel (small_lanes). A lane accumulates the 28
-// normal-matrix entries and 7 right-hand sides in registers over its share of the measurements, a
-// butterfly sums the lanes' shares, each lane solves the 7 x 7 system by L D L^T in registers, and the first
+// DTI (p = 7): four or eight neighbouring lanes per voxel (small_lanes). A lane accumulates the 28
+// normal-matrix entries and 7 right-hand sides in registers over its share of the measurements (or half of them
+// over a share it shares), a butterfly sums the lanes' shares, each lane solves the 7 x 7 system by L D L^T in registers, and the first
 // finishes with the tensor's eigen-decomposition (cyclic Jacobi) and the DTI maps.
 
 #include <cmath>
@@ -71,15 +71,35 @@ __device__ __forceinline__ bool all_finite(const T (&v)[P]) {
 
 // ---- the IRLS of the 7-column design ------------------------------------------------------
 
-constexpr int kSmallThreads = 64;
-constexpr int kSmallCtas = 6;  // an SM's, by registers: with eight the fit spills (79,912 voxels: 277 us against 274)
+constexpr int kSmallThreads = 128;  // most of a CTA
+constexpr int kSmallCtas = 3;  // an SM's, by registers (a third more, spilling: 289 us against 293 at 79,912 voxels, 78 against 73 at 12,000)
 
-// Lanes per voxel of a fit of v voxels on n measurements. More lanes shorten a voxel's serial chain, while each
-// adds its part of the sums' butterfly (35 values) and repeats the solve. Measured, microseconds with 8, 4 and 2
-// lanes (one lane before: 115 to 139 up to 24,000 voxels of 31 measurements, 339 at 79,912):
-//   n = 31, v = 2,003: 42, 53, 75; 5,000: 53, 55, 76; 8,000: 76, 59, 76; 16,000: 113, 95, 98; 79,912: 464, 317, 274
-//   n = 94, v = 16,000: 204, 217, 219; 79,912: 801, 680, 700.   n = 134, v = 79,912: 906, 903, 971.
-__host__ __device__ inline int small_lanes(int64_t v, int n) { return v <= 5000 ? 8 : (v <= 10000 || n >= 80 ? 4 : 2); }
+// How a voxel's lanes share its sums over the measurements. Each sum is the sum of C partial sums, of the
+// measurements j = c mod C in increasing j, added in a butterfly of the distances C / 2, ..., 1; C depends on the
+// table alone, so a voxel's fit has the same bits in a slice, in a shard and in the whole volume.
+//   kTwo     C = 4: two lanes, two classes each (large unweighted calls)
+//   kFour    C = 4: four lanes, a class each
+//   kPairs   C = 4: eight lanes, lanes c and c + 4 sharing class c (normal_equations_halved)
+//   kEight   C = 8: eight lanes, a class each
+// Measured, microseconds:
+//   n = 31, v = 2,003 / 5,000 / 8,000 / 16,000 / 79,912: kFour 51 / 51 / 57 / 90 / 293, kPairs 49 / 57 / 86 / 128 / 529
+//   n = 94: kFour 102 / 106 / 120 / 210 / 650, kPairs 75 / 96 / 149 / 232 / 964, kEight 69 / 86 / 133 / 205 / 799
+//   n = 134: kFour 108 / 129 / 135 / 244 / 872, kEight 67 / 98 / 151 / 229 / 907;  n = 270, v = 79,912: 3,487, 2,811
+// (n = 31 with two lanes, C = 2: 274 at 79,912; with two lanes of two classes each, C = 4: 326, by its registers.)
+// An unweighted fit is seven sums and the maps, so that two lanes do where the call fills the GPU (a pass over 79,912
+// voxels of 31 measurements: 52 against 82 us with four; 20,000 of 134: 86 against 69). Past 500 measurements a
+// batch's CTA would not hold the signals of two lanes' voxels.
+enum class Lanes { kTwo, kFour, kPairs, kEight };
+__host__ __device__ constexpr int lane_count(Lanes lanes) {
+    return lanes == Lanes::kTwo ? 2 : lanes == Lanes::kFour ? 4 : 8;
+}
+__host__ __device__ constexpr int class_count(Lanes lanes) { return lanes == Lanes::kEight ? 8 : 4; }
+__host__ __device__ inline Lanes small_lanes(int64_t v, int n, bool weighted) {
+    if (!weighted) return n > 500 ? Lanes::kEight : v <= 20000 ? Lanes::kFour : Lanes::kTwo;
+    return n >= 128 ? Lanes::kEight : v <= 4000 ? Lanes::kPairs : Lanes::kFour;
+}
+
+__host__ __device__ constexpr int small_ctas(Lanes lanes) { return lanes == Lanes::kTwo ? 2 * kSmallCtas : kSmallCtas; }
 
 // Row strides in shared memory: of x and pinv^T (7 entries in whole 16-byte loads, eight rows of which
 // fall in distinct banks), and of the log signals of `voxels` voxels.
@@ -165,14 +185,17 @@ __device__ __forceinline__ bool ldlt_solve(T (&g)[P * (P + 1) / 2], T (&b)[P]) {
     return true;
 }
 
-// The sum and the maximum over the G lanes of a voxel, the same bits in each (mask: those lanes).
-template <int G, class T, int N>
-__device__ __forceinline__ void lanes_sum(T (&v)[N], unsigned mask) {
+// The sum of C classes, lane g of the voxel's G holding class g % C in v (or, fewer, the sum of g's and g + G's), the
+// same bits in each lane (mask: the voxel's lanes).
+template <int C, int G = C, class T, int N>
+__device__ __forceinline__ void class_sum(T (&v)[N], unsigned mask) {
 #pragma unroll
-    for (int o = 1; o < G; o *= 2)
+    for (int o = (G < C ? G : C) / 2; o > 0; o /= 2)
 #pragma unroll
         for (int i = 0; i < N; ++i) v[i] += __shfl_xor_sync(mask, v[i], o);
 }
+
+// The maximum over a voxel's G lanes, in each.
 template <int G, class T>
 __device__ __forceinline__ T lanes_max(T v, unsigned mask) {
 #pragma unroll
@@ -180,41 +203,136 @@ __device__ __forceinline__ T lanes_max(T v, unsigned mask) {
     return v;
 }
 
-// Fits one voxel from its log signals ys[j * stride], lane g of its G, and leaves its scaled parameters in p
+template <class T>
+__device__ __forceinline__ T predict(const T (&x)[8], const T (&q)[7]) {
+    T pred = T(0);
+#pragma unroll
+    for (int a = 0; a < 7; ++a) pred = fma(x[a], q[a], pred);
+    return pred;
+}
+
+// The weighted normal matrix m and right-hand side r of one voxel, weights exp(2 (x p - mx)), the same bits in each
+// of its lanes (g: this one). Each lane sums all 35 entries of its class.
+template <class T, int C>
+__device__ __forceinline__ void normal_equations(const T* __restrict__ xs, int n, const T* __restrict__ ys, int stride,
+                                                 const T (&p)[7], T mx, int g, unsigned mask, T (&m)[28], T (&r)[7]) {
+    constexpr int P = 7, PP = 28, LD = row_ld<T>();
+#pragma unroll
+    for (int k = 0; k < PP; ++k) m[k] = T(0);
+#pragma unroll
+    for (int a = 0; a < P; ++a) r[a] = T(0);
+    for (int j = g; j < n; j += C) {
+        T x[8];
+        load_row(xs + j * LD, x);
+        const T w = dev_exp<T>(T(2) * (predict(x, p) - mx));
+        const T y = ys[j * stride];
+        // The products x_a x_b come from the row itself: a table of them was four times the loads.
+        T wx[P];
+#pragma unroll
+        for (int a = 0; a < P; ++a) {
+            wx[a] = w * x[a];
+            r[a] = fma(wx[a], y, r[a]);
+        }
+#pragma unroll
+        for (int k = 0; k < PP; ++k) m[k] = fma(wx[packed_row(k, P)], x[packed_column(k, P)], m[k]);
+    }
+    class_sum<C>(m, mask);
+    class_sum<C>(r, mask);
+}
+
+// The same from eight lanes and four classes: of the class it shares, a lane takes every other exponential,
+// kAhead of them before the sums, and half the rows of [x, y]^T W [x, y]: rows 0, 3, 4, 7 or 1, 2, 5, 6, from the
+// columns 0, 2, 4 and 6 on (an entry or two below the diagonal too, which no one reads).
+template <class T>
+__device__ __forceinline__ void normal_equations_halved(const T* __restrict__ xs, int n, const T* __restrict__ ys,
+                                                        int stride, const T (&p)[7], T mx, int g, unsigned mask,
+                                                        T (&m)[28], T (&r)[7]) {
+    constexpr int P = 7, LD = row_ld<T>(), C = 4, kAhead = 4;
+    const int c = g % C, half = g / C;
+    T acc[4][8];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int b = 0; b < 8; ++b) acc[k][b] = T(0);
+    for (int j0 = c; j0 - c < n; j0 += 2 * kAhead * C) {
+        T mine[kAhead], x[8];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            load_row(xs + min(j0 + (2 * u + half) * C, n - 1) * LD, x);
+            mine[u] = dev_exp<T>(T(2) * (predict(x, p) - mx));
+        }
+#pragma unroll
+        for (int u = 0; u < 2 * kAhead; ++u) {
+            const T from = __shfl_sync(mask, mine[u / 2], int(threadIdx.x % 32) - g + c + C * (u & 1));
+            const int j = j0 + C * u, at = min(j, n - 1);
+            const T w = j < n ? from : T(0);  // adds zeros past the last
+            load_row(xs + at * LD, x);
+            x[7] = ys[at * stride];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                constexpr int kFirst[4] = {0, 3, 4, 7}, kSecond[4] = {1, 2, 5, 6};
+                const T wx = w * (half == 0 ? x[kFirst[k]] : x[kSecond[k]]);
+#pragma unroll
+                for (int b = 0; b < 8; ++b)
+                    if (b >= 2 * k) acc[k][b] = fma(wx, x[b], acc[k][b]);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) class_sum<C>(acc[k], mask);
+#pragma unroll
+    for (int a = 0; a < P; ++a) {
+        constexpr int kHalf[P] = {0, 1, 1, 0, 0, 1, 1}, kSlot[P] = {0, 0, 1, 1, 2, 2, 3};
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+            if (b < a) continue;
+            const T own = acc[kSlot[a]][b], other = __shfl_xor_sync(mask, own, C);
+            const T entry = half == kHalf[a] ? own : other;
+            if (b < P)
+                m[packed(a, b, P)] = entry;
+            else
+                r[a] = entry;
+        }
+    }
+}
+
+// Fits one voxel from its log signals ys[j * stride] on its lanes, and leaves its scaled parameters in p
 // (the same in every lane); returns the number of weighted fits. Follows reweighted_fit
 // (cpp/src/dwi/log_fit.cpp:114-147) from the ordinary fit pinv y (:251).
 // What bounds it: the latencies of a measurement's chain (a product, an exponential, the sums) with twelve warps
-// in an SM, and the lanes that wait for their warp's slowest voxel: 44% of the FP64 pipe at 79,912 voxels.
-template <class T, int G>
+// in an SM, and the lanes that wait for their warp's slowest voxel.
+template <class T, Lanes LANES>
 __device__ __forceinline__ int fit_voxel_small(const T* __restrict__ xs, const T* __restrict__ pinvt, int n,
                                                const T* __restrict__ ys, int stride, bool weighted, int max_rw, T tol,
                                                T (&p)[7]) {
-    constexpr int P = 7, PP = 28, LD = row_ld<T>();
+    constexpr int P = 7, PP = 28, LD = row_ld<T>(), G = lane_count(LANES), C = class_count(LANES);
     const int g = int(threadIdx.x) % G;
     const unsigned mask = ((1u << G) - 1u) << (threadIdx.x % 32 - g);
     auto ordinary = [&] {
-        T sum[P];
+        constexpr int K = G < C ? C / G : 1;
+        T sum[K][P];
 #pragma unroll
-        for (int a = 0; a < P; ++a) sum[a] = T(0);
+        for (int q = 0; q < K; ++q)
+#pragma unroll
+            for (int a = 0; a < P; ++a) sum[q][a] = T(0);
 #pragma unroll 2
-        for (int j = g; j < n; j += G) {
-            const T y = ys[j * stride];
-            T row[8];
-            load_row(pinvt + j * LD, row);
+        for (int j0 = g % C; j0 < n; j0 += C)
 #pragma unroll
-            for (int a = 0; a < P; ++a) sum[a] = fma(row[a], y, sum[a]);
-        }
-        lanes_sum<G>(sum, mask);
+            for (int q = 0; q < K; ++q) {
+                const int j = j0 + q * G;
+                if (q > 0 && j >= n) continue;
+                const T y = ys[j * stride];
+                T row[8];
+                load_row(pinvt + j * LD, row);
 #pragma unroll
-        for (int a = 0; a < P; ++a) p[a] = sum[a];
-    };
-    auto predict = [](const T (&x)[8], const T (&q)[P]) {
-        T pred = T(0);
+                for (int a = 0; a < P; ++a) sum[q][a] = fma(row[a], y, sum[q][a]);
+            }
 #pragma unroll
-        for (int a = 0; a < P; ++a) pred = fma(x[a], q[a], pred);
-        return pred;
+        for (int a = 0; a < P; ++a) p[a] = K > 1 ? sum[0][a] + sum[K - 1][a] : sum[0][a];
+        class_sum<C, G>(p, mask);
     };
     ordinary();
+    if constexpr (LANES == Lanes::kTwo) return 0;  // unweighted fits only (small_lanes)
     if (!weighted || !all_finite(p)) return 0;
     T mx = -INFINITY;
 #pragma unroll 2
@@ -227,28 +345,10 @@ __device__ __forceinline__ int fit_voxel_small(const T* __restrict__ xs, const T
     int it = 0;
     for (; it < max_rw; ++it) {
         T m[PP], r[P];
-#pragma unroll
-        for (int k = 0; k < PP; ++k) m[k] = T(0);
-#pragma unroll
-        for (int a = 0; a < P; ++a) r[a] = T(0);
-#pragma unroll 2
-        for (int j = g; j < n; j += G) {
-            T x[8];
-            load_row(xs + j * LD, x);
-            const T w = dev_exp<T>(T(2) * (predict(x, p) - mx));
-            const T y = ys[j * stride];
-            // The products x_a x_b come from the row itself: a table of them was four times the loads.
-            T wx[P];
-#pragma unroll
-            for (int a = 0; a < P; ++a) {
-                wx[a] = w * x[a];
-                r[a] = fma(wx[a], y, r[a]);
-            }
-#pragma unroll
-            for (int k = 0; k < PP; ++k) m[k] = fma(wx[packed_row(k, P)], x[packed_column(k, P)], m[k]);
-        }
-        lanes_sum<G>(m, mask);
-        lanes_sum<G>(r, mask);
+        if constexpr (LANES == Lanes::kPairs)
+            normal_equations_halved<T>(xs, n, ys, stride, p, mx, g, mask, m, r);
+        else
+            normal_equations<T, C>(xs, n, ys, stride, p, mx, g, mask, m, r);
         if (!ldlt_solve<T, P>(m, r) || !all_finite(r)) {
             ordinary();
             return it + 1;
@@ -292,14 +392,15 @@ __device__ __forceinline__ void stage_signals(const Src& src, int64_t first, int
     }
 }
 
-template <class T, int G, class Src>
-__global__ void __launch_bounds__(kSmallThreads, kSmallCtas) fit_log_small_kernel(LogDesignDevice<T> d, Src src, int64_t v,
+template <class T, Lanes LANES, class Src>
+__global__ void __launch_bounds__(kSmallThreads, small_ctas(LANES)) fit_log_small_kernel(LogDesignDevice<T> d, Src src, int64_t v,
                                                                      int weighted, int max_rw, T tol,
                                                                      double* __restrict__ params,
                                                                      uint8_t* __restrict__ broke,
                                                                      int32_t* __restrict__ iterations) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* sm = reinterpret_cast<T*>(smem_raw);
+    constexpr int G = lane_count(LANES);
     const int n = d.n, voxels = blockDim.x / G, ld = voxel_ld(voxels), local = threadIdx.x / G;
     T* ys = stage_design<T>(d, sm);
     const int64_t first = int64_t(blockIdx.x) * voxels;
@@ -309,7 +410,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallCtas) fit_log_small_kerne
     if (local >= count) return;
     const int64_t voxel = first + local;
     T p[7];
-    const int it = fit_voxel_small<T, G>(sm, sm + n * row_ld<T>(), n, ys + local, ld, weighted != 0, max_rw, tol, p);
+    const int it = fit_voxel_small<T, LANES>(sm, sm + n * row_ld<T>(), n, ys + local, ld, weighted != 0, max_rw, tol, p);
     if (threadIdx.x % G) return;
 #pragma unroll
     for (int a = 0; a < 7; ++a) params[voxel * 7 + a] = double(p[a]) / d.scales64[a];
@@ -317,14 +418,15 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallCtas) fit_log_small_kerne
     if (iterations) iterations[voxel] = it;
 }
 
-template <class T, int G>
-__global__ void __launch_bounds__(kSmallThreads, kSmallCtas) fit_dti_maps_kernel(LogDesignDevice<T> d, FlooredSource src,
+template <class T, Lanes LANES>
+__global__ void __launch_bounds__(kSmallThreads, small_ctas(LANES)) fit_dti_maps_kernel(LogDesignDevice<T> d, FlooredSource src,
                                                                     int64_t v, int weighted, int max_rw, T tol,
                                                                     float* __restrict__ maps,
                                                                     uint8_t* __restrict__ npd,
                                                                     double* __restrict__ params) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* sm = reinterpret_cast<T*>(smem_raw);
+    constexpr int G = lane_count(LANES);
     const int n = d.n, voxels = blockDim.x / G, ld = voxel_ld(voxels), local = threadIdx.x / G;
     T* ys = stage_design<T>(d, sm);
     const int64_t first = int64_t(blockIdx.x) * voxels;
@@ -334,7 +436,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallCtas) fit_dti_maps_kernel
     if (local >= count) return;
     const int64_t voxel = first + local;
     T p[7];
-    fit_voxel_small<T, G>(sm, sm + n * row_ld<T>(), n, ys + local, ld, weighted != 0, max_rw, tol, p);
+    fit_voxel_small<T, LANES>(sm, sm + n * row_ld<T>(), n, ys + local, ld, weighted != 0, max_rw, tol, p);
     if (threadIdx.x % G) return;
     T dt[6];
 #pragma unroll
@@ -350,9 +452,10 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallCtas) fit_dti_maps_kernel
 // dti_ticket_voxels(v, n) voxels of one volume from a device counter across every DTI volume; a CTA
 // restages the design when its ticket moves to another volume. Per voxel the same fit and maps
 // as fit_dti_maps_kernel (FP64).
-template <int G>
+template <Lanes LANES>
 __device__ __noinline__ void batch_dti_ticket(const DtiBatchJob& job, int64_t ticket, int weighted, int max_rw,
                                               double tol, double* sm) {
+    constexpr int G = lane_count(LANES);
     const int n = job.d.n, local = threadIdx.x / G;
     constexpr int kVoxels = kDtiBatchThreads / G, kLd = voxel_ld(kVoxels), LD = row_ld<double>();
     double* ys = sm + 2 * n * LD;
@@ -362,7 +465,7 @@ __device__ __noinline__ void batch_dti_ticket(const DtiBatchJob& job, int64_t ti
     __syncthreads();
     if (local < count) {
         double p[7];
-        fit_voxel_small<double, G>(sm, sm + n * LD, n, ys + local, kLd, weighted != 0, max_rw, tol, p);
+        fit_voxel_small<double, LANES>(sm, sm + n * LD, n, ys + local, kLd, weighted != 0, max_rw, tol, p);
         if (threadIdx.x % G == 0) {
             double dt[6];
 #pragma unroll
@@ -391,10 +494,11 @@ __global__ void __launch_bounds__(kDtiBatchThreads, kSmallCtas * kSmallThreads /
             stage_design<double>(job.d, sm);
             cur = j;
         }
-        switch (small_lanes(job.v, job.d.n)) {
-            case 8: batch_dti_ticket<8>(job, t - first[j], weighted, max_rw, tol, sm); break;
-            case 4: batch_dti_ticket<4>(job, t - first[j], weighted, max_rw, tol, sm); break;
-            default: batch_dti_ticket<2>(job, t - first[j], weighted, max_rw, tol, sm);
+        switch (small_lanes(job.v, job.d.n, weighted != 0)) {
+            case Lanes::kTwo: batch_dti_ticket<Lanes::kTwo>(job, t - first[j], weighted, max_rw, tol, sm); break;
+            case Lanes::kEight: batch_dti_ticket<Lanes::kEight>(job, t - first[j], weighted, max_rw, tol, sm); break;
+            case Lanes::kPairs: batch_dti_ticket<Lanes::kPairs>(job, t - first[j], weighted, max_rw, tol, sm); break;
+            default: batch_dti_ticket<Lanes::kFour>(job, t - first[j], weighted, max_rw, tol, sm);
         }
         __syncthreads();
     }
@@ -407,12 +511,14 @@ const LogDesignDevice<double>& device_view<double>(const lar_log_design_s* h) { 
 template <>
 const LogDesignDevice<float>& device_view<float>(const lar_log_design_s* h) { return h->d32; }
 
-// Threads per CTA of the shared-memory fits: those of 64 voxels or kSmallThreads, or fewer when the design and
-// the CTA's signals do not fit in shared memory (tables of more than about 300 measurements).
+// Threads per CTA of the shared-memory fits: few for a small call, so that it spreads over the SMs, else
+// kSmallThreads, whose voxels share the staged design (20,000 voxels of 270 measurements: 639 us, with 64 threads
+// 735); fewer when the design and the CTA's signals do not fit in shared memory (tables of more than about 700 measurements).
 template <class T>
-int small_threads(int n, int lanes) {
+int small_threads(int64_t v, int n, int lanes) {
     const int64_t want = launch_setting("dti.voxels_per_cta");
-    int threads = std::min<int>(kSmallThreads, (want == 16 || want == 32 || want == 64 ? int(want) : 64) * lanes);
+    int threads = v <= 4000 ? 64 : kSmallThreads;
+    if (want == 16 || want == 32 || want == 64) threads = int(std::min<int64_t>(kSmallThreads, want * lanes));
     while (threads > 16 && small_bytes<T>(n, threads / lanes) > 227 * 1024) threads /= 2;
     return threads;
 }
@@ -484,7 +590,7 @@ void launch_fit(lar_log_design_s* h, const double* log_s, int64_t v, int weighte
     LogSource src{log_s, h->host.n};
     if (p == 7 && h->host.m == 0) {
         auto run = [&](auto kernel, int lanes) {
-            const int threads = small_threads<T>(d.n, lanes), voxels = threads / lanes;
+            const int threads = small_threads<T>(v, d.n, lanes), voxels = threads / lanes;
             const size_t sm = small_bytes<T>(d.n, voxels);
             set_smem(kernel, sm);
             const int64_t grid = (v + voxels - 1) / voxels;
@@ -493,10 +599,12 @@ void launch_fit(lar_log_design_s* h, const double* log_s, int64_t v, int weighte
                                                             iterations);
             cuda_check(cudaGetLastError(), "fit_log_small_kernel launch");
         };
-        const int lanes = small_lanes(v, d.n);
-        if (lanes == 8) run(fit_log_small_kernel<T, 8, LogSource>, 8);
-        else if (lanes == 4) run(fit_log_small_kernel<T, 4, LogSource>, 4);
-        else run(fit_log_small_kernel<T, 2, LogSource>, 2);
+        switch (small_lanes(v, d.n, weighted != 0)) {
+            case Lanes::kTwo: run(fit_log_small_kernel<T, Lanes::kTwo, LogSource>, 2); break;
+            case Lanes::kEight: run(fit_log_small_kernel<T, Lanes::kEight, LogSource>, 8); break;
+            case Lanes::kPairs: run(fit_log_small_kernel<T, Lanes::kPairs, LogSource>, 8); break;
+            default: run(fit_log_small_kernel<T, Lanes::kFour, LogSource>, 4);
+        }
         return;
     }
     launch_general<T>(h, src, v, weighted, max_rw, tol, params, broke, iterations, stream);
@@ -509,7 +617,7 @@ void launch_dti_maps(const lar_log_design_s* h, const float* s, const double* fl
     const auto& d = device_view<T>(h);
     FlooredSource src{s, floor, h->host.n};
     auto run = [&](auto kernel, int lanes) {
-        const int threads = small_threads<T>(d.n, lanes), voxels = threads / lanes;
+        const int threads = small_threads<T>(v, d.n, lanes), voxels = threads / lanes;
         const size_t sm = small_bytes<T>(d.n, voxels);
         set_smem(kernel, sm);
         const int64_t grid = (v + voxels - 1) / voxels;
@@ -517,23 +625,28 @@ void launch_dti_maps(const lar_log_design_s* h, const float* s, const double* fl
         kernel<<<unsigned(grid), threads, sm, stream>>>(d, src, v, weighted, max_rw, T(tol), maps, npd, params);
         cuda_check(cudaGetLastError(), "fit_dti_maps_kernel launch");
     };
-    const int lanes = small_lanes(v, d.n);
-    if (lanes == 8) run(fit_dti_maps_kernel<T, 8>, 8);
-    else if (lanes == 4) run(fit_dti_maps_kernel<T, 4>, 4);
-    else run(fit_dti_maps_kernel<T, 2>, 2);
+    switch (small_lanes(v, d.n, weighted != 0)) {
+        case Lanes::kTwo: run(fit_dti_maps_kernel<T, Lanes::kTwo>, 2); break;
+        case Lanes::kEight: run(fit_dti_maps_kernel<T, Lanes::kEight>, 8); break;
+        case Lanes::kPairs: run(fit_dti_maps_kernel<T, Lanes::kPairs>, 8); break;
+        default: run(fit_dti_maps_kernel<T, Lanes::kFour>, 4);
+    }
 }
 
 }  // namespace
 
-size_t batch_dti_smem(int n_max) { return small_bytes<double>(n_max, kDtiBatchThreads / 2); }
+int dti_ticket_voxels(int64_t v, int n, bool weighted) {
+    return kDtiBatchThreads / lane_count(small_lanes(v, n, weighted));
+}
 
-int dti_ticket_voxels(int64_t v, int n) { return kDtiBatchThreads / small_lanes(v, n); }
+size_t batch_dti_smem(int64_t v, int n, bool weighted) {
+    return small_bytes<double>(n, dti_ticket_voxels(v, n, weighted));
+}
 
-void launch_batch_dti(const DtiBatchJob* jobs, const int64_t* first, int n_jobs, int n_max, int64_t tickets,
+void launch_batch_dti(const DtiBatchJob* jobs, const int64_t* first, int n_jobs, size_t sm, int64_t tickets,
                       int weighted, int max_rw, double tol, int* queue, cudaStream_t stream) {
     if (n_jobs == 0 || tickets == 0) return;
     auto kernel = batch_dti_kernel;
-    const size_t sm = batch_dti_smem(n_max);
     set_smem(kernel, sm);
     int per_sm = 0;
     cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kDtiBatchThreads, sm),
