@@ -22,7 +22,7 @@
 // a fixed order, so the stopping test does not depend on the schedule. Converged voxels keep their
 // FOD while the tile's others iterate.
 //
-// What bounds it: the FP64 pipe. 100,003 voxels, 300 directions, 200 iterations: 130 ms, of which the
+// What bounds it: the FP64 pipe. 100,003 voxels, 300 directions, 200 iterations: 134 ms, of which the
 // products take 97 at the tensor cores' rate and 8 more for the columns past the 38th tile (through the
 // stage: 261 ms). With 32 voxels to a CTA and 8 warps nothing hides the update behind another tile's
 // products: two CTAs would need K^T K's traffic twice.
@@ -135,30 +135,26 @@ __device__ __forceinline__ void open_tile(DrlTile<ROWS>& t, const DrlSignal& S, 
     }
 }
 
-// a / b by Newton's iteration on the hardware's approximate reciprocal and one step on the quotient, without
-// the branches of the general division, so that a lane's quotients overlap (the 100,003 voxels below took
-// 149 ms with them). For |b| well inside the range of the exponent: (f^8 + nu^8) (p + 1e-16) is, with
-// f >= 1e-6 from the first update on.
-__device__ __forceinline__ double quotient(double a, double b) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
-    r = fma(r, fma(-b, r, 1.0), r);
-    r = fma(r, fma(-b, r, 1.0), r);
-    const double q = a * r;
-    return fma(r, fma(-b, q, a), q);
-}
-
-// The update's relative step as it is written, for a start and a nu so small that the quotient's range may end.
+// The update's relative step as it is written (cpp/src/sd/drl.cpp:13-20).
 __device__ __noinline__ double plain_step(double f8, double nu8, double strength, double ks, double pred) {
     return (1.0 - strength * (1.0 - f8 / (f8 + nu8))) * ((ks - pred) / (pred + 1e-16));
 }
 
+// Whether |x| lies between about 1e-200 and 1e200 (by its exponent).
+__device__ __forceinline__ bool mid_range(double x) {
+    return ((unsigned(__double2hiint(x)) >> 20) & 0x7ffu) - 359u <= 1328u;
+}
+
 // The damped update of the still-active voxels from the prediction acc (column tile t of the warp in
 // acc[.][t]), each one's total change into part, and whether any voxel is still active. The damping
-// 1 - strength (1 - f^8 / (f^8 + nu^8)) and the ratio (K^T s - p) / (p + 1e-16) share one division.
+// 1 - strength (1 - f^8 / (f^8 + nu^8)) and the ratio (K^T s - p) / (p + 1e-16) have the product of their
+// denominators below one fraction bar, and a lane's two entries share one reciprocal of both products (Montgomery,
+// Math. Comp. 48 (1987) 243-264): 100,003 voxels of 300 directions, 200 iterations, 133.6 ms, with a reciprocal each
+// 138.5, with a division each 143.5. Where that is 0, out of the middle of the range or not a number, the two are
+// taken as written.
 template <int RT, int CT>
 __device__ __forceinline__ bool update_tile(DrlTile<8 * RT>& tile, const double (&acc)[RT][CT][2], double* F,
-                                            const double* KS, int ld, int c, double nu8, bool plain) {
+                                            const double* KS, int ld, int c, double nu8) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 #pragma unroll
     for (int rt = 0; rt < RT; ++rt) {
@@ -172,13 +168,24 @@ __device__ __forceinline__ bool update_tile(DrlTile<8 * RT>& tile, const double 
                 double* at = F + r * ld + min(d, c - 1) / 2 * 2;
                 const double2 f = *reinterpret_cast<const double2*>(at);
                 const double2 ks = *reinterpret_cast<const double2*>(KS + (at - F));
-                double to[2];
+                double below[2], step[2], to[2];
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const double fh = h ? f.y : f.x, f8 = power_8(fh), pred = acc[rt][t][h];
-                    double step = quotient((f8 + off) * ((h ? ks.y : ks.x) - pred), (f8 + nu8) * (pred + 1e-16));
-                    if (plain) step = plain_step(f8, nu8, tile.strength[r], h ? ks.y : ks.x, pred);
-                    to[h] = fmax(fh * (1.0 + step), 1e-6);
+                    const double f8 = power_8(h ? f.y : f.x), pred = acc[rt][t][h];
+                    below[h] = (f8 + nu8) * (pred + 1e-16);
+                    step[h] = (f8 + off) * ((h ? ks.y : ks.x) - pred);
+                }
+                const double both = below[0] * below[1], inverse = __drcp_rn(both);
+                step[0] *= inverse * below[1];
+                step[1] *= inverse * below[0];
+                if (!mid_range(both)) {
+                    step[0] = plain_step(power_8(f.x), nu8, tile.strength[r], ks.x, acc[rt][t][0]);
+                    step[1] = plain_step(power_8(f.y), nu8, tile.strength[r], ks.y, acc[rt][t][1]);
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const double fh = h ? f.y : f.x;
+                    to[h] = fmax(fh * (1.0 + step[h]), 1e-6);
                     if (d + h < c) change += fabs(to[h] - fh);
                 }
                 if (d < c) at[0] = to[0];
@@ -215,7 +222,6 @@ __global__ void __launch_bounds__(kDrlWarps * 32, 2)
     double* GS = KS + kRows * ldf;                // (cp, ldg)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const double nu8 = power_8(P.nu);
-    const bool plain = !(nu8 + power_8(P.init) > 1e-200);
     // All of K^T K, zero past c (made visible by the barrier at the first tile's start).
     for (int e = threadIdx.x; e < cp * ldg; e += blockDim.x) {
         const int k = e / ldg, d = e - k * ldg;
@@ -253,7 +259,7 @@ __global__ void __launch_bounds__(kDrlWarps * 32, 2)
                 }
             // The update overwrites F: every warp is done reading it first.
             __syncthreads();
-            if (!update_tile<RT, 1>(tile, acc, F, KS, ldf, c, nu8, plain)) break;
+            if (!update_tile<RT, 1>(tile, acc, F, KS, ldf, c, nu8)) break;
         }
         for (int e = tid; e < kRows * ldf; e += blockDim.x) {
             const int r = e / ldf, d = e - r * ldf;
@@ -338,7 +344,6 @@ __global__ void __launch_bounds__(kDrlWarps * 32, 1)
     double* KS = F + kRows * ld;                  // (kRows, ld)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const double nu8 = power_8(P.nu);
-    const bool plain = !(nu8 + power_8(P.init) > 1e-200);
     StreamedProduct<RT, CT> product;
     double acc[RT][CT][2];
     auto clear = [&] {
@@ -385,7 +390,7 @@ __global__ void __launch_bounds__(kDrlWarps * 32, 1)
             if (it + 1 < P.n_iter) product.open(P.gram, c, c, 0, c);
             // The update overwrites F: every warp is done reading it first.
             __syncthreads();
-            if (!update_tile<RT, CT>(tile, acc, F, KS, ld, c, nu8, plain)) break;
+            if (!update_tile<RT, CT>(tile, acc, F, KS, ld, c, nu8)) break;
         }
         for (int e = tid; e < kRows * cp; e += blockDim.x) {
             const int r = e / cp, d = e - r * cp;
