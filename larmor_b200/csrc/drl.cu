@@ -165,9 +165,12 @@ __device__ __forceinline__ bool update_tile(DrlTile<8 * RT>& tile, const double 
 #pragma unroll
             for (int t = 0; t < CT; ++t) {
                 const int d = 8 * (warp + kDrlWarps * t) + 2 * (lane & 3);
-                double* at = F + r * ld + min(d, c - 1) / 2 * 2;
-                const double2 f = *reinterpret_cast<const double2*>(at);
-                const double2 ks = *reinterpret_cast<const double2*>(KS + (at - F));
+                double* at = F + r * ld + d;
+                double2 f = make_double2(1.0, 1.0), ks = make_double2(0.0, 0.0);
+                if (d < c) {  // a column of no one's is neither read nor written
+                    f = *reinterpret_cast<const double2*>(at);
+                    ks = *reinterpret_cast<const double2*>(KS + (at - F));
+                }
                 double below[2], step[2], to[2];
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
