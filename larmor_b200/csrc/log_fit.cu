@@ -5,13 +5,14 @@
 //
 // Layout: the masked signals are (v, n) row-major, one voxel's n samples contiguous, as the
 // reference's chunk arrays are. The per-table design (unit-norm columns X (n, p), its
-// pseudo-inverse, the products Z[n][ab] = X_na X_nb of the normal matrix, constraints) is small
-// and shared by every voxel: each CTA stages it once into shared memory.
+// pseudo-inverse, constraints) is small and shared by every voxel: each CTA stages X and the pseudo-inverse
+// once into shared memory.
 //
 // DTI (p = 7): four or eight neighbouring lanes per voxel (small_lanes). A lane accumulates the 28
-// normal-matrix entries and 7 right-hand sides in registers over its share of the measurements (or half of them
-// over a share it shares), a butterfly sums the lanes' shares, each lane solves the 7 x 7 system by L D L^T in registers, and the first
-// finishes with the tensor's eigen-decomposition (cyclic Jacobi) and the DTI maps.
+// normal-matrix entries and 7 right-hand sides in registers over its share of the measurements (or half of the
+// entries over a share it has in common), a butterfly sums the lanes' shares, each lane solves the 7 x 7 system by
+// L D L^T in registers, and the first finishes with the tensor's eigen-decomposition (cyclic Jacobi) and the DTI
+// maps.
 
 #include <cmath>
 #include <cstdio>
@@ -51,8 +52,8 @@ struct lar_log_design_s {
     LogScratch scratch;
     lar::LogDesignDevice<double> d64;
     lar::LogDesignDevice<float> d32;
-    lar::DeviceArray<double> x64, pinvt64, z64, g64, scales64;
-    lar::DeviceArray<float> x32, pinvt32, z32, g32, scales32;
+    lar::DeviceArray<double> x64, pinvt64, g64, scales64;
+    lar::DeviceArray<float> x32, pinvt32, g32, scales32;
 };
 
 namespace lar {
@@ -661,22 +662,16 @@ void launch_batch_dti(const DtiBatchJob* jobs, const int64_t* first, int n_jobs,
 namespace {
 
 template <class T>
-void upload_design(lar_log_design_s* h, DeviceArray<T>& x, DeviceArray<T>& pinvt, DeviceArray<T>& z,
-                   DeviceArray<T>& g, DeviceArray<T>& scales, LogDesignDevice<T>& view) {
+void upload_design(lar_log_design_s* h, DeviceArray<T>& x, DeviceArray<T>& pinvt, DeviceArray<T>& g,
+                   DeviceArray<T>& scales, LogDesignDevice<T>& view) {
     const auto& hd = h->host;
-    const int64_t n = hd.n, p = hd.p, m = hd.m, pp = p * (p + 1) / 2;
-    std::vector<T> xv(static_cast<size_t>(n * p)), pt(static_cast<size_t>(n * p)), zv(static_cast<size_t>(n * pp)),
-        gv(static_cast<size_t>(2 * m * p)), sv(static_cast<size_t>(p));
+    const int64_t n = hd.n, p = hd.p, m = hd.m;
+    std::vector<T> xv(static_cast<size_t>(n * p)), pt(static_cast<size_t>(n * p)), gv(static_cast<size_t>(2 * m * p)), sv(static_cast<size_t>(p));
     for (int64_t i = 0; i < n; ++i)
         for (int64_t a = 0; a < p; ++a) {
             xv[size_t(i * p + a)] = T(hd.x[size_t(i * p + a)]);
             pt[size_t(i * p + a)] = T(hd.pinv[size_t(a * n + i)]);
         }
-    for (int64_t i = 0; i < n; ++i) {
-        int64_t k = 0;
-        for (int64_t a = 0; a < p; ++a)
-            for (int64_t b = a; b < p; ++b) zv[size_t(i * pp + k++)] = T(hd.x[size_t(i * p + a)] * hd.x[size_t(i * p + b)]);
-    }
     // g (m, p) row-major, then its transpose (p, m).
     for (int64_t c = 0; c < m; ++c)
         for (int64_t a = 0; a < p; ++a) {
@@ -686,7 +681,6 @@ void upload_design(lar_log_design_s* h, DeviceArray<T>& x, DeviceArray<T>& pinvt
     for (int64_t a = 0; a < p; ++a) sv[size_t(a)] = T(hd.scales[size_t(a)]);
     x.upload(xv.data(), xv.size());
     pinvt.upload(pt.data(), pt.size());
-    z.upload(zv.data(), zv.size());
     g.upload(gv.data(), gv.size());
     scales.upload(sv.data(), sv.size());
     view.n = int(n);
@@ -694,7 +688,6 @@ void upload_design(lar_log_design_s* h, DeviceArray<T>& x, DeviceArray<T>& pinvt
     view.m = int(m);
     view.x = x.ptr;
     view.pinvt = pinvt.ptr;
-    view.z = z.ptr;
     view.g = g.ptr;
     view.gt = m > 0 ? g.ptr + m * p : nullptr;
     view.scales = scales.ptr;
@@ -725,8 +718,8 @@ int lar_log_design_create(const double* x, int64_t n, int64_t p, const double* g
         h->host = host::prepare_log_design(x, n, p, g, m);
         double bound = 0.0;
         h->host.dki = dki_constraint_bound(h->host.g.data(), m, p, &bound);
-        upload_design<double>(h.get(), h->x64, h->pinvt64, h->z64, h->g64, h->scales64, h->d64);
-        upload_design<float>(h.get(), h->x32, h->pinvt32, h->z32, h->g32, h->scales32, h->d32);
+        upload_design<double>(h.get(), h->x64, h->pinvt64, h->g64, h->scales64, h->d64);
+        upload_design<float>(h.get(), h->x32, h->pinvt32, h->g32, h->scales32, h->d32);
         h->d64.dki = h->host.dki;
         h->d64.bound = bound;
         h->d64.scales64 = h->scales64.ptr;

@@ -146,7 +146,6 @@ extern "C" int lar_fit_log_signal_noalloc(const double* x, int64_t n, int64_t p,
         d.m = int(m);
         d.x = dx;
         d.pinvt = dx + n * p;
-        d.z = nullptr;
         d.g = dx + 2 * n * p;
         d.gt = m > 0 ? dx + 2 * n * p + m * p : nullptr;
         d.scales = dx + 2 * n * p + 2 * m * p;
