@@ -1,0 +1,66 @@
+"""The eight-warp QR variant of the LSI group kernel: every constraint twice, the copies 1e-7 apart, so that the
+Cholesky factor fails, with active sets past 32 whose early columns leave (in a Lawson-Hanson of the same problems each
+voxel drops 6 to 22 columns, nearly all from a position below 32 while more than 32 are active), which splits a
+removal's columns over two warps."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _fit(torch, a, g, signals):
+    from larmor_b200 import _core
+
+    v, n = len(signals), a.shape[1]
+    out = {name: torch.empty(shape, dtype=kind, device="cuda") for name, shape, kind in (
+        ("x", (v, n), torch.float64), ("converged", v, torch.uint8), ("status", v, torch.uint8),
+        ("outer", v, torch.int32), ("active", (v, len(g)), torch.uint8))}
+    design = _core.LsiDesign(a, g, 0.0)
+    _core.kernel_timing(True)
+    _core.fit_lsi_device(design, torch.from_numpy(signals).cuda(), *out.values())
+    torch.cuda.synchronize()
+    ms = {name: _core.kernel_time(name)[0] for name in ("lsi_group_qr_kernel", "lsi_kernel")}
+    _core.kernel_timing(False)
+    return {name: t.cpu().numpy() for name, t in out.items()}, ms
+
+
+def _doubled(rng, g):
+    return np.ascontiguousarray(np.vstack([g, g + 1e-7 * rng.standard_normal(g.shape)]))
+
+
+@pytest.mark.parametrize(("n", "shift", "mix"), [(47, 1.0, 0.5), (47, 2.0, 0.5), (60, 1.0, 1.0), (63, 0.8, 0.3), (63, 2.0, 0.7)])
+def test_active_sets_past_one_warp(cuda, oracle, n, shift, mix):
+    """Which copy is active moves x by about their distance."""
+    rng = np.random.default_rng(n)
+    m = 2 * n
+    a = rng.standard_normal((m, n))
+    g = _doubled(rng, np.eye(n) + mix * rng.standard_normal((n, n)) / np.sqrt(n))
+    signals = np.ascontiguousarray((rng.standard_normal((40, n)) - shift) @ a.T + 0.3 * rng.standard_normal((40, m)))
+    got, ms = _fit(cuda, a, g, signals)
+    rx, rconverged, rstatus, *_ = oracle.fit_lsi(a, g, 0.0, signals, details=True)
+    np.testing.assert_array_equal(got["status"], rstatus)
+    np.testing.assert_array_equal(got["converged"], rconverged)
+    by_qr = got["status"] == 1
+    assert by_qr.sum() >= 30 and got["active"][by_qr].sum(axis=1).max() > 32
+    # The variant's own fits, not handed on: the kernel behind it looks for marked voxels and finds none.
+    assert ms["lsi_kernel"] < 0.1 * ms["lsi_group_qr_kernel"], ms
+    assert np.abs(got["x"] - rx).max() <= 1e-5 * np.abs(rx).max()
+    assert (got["x"] @ g.T).min() >= -1e-8 * np.abs(got["x"]).max()
+    again, _ = _fit(cuda, a, g, signals)
+    for name in ("x", "active"):
+        np.testing.assert_array_equal(again[name], got[name])
+
+
+def test_small_near_dependent_sets_reach_the_variant(cuda, oracle):
+    rng = np.random.default_rng(7)
+    a = rng.standard_normal((60, 12))
+    g = _doubled(rng, np.vstack([np.eye(12), rng.uniform(0.0, 1.0, (28, 12))]))
+    signals = 3.0 * rng.standard_normal((64, 60))
+    got, _ = _fit(cuda, a, g, signals)
+    rx, _, rstatus, *_ = oracle.fit_lsi(a, g, 0.0, signals, details=True)
+    assert (got["status"] == 1).any()
+    np.testing.assert_array_equal(got["status"], rstatus)
+    assert np.abs(got["x"] - rx).max() <= 1e-5 * np.abs(rx).max()
