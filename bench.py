@@ -51,6 +51,15 @@ def peaks() -> tuple[dict, str]:
 NOMINAL_FP64_TENSOR_TFLOPS = 37.0
 
 
+# FP64 FMAs that an SM's CUDA cores start in a cycle (a chain-free DFMA loop measured 36.8 TFLOP/s, 37.2 by this).
+FP64_FMA_PER_SM_CYCLE = 64
+
+
+def fp64_core_tflops(sms: int, sm_mhz: float) -> float:
+    """The FP64 rate of the CUDA cores in TFLOP/s."""
+    return sms * FP64_FMA_PER_SM_CYCLE * 2 * sm_mhz * 1e6 / 1e12
+
+
 def fp64_tensor_roofline(flops_per_launch: float, avg_launch_s: float) -> dict:
     """The roofline fields of a kernel bound by the FP64 tensor cores."""
     achieved = flops_per_launch / avg_launch_s / 1e12 if avg_launch_s > 0 else 0.0
@@ -1569,16 +1578,15 @@ def measure(wl, args, world: int, rank: int, dist, dev) -> dict:
     fp64 = committed_fp64(top, wl.name)
     if fp64 is not None and avg_launch_s > 0:
         # The FP64 roofline of a CUDA-core FP64 kernel: its FLOP (counted per voxel by ncu)
-        # against the FP64 pipe's rate, 32 FP64 FMA per SM per cycle (the pipe's active
-        # fraction in the capture matches this rate: 38.6% busy at 7.5 TFLOP/s).
+        # against the FP64 pipe's rate.
         sm_mhz = line["clocks"].get("sm_mhz") or line["clocks"].get("sm_max_mhz") or 1965.0
         sms = torch.cuda.get_device_properties(dev).multi_processor_count
-        peak = sms * 32 * 2 * sm_mhz * 1e6 / 1e12
+        peak = fp64_core_tflops(sms, sm_mhz)
         achieved = fp64["fp64_flop_per_voxel"] * (voxels_all / world) * args.steps / max(top_launches, 1) \
             / avg_launch_s / 1e12
         line["fp64_roofline"] = {
             "kernel": top, "unit": "TFLOP/s", "achieved": achieved, "peak": peak, "frac": achieved / peak,
-            "peak_basis": f"{sms} SMs x 32 FP64 FMA x 2 per cycle at the median SM clock {sm_mhz} MHz",
+            "peak_basis": f"{sms} SMs x {FP64_FMA_PER_SM_CYCLE} FP64 FMA x 2 per cycle at the median SM clock {sm_mhz} MHz",
             "fp64_flop_per_voxel": fp64["fp64_flop_per_voxel"],
             "source": "profiles/fp64.json (ncu FP64 instruction counts of the same kernel and volume)"}
     if hasattr(wl, "extra"):
