@@ -72,7 +72,8 @@ const char* lar_version(void);
 int64_t lar_launch_count(void);
 
 /* Launch settings a tuner may set (no counterpart in the reference): "dti.voxels_per_cta"
- * (16, 32 or 64; used when the table fits), "log.warp.waves" (resident-CTA waves of the
+ * (16, 32 or 64, as far as a CTA of 128 threads, two to eight per voxel, and the table's
+ * shared memory allow), "log.warp.waves" (resident-CTA waves of the
  * warp-per-voxel log fit's grid, default 4), and the resident CTAs per SM of the persistent
  * grids, "dki.refit.ctas_per_sm", "lsi.ctas_per_sm", "sd.nnls.ctas_per_sm" and
  * "sd.fractions.ctas_per_sm" (at most the occupancy limit). 0 restores the library's choice.

@@ -25,7 +25,7 @@ from larmor_b200 import _lib
 
 # The settings each model's kernels read, with the values worth trying.
 CANDIDATES = {
-    "dti": {"dti.voxels_per_cta": [16, 32, 64]},
+    "dti": {"dti.voxels_per_cta": [16, 32]},
     "dki": {"log.warp.waves": [1, 2, 4, 8], "dki.refit.ctas_per_sm": [2, 3, 4]},
     "mfod": {"sd.nnls.ctas_per_sm": [2, 4, 6, 8], "sd.fractions.ctas_per_sm": [2, 3, 4]},
     "msmt": {"lsi.ctas_per_sm": [2, 3, 4, 5]},

@@ -49,7 +49,7 @@ std::mutex settings_mutex;
 std::map<std::string, int64_t> settings;
 // name -> largest accepted value
 const std::map<std::string, int64_t> kSettings = {
-    {"dti.voxels_per_cta", 64},     // voxels per CTA of the shared-memory DTI fit: 16, 32 or 64
+    {"dti.voxels_per_cta", 64},     // voxels per CTA of the shared-memory DTI fit: 16, 32 or 64, up to 128 threads
     {"log.warp.waves", 64},         // waves of resident CTAs in the warp-per-voxel log fit's grid
     {"dki.refit.ctas_per_sm", 32},  // CTAs per SM of the constrained re-fit
     {"lsi.ctas_per_sm", 32},        // CTAs per SM of the LSI

@@ -498,7 +498,7 @@ __device__ __forceinline__ void refit_violator(const LogDesignDevice<double>& d,
 // column that rounding makes dependent, a table past kFastMaxRows) they fit from the start.
 
 constexpr int kFastWarps = 12;
-constexpr int kFastMaxRows = 302;
+constexpr int kFastMaxRows = 302;  // up to here a table's weights and signals take no more of a warp's state than the NNLS
 constexpr int kP = kDkiP, kR = kP + 1;           // parameters; rows of the NNLS problem
 constexpr int kTile = 25;                        // row stride of an 8-row tile of Q
 constexpr int kNnlsDoubles = kR * kR + kR * (kR + 1) / 2;

@@ -5,11 +5,12 @@
 //
 // What bounds it: instructions and their latency (a fit is ~14 steps on 8 active of 44 columns at low
 // resolution, 22 on 12 of 300 at high). With the factor and its inverse both kept, in global slots, and two voxels
-// per warp, a low-resolution fit took 18 k warp instructions; here 7.3 k, and the shared memory of a
-// warp (6.1 KB) allows 32 warps per SM. 250,000 voxels of 280 measurements, ten rounds: low resolution 70.3 ->
-// 26.6 ms, high 35.6 -> 13.6 ms; 8,191 voxels (latency): 12.8 -> 2.9 ms and 1.66 -> 0.65 ms. Eight voxels per warp
-// with their gradients as one FP64 tensor-core product was slower at every size (42 ms, 10.5 ms): the
-// voxels' other loops diverge.
+// per warp, a low-resolution fit took 18 k warp instructions; here 7.3 k, and a warp's state is 6.1 KB of shared
+// memory: sixteen warps per SM at low resolution (one CTA; with the 44 x 44 Gram matrix it takes 115,840 bytes, and
+// two CTAs and the kilobyte that each reserves 256 bytes more than an SM has; up to 43 columns two run), twenty at
+// high. 250,000 voxels of 280 measurements, ten rounds: low resolution 70.3 -> 26.6 ms, high 35.6 -> 13.6 ms; 8,191
+// voxels (latency): 12.8 -> 2.9 ms and 1.66 -> 0.65 ms. Eight voxels per warp with their gradients as one FP64
+// tensor-core product was slower at every size (42 ms, 10.5 ms): the voxels' other loops diverge.
 //
 // - The factor is M = L^-1 alone (packed rows in shared memory) with y = M c_A and z = M^T y. Appending
 //   column e: w = M h, then one loop over the rows gives w^T M, w.w and w.y at once (every lane reads

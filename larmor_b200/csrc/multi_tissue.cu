@@ -1148,7 +1148,8 @@ __global__ void __launch_bounds__(kFracWarps * 32) lane_fractions_kernel(
     uint8_t* cols = reinterpret_cast<uint8_t*>(fsm + n + kFracWarps * 32 * kFracList) + warp * 32 * kFracList + lane;
     const FracSlot sl =
         carve_frac(workspace + (size_t(blockIdx.x) * kFracWarps + warp) * slot_size, T.m, T.ca, 1 + T.ci);
-    // Units of 32 voxels dealt to the CTAs first.
+    // Units of 32 voxels dealt to the CTAs first (a grid of a CTA per four units of the whole call: a later round's
+    // shorter list has a CTA for each of its own).
     for (int64_t p0 = (blockIdx.x + int64_t(gridDim.x) * warp) * 32; p0 < count;
          p0 += int64_t(gridDim.x) * kFracWarps * 32)
         lane_fractions_unit(T, F, R, p0 + lane < count ? listed(list, p0 + lane) : -1, vals, cols, sl, states[warp],
