@@ -8,9 +8,9 @@
 // pseudo-inverse, constraints) is small and shared by every voxel: each CTA stages X and the pseudo-inverse
 // once into shared memory.
 //
-// DTI (p = 7): four or eight neighbouring lanes per voxel (small_lanes). A lane accumulates the 28
-// normal-matrix entries and 7 right-hand sides in registers over its share of the measurements (or half of the
-// entries over a share it has in common), a butterfly sums the lanes' shares, each lane solves the 7 x 7 system by
+// DTI (p = 7): two to eight neighbouring lanes per voxel (small_lanes). A lane accumulates the 28
+// normal-matrix entries and 7 right-hand sides in registers over its share of the measurements (or some of the
+// entries over a share it has in common with others), a butterfly sums the lanes' shares, each lane solves the 7 x 7 system by
 // L D L^T in registers, and the first finishes with the tensor's eigen-decomposition (cyclic Jacobi) and the DTI
 // maps.
 
@@ -18,6 +18,7 @@
 #include <cstdio>
 #include <memory>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -73,34 +74,47 @@ __device__ __forceinline__ bool all_finite(const T (&v)[P]) {
 // ---- the IRLS of the 7-column design ------------------------------------------------------
 
 constexpr int kSmallThreads = 128;  // most of a CTA
-constexpr int kSmallCtas = 3;  // an SM's, by registers (a third more, spilling: 289 us against 293 at 79,912 voxels, 78 against 73 at 12,000)
+constexpr int kSmallCtas = 3;  // an SM's, by registers (a third more, spilling: no faster)
 
 // How a voxel's lanes share its sums over the measurements. Each sum is the sum of C partial sums, of the
 // measurements j = c mod C in increasing j, added in a butterfly of the distances C / 2, ..., 1; C depends on the
-// table alone, so a voxel's fit has the same bits in a slice, in a shard and in the whole volume.
-//   kTwo     C = 4: two lanes, two classes each (large unweighted calls)
-//   kFour    C = 4: four lanes, a class each
-//   kPairs   C = 4: eight lanes, lanes c and c + 4 sharing class c (normal_equations_halved)
-//   kEight   C = 8: eight lanes, a class each
-// Measured, microseconds:
-//   n = 31, v = 2,003 / 5,000 / 8,000 / 16,000 / 79,912: kFour 51 / 51 / 57 / 90 / 293, kPairs 49 / 57 / 86 / 128 / 529
-//   n = 94: kFour 102 / 106 / 120 / 210 / 650, kPairs 75 / 96 / 149 / 232 / 964, kEight 69 / 86 / 133 / 205 / 799
-//   n = 134: kFour 108 / 129 / 135 / 244 / 872, kEight 67 / 98 / 151 / 229 / 907;  n = 270, v = 79,912: 3,487, 2,811
-// (n = 31 with two lanes, C = 2: 274 at 79,912; with two lanes of two classes each, C = 4: 326, by its registers.)
-// An unweighted fit is seven sums and the maps, so that two lanes do where the call fills the GPU (a pass over 79,912
-// voxels of 31 measurements: 52 against 82 us with four; 20,000 of 134: 86 against 69). Past 500 measurements a
-// batch's CTA would not hold the signals of two lanes' voxels.
-enum class Lanes { kTwo, kFour, kPairs, kEight };
-__host__ __device__ constexpr int lane_count(Lanes lanes) {
-    return lanes == Lanes::kTwo ? 2 : lanes == Lanes::kFour ? 4 : 8;
+// table alone (and on whether the fit is weighted), so a voxel's fit has the same bits in a slice, in a shard and in
+// the whole volume. kCxR are C R lanes, R of them sharing a class (normal_equations_shared).
+// Measured, microseconds, at 2,003 / 5,000 / 8,000 / 12,000 / 16,000 / 24,000 / 79,912 voxels:
+//   n = 31: k2x1 73, 73, 73, 94, 96, 100, 262; k2x2 62, 69, 68, 88, 114, 137, 381; k2x4 43, 51, 77, 97, 119, 166, 494;
+//           k8x1 39, 45, 70, 88, 103, 143, 404
+//   n = 94: k2x1 171, 170, 180, 194, 216, 239, 634; k2x2 111, 124, 135, 163, 238, 285, 778; k2x4 74, 100, 160, 193, 244,
+//           336, 1013; k8x1 67, 80, 125, 150, 192, 253, 747
+//   n = 120: k2x1 182 to 924, k8x1 66, 93, 138, 167, 210, 287, 844
+// (one lane: 107 at 2,003 and 321 at 79,912 voxels of 31; four classes in four lanes: 50 and 296.)
+// kPlain is k2x1 without the reweighting, for unweighted fits: seven sums and the maps (a pass over 79,912 voxels of
+// 31 measurements: 52 us, with four lanes 82; 20,000 of 134: 86, with four lanes 65). Past 500 measurements a batch's
+// CTA would not hold the signals of two lanes' voxels.
+enum class Lanes { kPlain, k2x1, k2x2, k2x4, k8x1 };
+__host__ __device__ constexpr int class_count(Lanes lanes) { return lanes == Lanes::k8x1 ? 8 : 2; }
+__host__ __device__ constexpr int part_count(Lanes lanes) {
+    return lanes == Lanes::k2x4 ? 4 : lanes == Lanes::k2x2 ? 2 : 1;
 }
-__host__ __device__ constexpr int class_count(Lanes lanes) { return lanes == Lanes::kEight ? 8 : 4; }
+__host__ __device__ constexpr int lane_count(Lanes lanes) { return class_count(lanes) * part_count(lanes); }
 __host__ __device__ inline Lanes small_lanes(int64_t v, int n, bool weighted) {
-    if (!weighted) return n > 500 ? Lanes::kEight : v <= 20000 ? Lanes::kFour : Lanes::kTwo;
-    return n >= 128 ? Lanes::kEight : v <= 4000 ? Lanes::kPairs : Lanes::kFour;
+    if (!weighted) return n > 500 ? Lanes::k8x1 : v <= 20000 ? Lanes::k2x2 : Lanes::kPlain;
+    if (n >= 104) return Lanes::k8x1;
+    return v <= 6000 ? Lanes::k2x4 : v <= 14000 ? Lanes::k2x2 : Lanes::k2x1;
 }
 
-__host__ __device__ constexpr int small_ctas(Lanes lanes) { return lanes == Lanes::kTwo ? 2 * kSmallCtas : kSmallCtas; }
+// f with the lanes as a compile-time constant.
+template <class F>
+__host__ __device__ inline void with_lanes(Lanes lanes, const F& f) {
+    switch (lanes) {
+        case Lanes::kPlain: f(std::integral_constant<Lanes, Lanes::kPlain>{}); break;
+        case Lanes::k2x1: f(std::integral_constant<Lanes, Lanes::k2x1>{}); break;
+        case Lanes::k2x2: f(std::integral_constant<Lanes, Lanes::k2x2>{}); break;
+        case Lanes::k2x4: f(std::integral_constant<Lanes, Lanes::k2x4>{}); break;
+        default: f(std::integral_constant<Lanes, Lanes::k8x1>{});
+    }
+}
+
+__host__ __device__ constexpr int small_ctas(Lanes lanes) { return lanes == Lanes::kPlain ? 2 * kSmallCtas : kSmallCtas; }
 
 // Row strides in shared memory: of x and pinv^T (7 entries in whole 16-byte loads, eight rows of which
 // fall in distinct banks), and of the log signals of `voxels` voxels.
@@ -186,12 +200,12 @@ __device__ __forceinline__ bool ldlt_solve(T (&g)[P * (P + 1) / 2], T (&b)[P]) {
     return true;
 }
 
-// The sum of C classes, lane g of the voxel's G holding class g % C in v (or, fewer, the sum of g's and g + G's), the
-// same bits in each lane (mask: the voxel's lanes).
-template <int C, int G = C, class T, int N>
+// The sum of C classes, lane g of the voxel holding class g % C in v, the same bits in each lane (mask: the
+// voxel's lanes).
+template <int C, class T, int N>
 __device__ __forceinline__ void class_sum(T (&v)[N], unsigned mask) {
 #pragma unroll
-    for (int o = (G < C ? G : C) / 2; o > 0; o /= 2)
+    for (int o = C / 2; o > 0; o /= 2)
 #pragma unroll
         for (int i = 0; i < N; ++i) v[i] += __shfl_xor_sync(mask, v[i], o);
 }
@@ -241,60 +255,72 @@ __device__ __forceinline__ void normal_equations(const T* __restrict__ xs, int n
     class_sum<C>(r, mask);
 }
 
-// The same from eight lanes and four classes: of the class it shares, a lane takes every other exponential,
-// kAhead of them before the sums, and half the rows of [x, y]^T W [x, y]: rows 0, 3, 4, 7 or 1, 2, 5, 6, from the
-// columns 0, 2, 4 and 6 on (an entry or two below the diagonal too, which no one reads).
-template <class T>
-__device__ __forceinline__ void normal_equations_halved(const T* __restrict__ xs, int n, const T* __restrict__ ys,
+// Row k of part `part` of R of the rows of [x, y], and the first column it is summed from (an entry or more below the
+// diagonal too for some parts, which no one reads): two parts 0, 3, 4, 7 and 1, 2, 5, 6 from the columns 0, 2, 4, 6;
+// four parts 0, 7 and 1, 6 and 2, 5 and 3, 4 from the columns 0, 4.
+__host__ __device__ constexpr int part_row(int R, int part, int k) {
+    if (R == 4) return k == 0 ? part : 7 - part;
+    return 2 * k + (k & 1 ? 1 - part : part);
+}
+__host__ __device__ constexpr int part_column(int R, int k) { return R * k; }
+
+// The same from C R lanes: of the class that R lanes share, each takes every R-th exponential, kAhead of them before
+// the sums, and the sums of 8 / R rows of [x, y]^T W [x, y].
+template <class T, int C, int R>
+__device__ __forceinline__ void normal_equations_shared(const T* __restrict__ xs, int n, const T* __restrict__ ys,
                                                         int stride, const T (&p)[7], T mx, int g, unsigned mask,
                                                         T (&m)[28], T (&r)[7]) {
-    constexpr int P = 7, LD = row_ld<T>(), C = 4, kAhead = 4;
-    const int c = g % C, half = g / C;
-    T acc[4][8];
+    constexpr int P = 7, LD = row_ld<T>(), kRows = 8 / R, kAhead = 4;
+    const int c = g % C, part = g / C, first = int(threadIdx.x % 32) - g + c;  // the class's lane of part 0
+    T acc[kRows][8];
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
+    for (int k = 0; k < kRows; ++k)
 #pragma unroll
         for (int b = 0; b < 8; ++b) acc[k][b] = T(0);
-    for (int j0 = c; j0 - c < n; j0 += 2 * kAhead * C) {
+    for (int j0 = c; j0 - c < n; j0 += kAhead * R * C) {
         T mine[kAhead], x[8];
 #pragma unroll
         for (int u = 0; u < kAhead; ++u) {
-            load_row(xs + min(j0 + (2 * u + half) * C, n - 1) * LD, x);
+            load_row(xs + min(j0 + (R * u + part) * C, n - 1) * LD, x);
             mine[u] = dev_exp<T>(T(2) * (predict(x, p) - mx));
         }
 #pragma unroll
-        for (int u = 0; u < 2 * kAhead; ++u) {
-            const T from = __shfl_sync(mask, mine[u / 2], int(threadIdx.x % 32) - g + c + C * (u & 1));
+        for (int u = 0; u < R * kAhead; ++u) {
+            const T from = __shfl_sync(mask, mine[u / R], first + C * (u % R));
             const int j = j0 + C * u, at = min(j, n - 1);
             const T w = j < n ? from : T(0);  // adds zeros past the last
             load_row(xs + at * LD, x);
             x[7] = ys[at * stride];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                constexpr int kFirst[4] = {0, 3, 4, 7}, kSecond[4] = {1, 2, 5, 6};
-                const T wx = w * (half == 0 ? x[kFirst[k]] : x[kSecond[k]]);
+            for (int k = 0; k < kRows; ++k) {
+                T row = x[part_row(R, 0, k)];
+#pragma unroll
+                for (int q = 1; q < R; ++q) row = part == q ? x[part_row(R, q, k)] : row;
+                const T wx = w * row;
 #pragma unroll
                 for (int b = 0; b < 8; ++b)
-                    if (b >= 2 * k) acc[k][b] = fma(wx, x[b], acc[k][b]);
+                    if (b >= part_column(R, k)) acc[k][b] = fma(wx, x[b], acc[k][b]);
             }
         }
     }
 #pragma unroll
-    for (int k = 0; k < 4; ++k) class_sum<C>(acc[k], mask);
+    for (int k = 0; k < kRows; ++k) class_sum<C>(acc[k], mask);
 #pragma unroll
-    for (int a = 0; a < P; ++a) {
-        constexpr int kHalf[P] = {0, 1, 1, 0, 0, 1, 1}, kSlot[P] = {0, 0, 1, 1, 2, 2, 3};
+    for (int q = 0; q < R; ++q)
 #pragma unroll
-        for (int b = 0; b < 8; ++b) {
-            if (b < a) continue;
-            const T own = acc[kSlot[a]][b], other = __shfl_xor_sync(mask, own, C);
-            const T entry = half == kHalf[a] ? own : other;
-            if (b < P)
-                m[packed(a, b, P)] = entry;
-            else
-                r[a] = entry;
+        for (int k = 0; k < kRows; ++k) {
+            const int a = part_row(R, q, k);
+            if (a >= P) continue;
+#pragma unroll
+            for (int b = 0; b < 8; ++b) {
+                if (b < a) continue;
+                const T entry = __shfl_sync(mask, acc[k][b], first + C * q);
+                if (b < P)
+                    m[packed(a, b, P)] = entry;
+                else
+                    r[a] = entry;
+            }
         }
-    }
 }
 
 // Fits one voxel from its log signals ys[j * stride] on its lanes, and leaves its scaled parameters in p
@@ -310,30 +336,20 @@ __device__ __forceinline__ int fit_voxel_small(const T* __restrict__ xs, const T
     const int g = int(threadIdx.x) % G;
     const unsigned mask = ((1u << G) - 1u) << (threadIdx.x % 32 - g);
     auto ordinary = [&] {
-        constexpr int K = G < C ? C / G : 1;
-        T sum[K][P];
 #pragma unroll
-        for (int q = 0; q < K; ++q)
-#pragma unroll
-            for (int a = 0; a < P; ++a) sum[q][a] = T(0);
+        for (int a = 0; a < P; ++a) p[a] = T(0);
 #pragma unroll 2
-        for (int j0 = g % C; j0 < n; j0 += C)
+        for (int j = g % C; j < n; j += C) {
+            const T y = ys[j * stride];
+            T row[8];
+            load_row(pinvt + j * LD, row);
 #pragma unroll
-            for (int q = 0; q < K; ++q) {
-                const int j = j0 + q * G;
-                if (q > 0 && j >= n) continue;
-                const T y = ys[j * stride];
-                T row[8];
-                load_row(pinvt + j * LD, row);
-#pragma unroll
-                for (int a = 0; a < P; ++a) sum[q][a] = fma(row[a], y, sum[q][a]);
-            }
-#pragma unroll
-        for (int a = 0; a < P; ++a) p[a] = K > 1 ? sum[0][a] + sum[K - 1][a] : sum[0][a];
-        class_sum<C, G>(p, mask);
+            for (int a = 0; a < P; ++a) p[a] = fma(row[a], y, p[a]);
+        }
+        class_sum<C>(p, mask);
     };
     ordinary();
-    if constexpr (LANES == Lanes::kTwo) return 0;  // unweighted fits only (small_lanes)
+    if constexpr (LANES == Lanes::kPlain) return 0;
     if (!weighted || !all_finite(p)) return 0;
     T mx = -INFINITY;
 #pragma unroll 2
@@ -346,8 +362,8 @@ __device__ __forceinline__ int fit_voxel_small(const T* __restrict__ xs, const T
     int it = 0;
     for (; it < max_rw; ++it) {
         T m[PP], r[P];
-        if constexpr (LANES == Lanes::kPairs)
-            normal_equations_halved<T>(xs, n, ys, stride, p, mx, g, mask, m, r);
+        if constexpr (G > C)
+            normal_equations_shared<T, C, G / C>(xs, n, ys, stride, p, mx, g, mask, m, r);
         else
             normal_equations<T, C>(xs, n, ys, stride, p, mx, g, mask, m, r);
         if (!ldlt_solve<T, P>(m, r) || !all_finite(r)) {
@@ -495,12 +511,9 @@ __global__ void __launch_bounds__(kDtiBatchThreads, kSmallCtas * kSmallThreads /
             stage_design<double>(job.d, sm);
             cur = j;
         }
-        switch (small_lanes(job.v, job.d.n, weighted != 0)) {
-            case Lanes::kTwo: batch_dti_ticket<Lanes::kTwo>(job, t - first[j], weighted, max_rw, tol, sm); break;
-            case Lanes::kEight: batch_dti_ticket<Lanes::kEight>(job, t - first[j], weighted, max_rw, tol, sm); break;
-            case Lanes::kPairs: batch_dti_ticket<Lanes::kPairs>(job, t - first[j], weighted, max_rw, tol, sm); break;
-            default: batch_dti_ticket<Lanes::kFour>(job, t - first[j], weighted, max_rw, tol, sm);
-        }
+        with_lanes(small_lanes(job.v, job.d.n, weighted != 0), [&](auto lanes) {
+            batch_dti_ticket<decltype(lanes)::value>(job, t - first[j], weighted, max_rw, tol, sm);
+        });
         __syncthreads();
     }
 }
@@ -518,7 +531,7 @@ const LogDesignDevice<float>& device_view<float>(const lar_log_design_s* h) { re
 template <class T>
 int small_threads(int64_t v, int n, int lanes) {
     const int64_t want = launch_setting("dti.voxels_per_cta");
-    int threads = v <= 4000 ? 64 : kSmallThreads;
+    int threads = v <= 6000 ? 64 : kSmallThreads;
     if (want == 16 || want == 32 || want == 64) threads = int(std::min<int64_t>(kSmallThreads, want * lanes));
     while (threads > 16 && small_bytes<T>(n, threads / lanes) > 227 * 1024) threads /= 2;
     return threads;
@@ -600,12 +613,10 @@ void launch_fit(lar_log_design_s* h, const double* log_s, int64_t v, int weighte
                                                             iterations);
             cuda_check(cudaGetLastError(), "fit_log_small_kernel launch");
         };
-        switch (small_lanes(v, d.n, weighted != 0)) {
-            case Lanes::kTwo: run(fit_log_small_kernel<T, Lanes::kTwo, LogSource>, 2); break;
-            case Lanes::kEight: run(fit_log_small_kernel<T, Lanes::kEight, LogSource>, 8); break;
-            case Lanes::kPairs: run(fit_log_small_kernel<T, Lanes::kPairs, LogSource>, 8); break;
-            default: run(fit_log_small_kernel<T, Lanes::kFour, LogSource>, 4);
-        }
+        with_lanes(small_lanes(v, d.n, weighted != 0), [&](auto lanes) {
+            constexpr Lanes kLanes = decltype(lanes)::value;
+            run(fit_log_small_kernel<T, kLanes, LogSource>, lane_count(kLanes));
+        });
         return;
     }
     launch_general<T>(h, src, v, weighted, max_rw, tol, params, broke, iterations, stream);
@@ -626,12 +637,10 @@ void launch_dti_maps(const lar_log_design_s* h, const float* s, const double* fl
         kernel<<<unsigned(grid), threads, sm, stream>>>(d, src, v, weighted, max_rw, T(tol), maps, npd, params);
         cuda_check(cudaGetLastError(), "fit_dti_maps_kernel launch");
     };
-    switch (small_lanes(v, d.n, weighted != 0)) {
-        case Lanes::kTwo: run(fit_dti_maps_kernel<T, Lanes::kTwo>, 2); break;
-        case Lanes::kEight: run(fit_dti_maps_kernel<T, Lanes::kEight>, 8); break;
-        case Lanes::kPairs: run(fit_dti_maps_kernel<T, Lanes::kPairs>, 8); break;
-        default: run(fit_dti_maps_kernel<T, Lanes::kFour>, 4);
-    }
+    with_lanes(small_lanes(v, d.n, weighted != 0), [&](auto lanes) {
+        constexpr Lanes kLanes = decltype(lanes)::value;
+        run(fit_dti_maps_kernel<T, kLanes>, lane_count(kLanes));
+    });
 }
 
 }  // namespace
