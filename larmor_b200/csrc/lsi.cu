@@ -15,8 +15,8 @@
 //   rows_product_kernel    rotated = q_t s for every voxel (a tiled FP64 product), left in x;
 //   lsi_group_kernel       the LDP steps, a group of warps per voxel (see below), x <- scale E^T u /
 //                          (1 - f.u) + rotated; a voxel whose factor fails is marked and listed;
-//   lsi_group_kernel<.., QR>  the listed voxels, with orthonormal rows instead of the Cholesky
-//                          factor; what it cannot take either stays marked for
+//   lsi_group_kernel<.., QR>  the listed voxels (and those past the list's end), with orthonormal rows instead of the
+//                          Cholesky factor; what it cannot take either stays marked for
 //   lsi_kernel             one warp per marked voxel by the QR-based NNLS (warp_nnls.cuh), also
 //                          the whole fit where the group kernel's shared memory does not hold the
 //                          problem or only_qr asks for it;
@@ -42,6 +42,7 @@ constexpr int kLsiWarps = 4;
 constexpr int kFactorCap = 64;   // active columns the Cholesky factor can hold (>= n + 1)
 constexpr double kMinRelativePivot = 1e-12;
 constexpr uint8_t kMarked = 2;     // converged[] of a voxel still to be fitted by a fallback
+constexpr uint8_t kUnlisted = 3;   // the same, for the QR variant, past what its list holds
 constexpr int kColsPerLane = 16;  // constraint columns a lane holds gradients for (k <= 512)
 
 struct LsiDevice {
@@ -406,7 +407,9 @@ __global__ void __launch_bounds__(kLsiWarps * 32, 4) lsi_kernel(LsiDevice D, con
 constexpr int kGroupNW = 1;       // warps per voxel (2: 102 ms on the volume below, 4: 135 ms)
 constexpr int kGroups = 8;        // voxels per CTA (one CTA per SM)
 constexpr int kQrNW = 8;          // the QR variant: one voxel per CTA
-constexpr int kRedoCap = 1 << 16;  // voxels the QR variant's list holds; the others stay marked
+// Voxels the QR variant's list holds (its size does not grow with the call, so that a captured call needs no larger
+// scratch); it looks the others up by their mark, so that they are fitted the same way.
+constexpr int kRedoCap = 1 << 16;
 constexpr double kQrMinPivot = 1e-26;  // squared, relative: below it a column is dependent
 
 struct GroupLayout {
@@ -805,22 +808,20 @@ __device__ __forceinline__ bool group_inner(const GroupLayout& lay, const GroupV
     }
 }
 
-// x holds the rotated signals and gets scale E^T u / (1 - f.u) + rotated. `list` (with its count
-// on the device) names the voxels, null for all v. K constraints per thread: 32 NW K >= k.
+// x holds the rotated signals and gets scale E^T u / (1 - f.u) + rotated, for all v voxels, or with QR for those of
+// `list` (redo_count of them, as many as it holds) and then those marked kUnlisted, 32 voxels to a ticket of queue[2]. K constraints per thread: 32 NW K >= k.
 template <int NW, int GROUPS, int K, bool QR>
 __global__ void __launch_bounds__(NW * GROUPS * 32, 1) lsi_group_kernel(
-    LsiDevice D, int64_t v, const int* __restrict__ list, const int* __restrict__ list_count, int* queue,
-    int* __restrict__ redo, int* redo_count, double* __restrict__ x, uint8_t* __restrict__ converged,
-    uint8_t* __restrict__ status, int32_t* __restrict__ outer_out, uint8_t* __restrict__ active_out) {
+    LsiDevice D, int64_t v, int* queue, int* list, int* list_count, double* __restrict__ x,
+    uint8_t* __restrict__ converged, uint8_t* __restrict__ status, int32_t* __restrict__ outer_out,
+    uint8_t* __restrict__ active_out) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* const sm = reinterpret_cast<double*>(smem_raw);
     const int n = D.n, k = D.k;
     const GroupLayout lay{n, k, NW, GROUPS, QR};
     const int kp = lay.kp(), cap = lay.cap(), words = lay.mask_words();
-    if (list_count != nullptr) {
-        v = min(int64_t(*list_count), int64_t(kRedoCap));
-        if (v == 0) return;
-    }
+    const int failed = QR ? *list_count : 0;
+    if (QR && failed == 0) return;
     const int warp = threadIdx.x >> 5;
     const Place<NW> at{int(threadIdx.x & 31), warp % NW, warp / NW};
     const int lane = at.lane, gtid = at.wig * 32 + lane;
@@ -851,13 +852,37 @@ __global__ void __launch_bounds__(NW * GROUPS * 32, 1) lsi_group_kernel(
     }
     __syncthreads();
     const int max_inner = 3 * k;
+    bool by_mark = false;
+    int64_t first = 0;   // by_mark: the ticket's 32 voxels, and
+    unsigned todo = 0u;  // those of them still to be fitted
     for (;;) {
         // The group's next voxel.
-        if (gtid == 0) *g.ticket = atomicAdd(queue, 1);
-        at.sync();
-        const int64_t p = *g.ticket;
-        if (p >= v) break;
-        const int64_t voxel = list ? int64_t(list[p]) : p;
+        int64_t voxel = first + __ffs(todo) - 1;
+        if (todo == 0u) {
+            if (gtid == 0) *g.ticket = atomicAdd(by_mark ? queue + 2 : queue, 1);
+            at.sync();
+            voxel = *g.ticket;
+            if constexpr (QR) {
+                if (by_mark) {
+                    first = 32 * voxel;
+                    if (first >= v) break;
+                    todo = __ballot_sync(0xffffffffu, first + lane < v && converged[first + lane] == kUnlisted);
+                    at.sync();  // every warp has read the ticket and the marks
+                    continue;
+                }
+                if (voxel >= min(failed, kRedoCap)) {
+                    if (failed <= kRedoCap) break;
+                    by_mark = true;
+                    at.sync();
+                    continue;
+                }
+                voxel = list[voxel];
+            } else if (voxel >= v) {
+                break;
+            }
+        } else {
+            todo &= todo - 1u;
+        }
         double rot[2];
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
@@ -1005,12 +1030,16 @@ __global__ void __launch_bounds__(NW * GROUPS * 32, 1) lsi_group_kernel(
             if (!group_append<QR, NW>(D, lay, et, g, na, e, at) ||
                 !group_inner<QR, NW>(lay, g, na, inner, max_inner, tol, at)) {
                 if (gtid == 0) {
-                    converged[voxel] = kMarked;
+                    uint8_t mark = kMarked;
                     if (!QR) {
                         if (outer_out) outer_out[voxel] = outer;
-                        const int slot = atomicAdd(redo_count, 1);
-                        if (slot < kRedoCap) redo[slot] = int(voxel);
+                        const int slot = atomicAdd(list_count, 1);
+                        if (slot < kRedoCap)
+                            list[slot] = int(voxel);
+                        else
+                            mark = kUnlisted;
                     }
+                    converged[voxel] = mark;
                 }
                 break;
             }
@@ -1078,8 +1107,7 @@ void launch_rows_product(const double* in, int64_t v, int m, const double* b, in
     cuda_check(cudaGetLastError(), "rows_product_kernel launch");
 }
 
-using GroupKernel = void (*)(LsiDevice, int64_t, const int*, const int*, int*, int*, int*, double*, uint8_t*, uint8_t*,
-                             int32_t*, uint8_t*);
+using GroupKernel = void (*)(LsiDevice, int64_t, int*, int*, int*, double*, uint8_t*, uint8_t*, int32_t*, uint8_t*);
 
 // The group kernels of a problem, or null where their shared memory does not hold it or k is past
 // their threads' constraints.
@@ -1217,9 +1245,9 @@ int lar_fit_lsi(lar_lsi_design design, const double* signals, int64_t v, int onl
         }
         auto st = static_cast<cudaStream_t>(stream);
         char* base = static_cast<char*>(design->scratch);
-        // [0] lsi_kernel's queue, [1] and [2] the group kernels', [3] the listed voxels.
+        // [0] lsi_kernel's queue, [1] and [2] the group kernels', [3] the listed voxels, [4] the QR variant's marks.
         int* counters = reinterpret_cast<int*>(base);
-        cuda_check(cudaMemsetAsync(base, 0, 4 * sizeof(int), st), "cudaMemsetAsync");
+        cuda_check(cudaMemsetAsync(base, 0, 5 * sizeof(int), st), "cudaMemsetAsync");
         LsiDevice D{int(h.m), int(h.n), int(h.k), design->qt.ptr, design->back.ptr, design->et.ptr,
                     design->e.ptr, design->gram.ptr, design->abs_sums.ptr};
         if (grouped) {
@@ -1232,13 +1260,13 @@ int lar_fit_lsi(lar_lsi_design design, const double* signals, int64_t v, int onl
             {
                 LaunchScope scope("lsi_group_kernel", st);
                 plan.main<<<grid, kGroupNW * kGroups * 32, plan.main_smem, st>>>(
-                    D, v, nullptr, nullptr, counters + 1, redo, counters + 3, x, converged, status, outer, active);
+                    D, v, counters + 1, redo, counters + 3, x, converged, status, outer, active);
                 cuda_check(cudaGetLastError(), "lsi_group_kernel launch");
             }
             {
                 LaunchScope scope("lsi_group_qr_kernel", st);
                 plan.qr<<<unsigned(std::min<int64_t>(v, sm_count())), kQrNW * 32, plan.qr_smem, st>>>(
-                    D, v, redo, counters + 3, counters + 2, nullptr, nullptr, x, converged, status, outer, active);
+                    D, v, counters + 2, redo, counters + 3, x, converged, status, outer, active);
                 cuda_check(cudaGetLastError(), "lsi_group_qr_kernel launch");
             }
             launch_rows_product(x, v, D.n, design->back_t.ptr, D.n, x, st);

@@ -64,3 +64,22 @@ def test_small_near_dependent_sets_reach_the_variant(cuda, oracle):
     assert (got["status"] == 1).any()
     np.testing.assert_array_equal(got["status"], rstatus)
     assert np.abs(got["x"] - rx).max() <= 1e-5 * np.abs(rx).max()
+
+
+def test_more_failed_factors_than_the_list_holds(cuda):
+    """75,000 or so of 110,000 voxels need the QR variant, whose list holds 65,536: the others are fitted by it too, so
+    that a voxel's bits depend neither on the size of its call nor on which voxels came onto the list first."""
+    rng = np.random.default_rng(12)
+    a = rng.standard_normal((24, 12))
+    g = np.vstack([np.eye(12), rng.uniform(0.0, 1.0, (28, 12))])
+    g = np.ascontiguousarray(np.vstack([g + 1e-7 * rng.standard_normal(g.shape) for _ in range(4)]))
+    signals = 3.0 * rng.standard_normal((110_000, 24))
+    whole, ms = _fit(cuda, a, g, signals)
+    assert (whole["status"] == 1).sum() > 65_536 and whole["converged"].all()
+    assert ms["lsi_kernel"] < 0.1 * ms["lsi_group_qr_kernel"], ms
+    again, _ = _fit(cuda, a, g, signals)
+    pieces = [_fit(cuda, a, g, signals[b:b + 55_000])[0] for b in (0, 55_000)]
+    assert max((p["status"] == 1).sum() for p in pieces) < 65_536
+    for name in ("x", "active", "status"):
+        np.testing.assert_array_equal(again[name], whole[name])
+        np.testing.assert_array_equal(np.concatenate([p[name] for p in pieces]), whole[name])
