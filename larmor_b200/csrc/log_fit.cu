@@ -78,27 +78,30 @@ constexpr int kSmallCtas = 3;  // an SM's, by registers (a third more, spilling:
 
 // How a voxel's lanes share its sums over the measurements. Each sum is the sum of C partial sums, of the
 // measurements j = c mod C in increasing j, added in a butterfly of the distances C / 2, ..., 1; C depends on the
-// table alone (and on whether the fit is weighted), so a voxel's fit has the same bits in a slice, in a shard and in
-// the whole volume. kCxR are C R lanes, R of them sharing a class (normal_equations_shared).
+// table alone, so a voxel's fit has the same bits in a slice, in a shard and in the whole volume. kCxR are C R lanes, R
+// of them sharing a class (normal_equations_shared).
 // Measured, microseconds, at 2,003 / 5,000 / 8,000 / 12,000 / 16,000 / 24,000 / 79,912 voxels:
-//   n = 31: k2x1 73, 73, 73, 94, 96, 100, 262; k2x2 62, 69, 68, 88, 114, 137, 381; k2x4 43, 51, 77, 97, 119, 166, 494;
-//           k8x1 39, 45, 70, 88, 103, 143, 404
-//   n = 94: k2x1 171, 170, 180, 194, 216, 239, 634; k2x2 111, 124, 135, 163, 238, 285, 778; k2x4 74, 100, 160, 193, 244,
-//           336, 1013; k8x1 67, 80, 125, 150, 192, 253, 747
-//   n = 120: k2x1 182 to 924, k8x1 66, 93, 138, 167, 210, 287, 844
+//   n = 31: k2x1 73, 73, 73, 96, 96, 100, 261; k2x2 62, 63, 68, 88, 114, 137, 382; k2x4 43, 51, 75, 94, 116, 160, 476;
+//           k8x1 39, 47, 69, 87, 102, 143, 405
+//   n = 94: k2x1 171, 172, 182, 193, 217, 238, 636; k2x2 112, 119, 135, 164, 239, 286, 778; k2x4 71, 101, 154, 186, 235,
+//           320, 961; k8x1 67, 82, 125, 151, 191, 254, 746
+//   n = 120: k2x1 182 to 924; k8x1 66, 93, 138, 167, 210, 287, 844
 // (one lane: 107 at 2,003 and 321 at 79,912 voxels of 31; four classes in four lanes: 50 and 296.)
-// kPlain is k2x1 without the reweighting, for unweighted fits: seven sums and the maps (a pass over 79,912 voxels of
-// 31 measurements: 52 us, with four lanes 82; 20,000 of 134: 86, with four lanes 65). Past 500 measurements a batch's
-// CTA would not hold the signals of two lanes' voxels.
-enum class Lanes { kPlain, k2x1, k2x2, k2x4, k8x1 };
+// The ordinary fit, an unweighted call's and the one a weighted fit starts from and falls back to, has eight classes
+// everywhere, one, two or four to a lane, so that the two have the same bits. An unweighted call is its seven sums and
+// the maps, on eight lanes in small calls and on four or two in larger ones (k8x1, kPlain4, kPlain2): 2,003 voxels of 31
+// measurements 13, 13, 18, 79,912 of them 100, 45, 37; of 134 20, 26, 41 and 172, 127, 180. Past 500 measurements a
+// batch's CTA would not hold the signals of two lanes' voxels.
+enum class Lanes { kPlain2, kPlain4, k2x1, k2x2, k2x4, k8x1 };
+__host__ __device__ constexpr bool plain(Lanes lanes) { return lanes == Lanes::kPlain2 || lanes == Lanes::kPlain4; }
 __host__ __device__ constexpr int class_count(Lanes lanes) { return lanes == Lanes::k8x1 ? 8 : 2; }
-__host__ __device__ constexpr int part_count(Lanes lanes) {
-    return lanes == Lanes::k2x4 ? 4 : lanes == Lanes::k2x2 ? 2 : 1;
+constexpr int kOrdinaryClasses = 8;
+__host__ __device__ constexpr int lane_count(Lanes lanes) {
+    return lanes == Lanes::kPlain2 || lanes == Lanes::k2x1 ? 2 : lanes == Lanes::kPlain4 || lanes == Lanes::k2x2 ? 4 : 8;
 }
-__host__ __device__ constexpr int lane_count(Lanes lanes) { return class_count(lanes) * part_count(lanes); }
 __host__ __device__ inline Lanes small_lanes(int64_t v, int n, bool weighted) {
-    if (!weighted) return n > 500 ? Lanes::k8x1 : v <= 20000 ? Lanes::k2x2 : Lanes::kPlain;
-    if (n >= 104) return Lanes::k8x1;
+    if (!weighted) return n > 500 || v <= 6000 ? Lanes::k8x1 : v <= 20000 || n >= 80 ? Lanes::kPlain4 : Lanes::kPlain2;
+    if (n >= 96) return Lanes::k8x1;
     return v <= 6000 ? Lanes::k2x4 : v <= 14000 ? Lanes::k2x2 : Lanes::k2x1;
 }
 
@@ -106,7 +109,8 @@ __host__ __device__ inline Lanes small_lanes(int64_t v, int n, bool weighted) {
 template <class F>
 __host__ __device__ inline void with_lanes(Lanes lanes, const F& f) {
     switch (lanes) {
-        case Lanes::kPlain: f(std::integral_constant<Lanes, Lanes::kPlain>{}); break;
+        case Lanes::kPlain2: f(std::integral_constant<Lanes, Lanes::kPlain2>{}); break;
+        case Lanes::kPlain4: f(std::integral_constant<Lanes, Lanes::kPlain4>{}); break;
         case Lanes::k2x1: f(std::integral_constant<Lanes, Lanes::k2x1>{}); break;
         case Lanes::k2x2: f(std::integral_constant<Lanes, Lanes::k2x2>{}); break;
         case Lanes::k2x4: f(std::integral_constant<Lanes, Lanes::k2x4>{}); break;
@@ -114,7 +118,7 @@ __host__ __device__ inline void with_lanes(Lanes lanes, const F& f) {
     }
 }
 
-__host__ __device__ constexpr int small_ctas(Lanes lanes) { return lanes == Lanes::kPlain ? 2 * kSmallCtas : kSmallCtas; }
+__host__ __device__ constexpr int small_ctas(Lanes lanes) { return plain(lanes) ? 2 * kSmallCtas : kSmallCtas; }
 
 // Row strides in shared memory: of x and pinv^T (7 entries in whole 16-byte loads, eight rows of which
 // fall in distinct banks), and of the log signals of `voxels` voxels.
@@ -200,8 +204,8 @@ __device__ __forceinline__ bool ldlt_solve(T (&g)[P * (P + 1) / 2], T (&b)[P]) {
     return true;
 }
 
-// The sum of C classes, lane g of the voxel holding class g % C in v, the same bits in each lane (mask: the
-// voxel's lanes).
+// The sum of C classes, or of the C sums that lanes hold of theirs, lane g of the voxel holding that of g % C in v, the
+// same bits in each lane (mask: the voxel's lanes).
 template <int C, class T, int N>
 __device__ __forceinline__ void class_sum(T (&v)[N], unsigned mask) {
 #pragma unroll
@@ -293,9 +297,12 @@ __device__ __forceinline__ void normal_equations_shared(const T* __restrict__ xs
             x[7] = ys[at * stride];
 #pragma unroll
             for (int k = 0; k < kRows; ++k) {
-                T row = x[part_row(R, 0, k)];
-#pragma unroll
-                for (int q = 1; q < R; ++q) row = part == q ? x[part_row(R, q, k)] : row;
+                // The part's row: of four parts from shared memory again (selecting it took a third of the loop).
+                T row;
+                if (R == 4)
+                    row = k == 0 ? xs[at * LD + part] : part == 0 ? x[7] : xs[at * LD + 7 - part];
+                else
+                    row = part == 0 ? x[part_row(R, 0, k)] : x[part_row(R, 1, k)];
                 const T wx = w * row;
 #pragma unroll
                 for (int b = 0; b < 8; ++b)
@@ -336,20 +343,36 @@ __device__ __forceinline__ int fit_voxel_small(const T* __restrict__ xs, const T
     const int g = int(threadIdx.x) % G;
     const unsigned mask = ((1u << G) - 1u) << (threadIdx.x % 32 - g);
     auto ordinary = [&] {
+        constexpr int K = kOrdinaryClasses / G;  // classes of a lane
+        T sum[K][P];
 #pragma unroll
-        for (int a = 0; a < P; ++a) p[a] = T(0);
+        for (int q = 0; q < K; ++q)
+#pragma unroll
+            for (int a = 0; a < P; ++a) sum[q][a] = T(0);
 #pragma unroll 2
-        for (int j = g % C; j < n; j += C) {
-            const T y = ys[j * stride];
-            T row[8];
-            load_row(pinvt + j * LD, row);
+        for (int j0 = g; j0 < n; j0 += kOrdinaryClasses)
 #pragma unroll
-            for (int a = 0; a < P; ++a) p[a] = fma(row[a], y, p[a]);
-        }
-        class_sum<C>(p, mask);
+            for (int q = 0; q < K; ++q) {
+                const int j = j0 + q * G;
+                if (q > 0 && j >= n) continue;
+                const T y = ys[j * stride];
+                T row[8];
+                load_row(pinvt + j * LD, row);
+#pragma unroll
+                for (int a = 0; a < P; ++a) sum[q][a] = fma(row[a], y, sum[q][a]);
+            }
+#pragma unroll
+        for (int o = K / 2; o > 0; o /= 2)
+#pragma unroll
+            for (int q = 0; q < o; ++q)
+#pragma unroll
+                for (int a = 0; a < P; ++a) sum[q][a] += sum[q + o][a];
+#pragma unroll
+        for (int a = 0; a < P; ++a) p[a] = sum[0][a];
+        class_sum<G>(p, mask);
     };
     ordinary();
-    if constexpr (LANES == Lanes::kPlain) return 0;
+    if constexpr (plain(LANES)) return 0;
     if (!weighted || !all_finite(p)) return 0;
     T mx = -INFINITY;
 #pragma unroll 2

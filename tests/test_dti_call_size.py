@@ -39,7 +39,7 @@ def _fit(torch, design, s, weighted, precision):
 
 # Tables of a voxel's smallest share of measurements, of whole and ragged shares, and around the table size where the
 # lanes' classes change; the pieces lie on both sides of every voxel count where the lanes per voxel do.
-@pytest.mark.parametrize("n", [7, 8, 31, 37, 64, 103, 104, 135])
+@pytest.mark.parametrize("n", [7, 8, 31, 37, 64, 95, 96, 135])
 @pytest.mark.parametrize(("weighted", "precision"), [(True, _lib.LAR_FP64), (False, _lib.LAR_FP64), (True, _lib.LAR_FP32)])
 def test_a_voxel_has_the_same_bits_in_any_call(cuda, n, weighted, precision):
     from larmor_b200 import _core
@@ -62,3 +62,25 @@ def test_large_tables_are_accepted_at_every_call_size(cuda):
     small, large = _fit(cuda, handle, s[:300].contiguous(), True, _lib.LAR_FP64), _fit(cuda, handle, s, True, _lib.LAR_FP64)
     for a, b in zip(small, large):
         np.testing.assert_array_equal(a, b[:300])
+
+
+@pytest.mark.parametrize("n", [31, 64, 95, 96, 135])
+@pytest.mark.parametrize("v", [50, 9_000, 25_000])
+def test_the_fallback_is_the_unweighted_fit(cuda, n, v):
+    """Every third voxel's diffusion-weighted signals lie e^2000 below its one b0: all their weights are exactly 0, the
+    normal matrix has exactly zero pivots, and the ordinary fit stands: the bits of an unweighted call's, whatever the
+    lanes of either."""
+    from larmor_b200 import _core
+
+    design, s = _problem(cuda, n, v)
+    handle = _core.LogDesign(design, np.zeros((0, 7)))
+    log_s = cuda.log(s.double())
+    log_s[::3, 1:] -= 2000.0
+    fits = []
+    for weighted in (True, False):
+        params = cuda.empty((v, 7), dtype=cuda.float64, device="cuda")
+        broke, steps = (cuda.empty(v, dtype=kind, device="cuda") for kind in (cuda.uint8, cuda.int32))
+        _core.fit_log_signal_device(handle, log_s, weighted, 20, 1e-6, params, broke, steps)
+        fits.append(params.cpu().numpy())
+    np.testing.assert_array_equal(fits[0][::3], fits[1][::3])
+    assert (fits[0][1::3] != fits[1][1::3]).any()
