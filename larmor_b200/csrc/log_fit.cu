@@ -81,10 +81,11 @@ constexpr int kSmallCtas = 3;  // an SM's, by registers (a third more, spilling:
 // table alone, so a voxel's fit has the same bits in a slice, in a shard and in the whole volume. kCxR are C R lanes, R
 // of them sharing a class (normal_equations_shared).
 // Measured, microseconds, at 2,003 / 5,000 / 8,000 / 12,000 / 16,000 / 24,000 / 79,912 voxels:
-//   n = 31: k2x1 73, 73, 73, 96, 96, 100, 261; k2x2 62, 63, 68, 88, 114, 137, 382; k2x4 43, 51, 75, 94, 116, 160, 476;
-//           k8x1 39, 47, 69, 87, 102, 143, 405
-//   n = 94: k2x1 171, 172, 182, 193, 217, 238, 636; k2x2 112, 119, 135, 164, 239, 286, 778; k2x4 71, 101, 154, 186, 235,
-//           320, 961; k8x1 67, 82, 125, 151, 191, 254, 746
+//   n = 13: k2x1 65, 66, 66, 77, 75, 93, 215; k2x2 75, 81, 85, 95, 132, 152; k2x4 55, 65, 92, 104, 130, 174
+//   n = 31: k2x1 74, 73, 73, 96, 97, 100, 261; k2x2 63, 65, 69, 90, 118, 140, 382; k2x4 43, 51, 76, 95, 116, 162, 476;
+//           k8x1 39, 47, 70, 87, 103, 142, 405
+//   n = 94: k2x1 172, 172, 182, 194, 217, 237, 636; k2x2 116, 123, 139, 167, 246, 293, 778; k2x4 74, 100, 154, 186, 240,
+//           324, 961; k8x1 67, 82, 124, 150, 191, 254, 746
 //   n = 120: k2x1 182 to 924; k8x1 66, 93, 138, 167, 210, 287, 844
 // (one lane: 107 at 2,003 and 321 at 79,912 voxels of 31; four classes in four lanes: 50 and 296.)
 // The ordinary fit, an unweighted call's and the one a weighted fit starts from and falls back to, has eight classes
@@ -102,7 +103,7 @@ __host__ __device__ constexpr int lane_count(Lanes lanes) {
 __host__ __device__ inline Lanes small_lanes(int64_t v, int n, bool weighted) {
     if (!weighted) return n > 500 || v <= 6000 ? Lanes::k8x1 : v <= 20000 || n >= 80 ? Lanes::kPlain4 : Lanes::kPlain2;
     if (n >= 96) return Lanes::k8x1;
-    return v <= 6000 ? Lanes::k2x4 : v <= 14000 ? Lanes::k2x2 : Lanes::k2x1;
+    return v <= 6000 ? Lanes::k2x4 : v <= 14000 && n >= 28 ? Lanes::k2x2 : Lanes::k2x1;
 }
 
 // f with the lanes as a compile-time constant.
@@ -268,30 +269,32 @@ __host__ __device__ constexpr int part_row(int R, int part, int k) {
 }
 __host__ __device__ constexpr int part_column(int R, int k) { return R * k; }
 
-// The same from C R lanes: of the class that R lanes share, each takes every R-th exponential, kAhead of them before
-// the sums, and the sums of 8 / R rows of [x, y]^T W [x, y].
+// The same from C R lanes: of the class that R lanes share, each takes every R-th exponential, four of them before
+// the sums (one at a time for a remainder), and the sums of 8 / R rows of [x, y]^T W [x, y].
 template <class T, int C, int R>
 __device__ __forceinline__ void normal_equations_shared(const T* __restrict__ xs, int n, const T* __restrict__ ys,
                                                         int stride, const T (&p)[7], T mx, int g, unsigned mask,
                                                         T (&m)[28], T (&r)[7]) {
-    constexpr int P = 7, LD = row_ld<T>(), kRows = 8 / R, kAhead = 4;
+    constexpr int P = 7, LD = row_ld<T>(), kRows = 8 / R;
     const int c = g % C, part = g / C, first = int(threadIdx.x % 32) - g + c;  // the class's lane of part 0
     T acc[kRows][8];
 #pragma unroll
     for (int k = 0; k < kRows; ++k)
 #pragma unroll
         for (int b = 0; b < 8; ++b) acc[k][b] = T(0);
-    for (int j0 = c; j0 - c < n; j0 += kAhead * R * C) {
+    // The sums of `ahead` measurements per lane of each class, from measurement j0 of all.
+    auto block = [&](auto ahead, int j0) {
+        constexpr int kAhead = decltype(ahead)::value;
         T mine[kAhead], x[8];
 #pragma unroll
         for (int u = 0; u < kAhead; ++u) {
-            load_row(xs + min(j0 + (R * u + part) * C, n - 1) * LD, x);
+            load_row(xs + min(j0 + c + (R * u + part) * C, n - 1) * LD, x);
             mine[u] = dev_exp<T>(T(2) * (predict(x, p) - mx));
         }
 #pragma unroll
         for (int u = 0; u < R * kAhead; ++u) {
             const T from = __shfl_sync(mask, mine[u / R], first + C * (u % R));
-            const int j = j0 + C * u, at = min(j, n - 1);
+            const int j = j0 + c + C * u, at = min(j, n - 1);
             const T w = j < n ? from : T(0);  // adds zeros past the last
             load_row(xs + at * LD, x);
             x[7] = ys[at * stride];
@@ -308,6 +311,15 @@ __device__ __forceinline__ void normal_equations_shared(const T* __restrict__ xs
                 for (int b = 0; b < 8; ++b)
                     if (b >= part_column(R, k)) acc[k][b] = fma(wx, x[b], acc[k][b]);
             }
+        }
+    };
+    for (int j0 = 0; j0 < n;) {
+        if (n - j0 > 3 * R * C) {
+            block(std::integral_constant<int, 4>{}, j0);
+            j0 += 4 * R * C;
+        } else {
+            block(std::integral_constant<int, 1>{}, j0);
+            j0 += R * C;
         }
     }
 #pragma unroll
